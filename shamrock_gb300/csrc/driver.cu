@@ -71,7 +71,7 @@ Ctx::~Ctx() {
                       &row_local, &row_flags, &row_offsets, &leaf_cnt, &leaf_off, &leaf_ent,
                       &owner, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
                       &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &su, &svx, &svy,
-                      &svz, &som, &sP, &scs, &srho, &sinv, &srom, &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &guard_state,
+                      &svz, &som, &sP, &scs, &srho, &sinv, &srom, &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
                       &h_old_row, &eps_row, &omega_local, &a_old, &du_old, &hnew_row, &omega_row,
                       &dt_part, &adj_state, &adj_snap, &adj_loc, &adj_rank, &adj_snap_av, &adj_snap_vg, &adj_vg, &aext, &av_arank,
                       &av_alpha_rank, &av_alpha_upd, &av_diag};
@@ -278,6 +278,9 @@ int gbsph_create(gbsph_ctx **out, int device) {
     gbsph_ctx *ctx = new gbsph_ctx();
     ctx->c.device  = device;
     ctx->c.stream  = 0;
+    int sms        = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
+        ctx->c.sms = (u32) sms;
     if (cudaMallocHost(&ctx->c.h_scalars, sizeof(Scalars)) != cudaSuccess ||
         ctx->c.d_scalars.ensure(sizeof(Scalars), 0) != cudaSuccess ||
         ctx->c.d_bbox.ensure(sizeof(BBox), 0) != cudaSuccess) {

@@ -104,6 +104,7 @@ struct Prof {
 struct Ctx {
     Prof prof;
     int device          = 0;
+    u32 sms             = 152; // multiprocessors of the device
     cudaStream_t stream = 0;
     std::string err;
     int last_status = 0;
@@ -152,6 +153,7 @@ struct Ctx {
     DevBuf srho, sinv, srom; // FP64 pair-loop factors per merged particle (HydroSpace)
     // mixed precision staging (rank order); f_comp: the compensated tier's extra records
     DevBuf f_pos, f_anchor, f_aux0, f_aux1, f_aux2, f_comp;
+    DevBuf f_sums; // pair sums of the mixed derivatives, by rank
     // error-controlled mixed precision: the tier the next step starts in (1 FP32 pair
     // arithmetic, 2 compensated) and the start state a step is recomputed from
     u32 guard_tier = 1;
