@@ -70,11 +70,11 @@ Ctx::~Ctx() {
                       &parent, &boxes, &visit, &fboxes, &fpairs, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
                       &row_local, &row_flags, &row_offsets, &leaf_cnt, &leaf_off, &leaf_ent,
                       &owner, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
-                      &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &su, &svx, &svy,
-                      &svz, &som, &sP, &scs, &srho, &sinv, &srom, &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
+                      &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &scs, &rec64,
+                      &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
                       &h_old_row, &eps_row, &omega_local, &a_old, &du_old, &hnew_row, &omega_row,
                       &dt_part, &adj_state, &adj_snap, &adj_loc, &adj_rank, &adj_snap_av, &adj_snap_vg, &adj_vg, &aext, &av_arank,
-                      &av_alpha_rank, &av_alpha_upd, &av_diag};
+                      &av_alpha_upd, &av_diag};
     cudaSetDevice(device);
     for (DevBuf *b : bufs) b->release(stream);
     cudaStreamSynchronize(stream);
@@ -791,27 +791,14 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         CU(cudaMemcpyAsync(p->omega, c.omega_local.p, 8 * (size_t) n, cudaMemcpyDeviceToDevice, s));
 
     // ---- corrector loop (Solver.cpp:2247-3171)
-    // FP64 rank-ordered hydro copies (the mixed path stages 32-byte records and keeps
-    // only h in FP64)
-    DevBuf *rank_bufs[] = {&c.sh2, &c.su,  &c.svx,  &c.svy, &c.svz, &c.som,
-                           &c.sP,  &c.scs, &c.srho, &c.sinv, &c.srom};
-    for (DevBuf *b : rank_bufs) {
-        CU(b->ensure(8 * (size_t) N, s));
-        if (mixed) break;
-    }
+    // the mixed path keeps h in FP64 in rank order
+    if (mixed) CU(c.sh2.ensure(8 * (size_t) N, s));
     if (tape) {
         CU(tape->snap->ensure(sizeof(f64) * 4 * (size_t) n * tape->forced_iters, s));
         if (cd10) CU(tape->snap_av->ensure(sizeof(f64) * 4 * (size_t) n * tape->forced_iters, s));
         if (cd10 && mixed && tape->snap_vg)
             CU(tape->snap_vg->ensure(sizeof(float) * 24 * (size_t) n * tape->forced_iters, s));
         tape->iters = 0;
-    }
-    HydroSpace hs{c.sh2.as<f64>(), c.su.as<f64>(),  c.svx.as<f64>(), c.svy.as<f64>(),
-                  c.svz.as<f64>(), c.som.as<f64>(), c.sP.as<f64>(),  c.scs.as<f64>()};
-    if (!mixed) {
-        hs.rho    = c.srho.as<f64>();
-        hs.inv_sub = c.sinv.as<f64>();
-        hs.rho_om = c.srom.as<f64>();
     }
     f64 next_cfl   = 0;
     bool rerun     = false;
@@ -825,8 +812,7 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                             "too large");
         if (mixed)
             CU(gather_stage_mixed(c, N, n, lf, c.omega_local.as<f64>(), cfg->pmass, eos, cd10, comp));
-        else CU(gather_eos64(c, N, n, lf, c.omega_local.as<f64>(), cfg->pmass, eos));
-        hs.alpha = nullptr;
+        else CU(gather_eos64(c, N, n, lf, c.omega_local.as<f64>(), cfg->pmass, eos, cd10 ? 1.0 : cfg->alpha_AV));
         if (cd10) {
             // varying viscosity (Solver.cpp:2261-2370): div v, curl v and d(div v)/dt from
             // the current velocities and the accelerations of the last evaluation, the
@@ -854,13 +840,7 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                                  dtdv, vg_sums));
                 if (vg_sums) tape->vg_recorded = true;
             } else {
-                CU(c.av_arank.ensure(sizeof(f64) * 3 * (size_t) N, s));
-                f64 *ar = c.av_arank.as<f64>();
-                CU(gather_merged64(c, N, n, lf.ax, lf.vs, ar));
-                CU(gather_merged64(c, N, n, lf.ay, lf.vs, ar + N));
-                CU(gather_merged64(c, N, n, lf.az, lf.vs, ar + 2 * (size_t) N));
-                CU(velgrad64(c, rs, hs, ar, ar + N, ar + 2 * (size_t) N, cfg->pmass, divv, cx, cy,
-                             cz, cvs, dtdv));
+                CU(velgrad64(c, rs, N, n, lf, cfg->pmass, divv, cx, cy, cz, cvs, dtdv));
             }
             if (cfg->av_kind == GBSPH_AV_VARYING_CD10)
                 CU(cd10_update(c, n, divv, cx, cy, cz, cvs, dtdv, p->soundspeed, lf.h, p->alpha_AV,
@@ -872,9 +852,7 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
             if (mixed) {
                 CU(stage_alpha_mixed(c, N, n, alpha_upd));
             } else {
-                CU(c.av_alpha_rank.ensure(sizeof(f64) * (size_t) N, s));
-                CU(gather_merged64(c, N, n, alpha_upd, 1, c.av_alpha_rank.as<f64>()));
-                hs.alpha = c.av_alpha_rank.as<f64>();
+                CU(stage_alpha64(c, N, n, alpha_upd));
             }
         }
         if (tape) {
@@ -904,8 +882,8 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
             CU(derivs_step_mixed(c, rs, cfg->pmass, cfg->alpha_u, cfg->alpha_AV, cfg->beta_AV,
                                  dt / 2, C_cour, C_force, lf, ext, cd10, cond));
         else
-            CU(derivs_step64(c, rs, hs, cfg->pmass, cfg->alpha_u, cfg->alpha_AV, cfg->beta_AV,
-                             dt / 2, C_cour, C_force, lf, ext));
+            CU(derivs_step64(c, rs, N, cfg->pmass, cfg->alpha_u, cfg->beta_AV, dt / 2, C_cour,
+                             C_force, lf, ext));
         CU(sync_scalars(c));
         f64 rank_veps_v = std::sqrt(ordered_to_f64(c.h_scalars->epsv2_max));
         f64 vmean       = std::sqrt(c.h_scalars->sum_v2 / f64(n));

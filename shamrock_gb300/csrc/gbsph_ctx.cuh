@@ -149,8 +149,8 @@ struct Ctx {
     DevBuf d_ghost_offsets;       // f64[26][3]
 
     // ---- per-step fields in rank order (corrector phase)
-    DevBuf su, svx, svy, svz, som, sP, scs, sh2;
-    DevBuf srho, sinv, srom; // FP64 pair-loop factors per merged particle (HydroSpace)
+    DevBuf scs, sh2;
+    DevBuf rec64; // FP64 pair-loop records, 20 doubles per merged particle (sph64.cu)
     // mixed precision staging (rank order); f_comp: the compensated tier's extra records
     DevBuf f_pos, f_anchor, f_aux0, f_aux1, f_aux2, f_comp;
     DevBuf f_sums; // pair sums of the mixed derivatives, by rank
@@ -172,9 +172,9 @@ struct Ctx {
     // ---- per-row / per-local work arrays
     DevBuf h_old_row, eps_row, omega_local, a_old, du_old, hnew_row, omega_row;
     DevBuf aext; // external acceleration of the step (3 n, SoA)
-    // varying AV: rank-ordered accelerations (3 N) and alpha (N), the updated alpha (n),
+    // varying AV: rank-ordered acceleration records (4 N), the updated alpha (n),
     // div v / curl v / d(div v)/dt when the caller does not take them (5 n)
-    DevBuf av_arank, av_alpha_rank, av_alpha_upd, av_diag;
+    DevBuf av_arank, av_alpha_upd, av_diag;
     DevBuf dt_part;
 
     // ---- adjoint: working state, tape, accumulators (local and rank order)

@@ -15,6 +15,7 @@
 //   predictor + wrap   Solver.cpp:390-524, ForwardEuler.hpp:62-84, integrators.cpp:207-237
 
 #include "gbsph_ctx.cuh"
+#include "lean64.cuh"
 #include "sph_kernels.cuh"
 
 namespace gbsph {
@@ -54,62 +55,153 @@ __device__ __forceinline__ f64 rho_h(f64 m, f64 h) {
 __device__ __forceinline__ f64 inv_sat_positive(f64 v) { return (v >= 1e-9) ? 1. / v : 0.; }
 __device__ __forceinline__ f64 inv_sat_zero(f64 v) { return (v != 0 && v == v) ? 1. / v : 0.; }
 
+// M4 and its derivative at q >= 0 in the expressions above with fewer FP64 instructions:
+// both pieces share their products (their difference is signs and constants), comparisons
+// and exact scalings act on the bits.
+__device__ __forceinline__ f64 quarter(f64 v) { return from64(bits64(v) - (2ull << 52)); } // |v| > 2^-1020
+__device__ __forceinline__ f64 lean_m4_f(f64 q) {
+    f64 t1 = 2 - q;
+    f64 t2 = 1 - q;
+    t1     = t1 * t1 * t1;
+    t2     = t2 * t2 * t2;
+    t1     = quarter(t1); // not zero below q = 2
+    const u32 hq = hi64(q);
+    const f64 t  = t1 - t2;
+    return hq < 0x3FF00000u ? t : (hq < 0x40000000u ? t1 : 0.0);
+}
+__device__ __forceinline__ f64 lean_m4_df(f64 q) {
+    const u32 hq  = hi64(q);
+    const bool in = hq < 0x3FF00000u;
+    const f64 t = 3 * q, u = t - 3;
+    const f64 s = (in ? 9. / 4. : -3. / 4.) * q * q;
+    const f64 v = (in ? -t : u) + s;
+    return hq < 0x40000000u ? v : 0.0;
+}
+
+// FP32 pre-test of a row's pairs from coordinates cut to floats: certainly inside or
+// outside a support radius away from a band about it.  Cutting moves a separation by at
+// most 2^-22 of the coordinates and r^2 / thr by four times that over the radius; rows
+// whose band would not be narrow (or whose radius leaves the float range) decide every
+// pair in FP64.
+struct RowCut {
+    float x, y, z, thr, lo, hi;
+    __device__ __forceinline__ RowCut(f64 xa, f64 ya, f64 za, f64 h) {
+        x = cut32(xa), y = cut32(ya), z = cut32(za);
+        const float r   = 2.f * cut32(h);
+        const float M   = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
+        const float eps = 2e-6f + 9.6e-7f * (M / r + 1.f);
+        thr             = r * r;
+        const bool ok   = thr > 1e-30f && thr < 1e30f && eps < 0.05f;
+        lo = ok ? 1.f - eps : -1.f;
+        hi = ok ? 1.f + eps : __int_as_float(0x7f800000);
+    }
+    __device__ __forceinline__ float r2(f64 xb, f64 yb, f64 zb) const {
+        const float dx = x - cut32(xb), dy = y - cut32(yb), dz = z - cut32(zb);
+        return dx * dx + dy * dy + dz * dz;
+    }
+};
+
 // ---------------------------------------------------------------- density sums
+// The pair terms of one row at h_a, with the plain operators
+__device__ __noinline__ void density_pair_plain(f64 rab2, f64 h_a, f64 &w, f64 &dw) {
+    const f64 rab = sqrt(rab2);
+    w             = W_3d(rab, h_a);
+    dw            = dhW_3d(rab, h_a);
+}
+
+// Called by all 32 lanes of a warp (a lane without work passes k0 = k1).  FP64 instructions
+// bound this loop (two lanes per clock and SM), so a lane first walks to its next pair
+// inside the support in FP32 and all lanes then evaluate one together, with the quotients
+// and the root of lean64.cuh: 44 FP64 instructions per pair instead of about 65, and none
+// for the cached pairs outside the support.
 __device__ __forceinline__ void density_sums(const RowSpace &rs, u32 a, u32 k0, u32 k1, f64 h_a,
                                              f64 pmass, f64 &rho_sum, f64 &sumdWdh) {
     f64 xa = rs.x[a], ya = rs.y[a], za = rs.z[a];
     f64 dint = h_a * h_a * kRkern * kRkern;
+    const RowCut cut(xa, ya, za, h_a);
+    const Denominator H = denominator(h_a), H3 = denominator(h_a * h_a * h_a),
+                      H4 = denominator(h_a * h_a * h_a * h_a);
     rho_sum  = 0;
     sumdWdh  = 0;
-    for (u32 k = k0; k < k1; k++) {
-        u32 b    = rs.ent[k];
-        f64 dx   = xa - rs.x[b], dy = ya - rs.y[b], dz = za - rs.z[b];
-        f64 rab2 = dx * dx + dy * dy + dz * dz;
-        if (rab2 > dint) continue;
-        f64 rab = sqrt(rab2);
-        rho_sum += pmass * W_3d(rab, h_a);
-        sumdWdh += pmass * dhW_3d(rab, h_a);
+    u32 k    = k0;
+    while (true) {
+        f64 rab2  = 0;
+        bool have = false;
+        while (k < k1) {
+            const u32 b  = rs.ent[k++];
+            const f64 xb = rs.x[b], yb = rs.y[b], zb = rs.z[b];
+            const float r2 = cut.r2(xb, yb, zb);
+            if (r2 > cut.thr * cut.hi) continue;
+            const f64 dx = xa - xb, dy = ya - yb, dz = za - zb;
+            rab2 = dx * dx + dy * dy + dz * dz;
+            if (!(r2 < cut.thr * cut.lo) && rab2 > dint) continue;
+            have = true;
+            break;
+        }
+        if (!__any_sync(0xffffffffu, have)) break;
+        if (!have) continue;
+        bool bad     = false;
+        const Root r = root64(rab2, bad);
+        const bool zero = (bits64(rab2) << 1) == 0;
+        bad             = bad && !zero;
+        const f64 rab = zero ? 0.0 : root_value(r);
+        const f64 q   = divide_by(rab, H, bad);
+        const f64 f = lean_m4_f(q), df = lean_m4_df(q);
+        f64 w  = divide_by(kNorm3d * f, H3, bad);
+        f64 dw = divide_by(-(kNorm3d) * (3 * f + q * df), H4, bad);
+        if (bad) density_pair_plain(rab2, h_a, w, dw);
+        rho_sum += pmass * w;
+        sumdWdh += pmass * dw;
     }
 }
 
 // ITERS Newton iterations per row (the reference's global loop is equivalent per
 // particle: a particle's update reads only its own h, so it iterates until its own
 // eps <= eps_p (1e-6 in the reference), becomes -1, or the iteration cap is reached).
-__global__ void __launch_bounds__(256) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
+// The rows of a warp iterate together until the last of them is done.
+__global__ void __launch_bounds__(128) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
                                                    f64 *__restrict__ h_new, f64 *__restrict__ eps,
                                                    f64 pmass, f64 h_evol_max, f64 h_evol_iter_max,
                                                    u32 iters, f64 eps_p, Scalars *sc) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 t      = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = t < rs.n;
     u64 emax = 0, emin = ~0ull;
     u32 used = 0;
-    if (t < rs.n) {
-        u32 a  = rs.row_rank ? rs.row_rank[t] : t;
-        u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
-        const f64 h_max_tot_max_evol = h_evol_max;
-        const f64 h_max_evol_p       = h_evol_iter_max;
-        const f64 h_max_evol_m       = 1 / h_evol_iter_max;
-        f64 ha_0 = h_old[t];
-        f64 h_a  = h_new[t];
-        f64 e    = eps[t];
-        for (u32 it = 0; it < iters; it++) {
-            if (!(e > eps_p)) break;
-            used++;
-            f64 rho_sum, sumdWdh;
-            density_sums(rs, a, k0, k1, h_a, pmass, rho_sum, sumdWdh);
-            f64 rho_ha  = rho_h(pmass, h_a);
-            f64 f_iter  = rho_sum - rho_ha;
-            f64 df_iter = sumdWdh + 3 * rho_ha / h_a;
-            f64 new_h   = h_a - f_iter / df_iter;
-            if (new_h < h_a * h_max_evol_m) new_h = h_max_evol_m * h_a;
-            if (new_h > h_a * h_max_evol_p) new_h = h_max_evol_p * h_a;
-            if (new_h < ha_0 * h_max_tot_max_evol) {
-                e   = fabs(new_h - h_a) / ha_0;
-                h_a = new_h;
-            } else {
-                h_a = ha_0 * h_max_tot_max_evol;
-                e   = -1;
-            }
+    u32 a = 0, k0 = 0, k1 = 0;
+    f64 ha_0 = 1, h_a = 1, e = 0;
+    if (valid) {
+        a    = rs.row_rank ? rs.row_rank[t] : t;
+        k0   = rs.off[t];
+        k1   = k0 + rs.cnt[t];
+        ha_0 = h_old[t];
+        h_a  = h_new[t];
+        e    = eps[t];
+    }
+    const f64 h_max_tot_max_evol = h_evol_max;
+    const f64 h_max_evol_p       = h_evol_iter_max;
+    const f64 h_max_evol_m       = 1 / h_evol_iter_max;
+    for (u32 it = 0; it < iters; it++) {
+        const bool go = valid && e > eps_p;
+        if (!__any_sync(0xffffffffu, go)) break;
+        f64 rho_sum, sumdWdh;
+        density_sums(rs, a, k0, go ? k1 : k0, h_a, pmass, rho_sum, sumdWdh);
+        if (!go) continue;
+        used++;
+        f64 rho_ha  = rho_h(pmass, h_a);
+        f64 f_iter  = rho_sum - rho_ha;
+        f64 df_iter = sumdWdh + 3 * rho_ha / h_a;
+        f64 new_h   = h_a - f_iter / df_iter;
+        if (new_h < h_a * h_max_evol_m) new_h = h_max_evol_m * h_a;
+        if (new_h > h_a * h_max_evol_p) new_h = h_max_evol_p * h_a;
+        if (new_h < ha_0 * h_max_tot_max_evol) {
+            e   = fabs(new_h - h_a) / ha_0;
+            h_a = new_h;
+        } else {
+            h_a = ha_0 * h_max_tot_max_evol;
+            e   = -1;
         }
+    }
+    if (valid) {
         h_new[t] = h_a;
         eps[t]   = e;
         emax     = f64_to_ordered(e);
@@ -119,70 +211,121 @@ __global__ void __launch_bounds__(256) k_h_iterate(RowSpace rs, const f64 *__res
     emin = block_reduce(emin, OpMinU64{}, ~0ull);
     u32 um = block_reduce((u64) used, OpMaxU64{}, 0ull);
     if (threadIdx.x == 0) {
-        atomicMax((unsigned long long *) &sc->eps_max, (unsigned long long) emax);
-        atomicMin((unsigned long long *) &sc->eps_min, (unsigned long long) emin);
-        atomicMax(&sc->iters_max, um);
+        raise_u64(&sc->eps_max, emax);
+        lower_u64(&sc->eps_min, emin);
+        raise_u32(&sc->iters_max, um);
     }
 }
 
-__global__ void __launch_bounds__(256) k_omega(RowSpace rs, const f64 *__restrict__ h_row,
+__global__ void __launch_bounds__(128) k_omega(RowSpace rs, const f64 *__restrict__ h_row,
                                                f64 pmass, f64 *__restrict__ omega_out,
                                                const u32 *__restrict__ out_index) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rs.n) return;
-    u32 a  = rs.row_rank ? rs.row_rank[t] : t;
-    u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
-    f64 h_a = h_row[t];
+    const u32 t      = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = t < rs.n;
+    u32 a = 0, k0 = 0, k1 = 0;
+    f64 h_a = 1;
+    if (valid) {
+        a   = rs.row_rank ? rs.row_rank[t] : t;
+        k0  = rs.off[t];
+        k1  = k0 + rs.cnt[t];
+        h_a = h_row[t];
+    }
     f64 rho_sum, part_omega_sum;
     density_sums(rs, a, k0, k1, h_a, pmass, rho_sum, part_omega_sum);
+    if (!valid) return;
     f64 rho_ha  = rho_h(pmass, h_a);
     f64 omega_a = 1 + (h_a / (3 * rho_ha)) * part_omega_sum;
     omega_out[out_index ? out_index[t] : t] = omega_a;
 }
 
-// gather h, u, v, omega of locals and ghosts into rank order + adiabatic EOS
+// Five 32-byte records per particle, in arrays of their own of N records each, that the
+// FP64 pair loops read with one 256-bit load apiece:
+//   0 {x, y, z, h}   1 {vx, vy, vz, u}   2 {P, alpha c_s, -rho / 2, inv_sat_zero(rho^2 Omega)}
+//   3 {rho, rho Omega, y(rho Omega), y(h)}   4 {h^4, y(h^4) | lo(h), lo(h^4), lo(rho Omega), -}
+// with the reciprocals y and lo of lean64.cuh.  Every factor is the pair loop's own
+// expression evaluated once per particle, so it has the same bits.
+struct __align__(32) D4 {
+    f64 x, y, z, w;
+};
+__device__ __forceinline__ D4 ldd4(const f64 *base, size_t N, u32 rec, u32 r) {
+    const F8 v  = ldg256(base + 4 * (rec * N + r));
+    auto two    = [](float lo, float hi) { return __hiloint2double(__float_as_int(hi), __float_as_int(lo)); };
+    return D4{two(v.a.x, v.a.y), two(v.a.z, v.a.w), two(v.b.x, v.b.y), two(v.b.z, v.b.w)};
+}
+__device__ __forceinline__ void std4(f64 *base, size_t N, u32 rec, u32 r, f64 x, f64 y, f64 z, f64 w) {
+    *(D4 *) (base + 4 * (rec * N + r)) = D4{x, y, z, w};
+}
+__device__ __forceinline__ f64 pack_floats(float lo, float hi) {
+    return __hiloint2double(__float_as_int(hi), __float_as_int(lo));
+}
+__device__ __forceinline__ float low_float(f64 v) { return __int_as_float(__double2loint(v)); }
+__device__ __forceinline__ float high_float(f64 v) { return __int_as_float(__double2hiint(v)); }
+
+__device__ __forceinline__ void stage_record(f64 *rec, size_t N, u32 r, f64 x, f64 y, f64 z, f64 h,
+                                             f64 vx, f64 vy, f64 vz, f64 u, f64 P, f64 acs,
+                                             f64 rho, f64 om) {
+    const f64 rho_om    = rho * om;
+    const Denominator H = denominator(h), H4 = denominator(h * h * h * h), R = denominator(rho_om);
+    std4(rec, N, 0, r, x, y, z, h);
+    std4(rec, N, 1, r, vx, vy, vz, u);
+    std4(rec, N, 2, r, P, acs, -f64(0.5) * rho, inv_sat_zero((rho * rho) * om));
+    std4(rec, N, 3, r, rho, rho_om, R.y, H.y);
+    std4(rec, N, 4, r, H4.b, H4.y, pack_floats(H.lo, H4.lo), pack_floats(R.lo, 0.f));
+}
+
+// gather h, u, v, omega of locals and ghosts into rank order + the equation of state;
+// alpha_AV: the constant viscosity (the varying one multiplies its alpha in later, record 2
+// then holds c_s here)
 __global__ void k_gather_eos(const u32 *__restrict__ sort_index, u32 N, u32 n_local,
                              const u32 *__restrict__ ghost_src, const f64 *__restrict__ h,
                              const f64 *__restrict__ u, const f64 *__restrict__ vx,
                              const f64 *__restrict__ vy, const f64 *__restrict__ vz, u32 vs,
-                             const f64 *__restrict__ omega, f64 pmass, EosParams eos,
+                             const f64 *__restrict__ omega, f64 pmass, EosParams eos, f64 alpha_AV,
                              const f64 *__restrict__ sx, const f64 *__restrict__ sy,
-                             const f64 *__restrict__ sz,
-                             f64 *__restrict__ sh, f64 *__restrict__ su, f64 *__restrict__ svx,
-                             f64 *__restrict__ svy, f64 *__restrict__ svz, f64 *__restrict__ som,
-                             f64 *__restrict__ sP, f64 *__restrict__ scs, f64 *__restrict__ srho,
-                             f64 *__restrict__ sinv, f64 *__restrict__ srom) {
+                             const f64 *__restrict__ sz, f64 *__restrict__ scs,
+                             f64 *__restrict__ rec) {
     u32 r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= N) return;
     u32 id  = sort_index[r];
     u32 src = id < n_local ? id : ghost_src[id - n_local];
-    f64 hh = h[src], uu = u[src];
-    sh[r]  = hh;
-    su[r]  = uu;
-    svx[r] = vx[(size_t) src * vs];
-    svy[r] = vy[(size_t) src * vs];
-    svz[r] = vz[(size_t) src * vs];
-    const f64 om = omega[src];
-    som[r] = om;
-    f64 rho = rho_h(pmass, hh);
-    if (srho) {
-        // the pair loop's per-neighbour factors, in its own expressions (derivs_row)
-        srho[r] = rho;
-        sinv[r] = inv_sat_zero((rho * rho) * om);
-        srom[r] = rho * om;
-    }
+    const f64 hh = h[src], uu = u[src];
+    const f64 x = sx[r], y = sy[r], z = sz[r];
+    const f64 rho = rho_h(pmass, hh);
+    f64 P, cs;
     if (eos.kind == 1) {
         // LP07 at the merged (rank-ordered) position
-        f64 x = sx[r], y = sy[r], z = sz[r];
         f64 Rsq   = x * x + y * y + z * z;
         f64 cs_sq = (eos.cs0 * eos.cs0) * pow(Rsq / (eos.r0 * eos.r0), -eos.q);
-        sP[r]     = cs_sq * rho;
-        scs[r]    = sqrt(cs_sq);
+        P         = cs_sq * rho;
+        cs        = sqrt(cs_sq);
     } else {
-        f64 P  = (eos.gamma - 1) * rho * uu;
-        sP[r]  = P;
-        scs[r] = sqrt(eos.gamma * P / rho);
+        P  = (eos.gamma - 1) * rho * uu;
+        cs = sqrt(eos.gamma * P / rho);
     }
+    scs[r] = cs;
+    stage_record(rec, N, r, x, y, z, hh, vx[(size_t) src * vs], vy[(size_t) src * vs],
+                 vz[(size_t) src * vs], uu, P, alpha_AV * cs, rho, omega[src]);
+}
+
+// the same records from the module's merged arrays
+__global__ void k_stage_modules(u32 N, const f64 *__restrict__ x, const f64 *__restrict__ y,
+                                const f64 *__restrict__ z, HydroSpace hs, f64 pmass, f64 alpha_AV,
+                                f64 *__restrict__ rec) {
+    u32 r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= N) return;
+    stage_record(rec, N, r, x[r], y[r], z[r], hs.h[r], hs.vx[r], hs.vy[r], hs.vz[r], hs.u[r], hs.P[r],
+                 alpha_AV * hs.cs[r], rho_h(pmass, hs.h[r]), hs.omega[r]);
+}
+
+// varying viscosity: alpha c_s of record 2 from the updated per-particle alpha
+__global__ void k_stage_alpha64(const u32 *__restrict__ sort_index, u32 N, u32 n_local,
+                                const u32 *__restrict__ ghost_src, const f64 *__restrict__ alpha,
+                                const f64 *__restrict__ scs, f64 *__restrict__ rec) {
+    u32 r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= N) return;
+    const u32 id  = sort_index[r];
+    const u32 src = id < n_local ? id : ghost_src[id - n_local];
+    rec[4 * (2 * (size_t) N + r) + 1] = alpha[src] * scs[r];
 }
 
 __global__ void k_eos_lp07(u32 n, const f64 *__restrict__ x, const f64 *__restrict__ y,
@@ -210,107 +353,257 @@ __global__ void k_eos(u32 n, const f64 *__restrict__ h, const f64 *__restrict__ 
 
 // ---------------------------------------------------------------- derivatives
 struct DerivParams {
-    f64 pmass, alpha_u, alpha_AV, beta_AV;
+    f64 pmass, alpha_u, beta_AV;
     f64 hdt;             // dt / 2 for the corrector
     f64 C_cour, C_force; // CFL factors (already x cfl multiplier)
     ExtAccel ext;        // external acceleration added to the hydro one (may be null)
 };
 
-// PRE: the neighbour's rho, inv_sat_zero(rho^2 Omega) and rho Omega are read from the
-// staged per-particle factors (hs.rho, hs.inv_sub, hs.rho_om) instead of recomputed per
-// pair: the same expressions evaluated once, so the same bits, and two FP64 divisions and
-// five multiplications fewer per pair on GB300's scarce FP64 pipe.
-template<bool VSIG, bool PRE = false>
-__device__ __forceinline__ void derivs_row(const RowSpace &rs, const HydroSpace &hs, u32 a, u32 k0,
-                                           u32 k1, const DerivParams &p, f64 &fx, f64 &fy, f64 &fz,
+// One row's particle, as the pair loop keeps it
+struct Row64 {
+    D4 p, v, e; // records 0, 1, 2
+    f64 rho, inv_rho_om, c_heat; // rho, 1 / (Omega rho), that times 1 / rho
+    Denominator H, H4;
+};
+// the pair's contributions and v.r_hat of the forces
+struct Pair64 {
+    f64 fx, fy, fz, t1, t2, vr;
+};
+
+// v / 2 where that is exact
+__device__ __forceinline__ f64 half(f64 v, bool &bad) {
+    const bool zero = (bits64(v) << 1) == 0;
+    bad |= !zero && (hi64(v) & 0x7FFFFFFFu) - 0x00200000u >= 0x7FD00000u;
+    return zero ? v : from64(bits64(v) - (1ull << 52));
+}
+// fmax(v, 0): 0 for NaN
+__device__ __forceinline__ f64 positive(f64 v) {
+    return bits64(v) - 1ull < 0x7FF0000000000000ull ? v : 0.0;
+}
+
+// The pair terms with the plain operators (UpdateDerivs.cpp:176-271)
+__device__ __noinline__ void force_pair_plain(const Row64 &A, const D4 &B0, const D4 &B1,
+                                              const D4 &B2, const D4 &B3, const DerivParams &p,
+                                              Pair64 &o) {
+    const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+    const f64 rab = sqrt(dx * dx + dy * dy + dz * dz);
+    f64 Fab_a   = dW_3d(rab, A.p.w);
+    f64 Fab_b   = dW_3d(rab, B0.w);
+    f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+    f64 inv = inv_sat_positive(rab);
+    f64 rx = dx * inv, ry = dy * inv, rz = dz * inv;
+    f64 vr      = vx * rx + vy * ry + vz * rz;
+    f64 bv      = p.beta_AV * fabs(vr);
+    f64 vsig_a  = A.e.y + bv;
+    f64 vsig_b  = B2.y + bv;
+    f64 rho_avg = (A.rho + B3.x) * 0.5;
+    f64 vsig_u  = sqrt(fabs(A.e.x - B2.x) / rho_avg);
+    f64 AV_P_a  = A.e.x + fmax(A.e.z * vsig_a * vr, f64(0));
+    f64 AV_P_b  = B2.x + fmax(B2.z * vsig_b * vr, f64(0));
+    f64 ca = AV_P_a * A.e.w, cb = AV_P_b * B2.w;
+    f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
+    f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
+    f64 mb = -p.pmass;
+    o.fx = mb * (ca * nax + cb * nbx);
+    o.fy = mb * (ca * nay + cb * nby);
+    o.fz = mb * (ca * naz + cb * nbz);
+    o.t1 = AV_P_a * A.c_heat * p.pmass * (vx * nax + vy * nay + vz * naz);
+    f64 Fa = Fab_a * A.inv_rho_om;
+    f64 Fb = Fab_b / B3.y;
+    o.t2 = p.pmass * p.alpha_u * vsig_u * (A.v.w - B1.w) * f64(0.5) * (Fa + Fb);
+    o.vr = vr;
+}
+
+// v.r_hat of the reference's separate v_sig kernel: r_hat = dr / r, zero below 1e-9
+__device__ __noinline__ f64 sig_speed_plain(const Row64 &A, const D4 &B0, const D4 &B1) {
+    const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+    const f64 rab = sqrt(dx * dx + dy * dy + dz * dz);
+    const f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+    f64 ux = dx / rab, uy = dy / rab, uz = dz / rab;
+    if (rab < 1e-9) ux = uy = uz = 0;
+    return fabs(vx * ux + vy * uy + vz * uz);
+}
+
+// The FP64 pair loop, called by all 32 lanes of a warp (no row: k0 = k1).  It is bound by
+// the FP64 pipe, so as in density_sums a lane first walks to its next pair inside either
+// support in FP32, then all lanes evaluate a pair together from the staged records with the
+// quotients, roots and reciprocals of lean64.cuh: 112 FP64 instructions per pair instead of
+// about 215, none for the quarter of the cached pairs outside both supports and no
+// divergence between the pieces of M4.  The particle itself adds zeros and is skipped
+// unless a field of the row is not finite.
+// The v_sig maximum, max over the pairs of c_s + 2 |v.u| with u = dr / r: rounding is
+// monotonic, so that of the largest |v.u|, which differs from the forces' v.r_hat = v.(dr
+// (1/r)) by a few units in the last place of |v|.  The loop keeps the pairs whose |v.r_hat|
+// could be the largest within that margin and evaluates the three quotients for those only
+// (every pair of the row where more than kSigCandidates are that close).
+constexpr u32 kSigCandidates = 12;
+
+template<bool VSIG>
+__device__ __forceinline__ void derivs_row(const u32 *__restrict__ ent, const f64 *__restrict__ rec,
+                                           size_t N, u32 a, u32 k0, u32 k1, f64 cs_a,
+                                           const DerivParams &p, f64 &fx, f64 &fy, f64 &fz,
                                            f64 &tdu, f64 &vsig_max) {
     const f64 Rker2 = kRkern * kRkern;
-    f64 h_a = hs.h[a];
-    f64 xa = rs.x[a], ya = rs.y[a], za = rs.z[a];
-    f64 vxa = hs.vx[a], vya = hs.vy[a], vza = hs.vz[a];
-    f64 P_a = hs.P[a], omega_a = hs.omega[a];
-    const f64 u_a         = hs.u[a];
-    f64 rho_a             = rho_h(p.pmass, h_a);
-    f64 rho_a_sq          = rho_a * rho_a;
-    f64 rho_a_inv         = 1. / rho_a;
-    f64 omega_a_rho_a_inv = 1 / (omega_a * rho_a);
-    f64 cs_a              = hs.cs[a];
-    const f64 alpha_a     = hs.alpha ? hs.alpha[a] : p.alpha_AV;
+    Row64 A;
+    bool plain_row;
+    {
+        A.p = ldd4(rec, N, 0, a), A.v = ldd4(rec, N, 1, a), A.e = ldd4(rec, N, 2, a);
+        const D4 c = ldd4(rec, N, 3, a), d = ldd4(rec, N, 4, a);
+        A.rho        = c.x;
+        A.inv_rho_om = 1 / c.y;
+        A.c_heat     = A.inv_rho_om * (1. / A.rho);
+        A.H          = Denominator{A.p.w, c.w, low_float(d.z)};
+        A.H4         = Denominator{d.x, d.y, high_float(d.z)};
+        // a sum is finite only if its terms are (or cancel infinities, which gives NaN)
+        const f64 all = fabs(A.v.x) + fabs(A.v.y) + fabs(A.v.z) + fabs(A.v.w) + fabs(A.e.x)
+                        + fabs(A.e.y) + fabs(A.e.z) + fabs(A.e.w) + fabs(A.c_heat);
+        plain_row = !(all < 1e300) || !(A.H.lo == A.H.lo) || !(A.H4.lo == A.H4.lo);
+    }
+    const RowCut cut(A.p.x, A.p.y, A.p.z, A.p.w);
     fx = fy = fz = tdu = 0;
-    vsig_max           = 0;
-    for (u32 k = k0; k < k1; k++) {
-        u32 b    = rs.ent[k];
-        f64 dx   = xa - rs.x[b], dy = ya - rs.y[b], dz = za - rs.z[b];
-        f64 rab2 = dx * dx + dy * dy + dz * dz;
-        f64 h_b  = hs.h[b];
-        if (rab2 > h_a * h_a * Rker2 && rab2 > h_b * h_b * Rker2) continue;
-        f64 rab       = sqrt(rab2);
-        const f64 u_b = hs.u[b];
-        f64 rho_b   = PRE ? hs.rho[b] : rho_h(p.pmass, h_b);
-        f64 P_b     = hs.P[b];
-        f64 cs_b    = hs.cs[b];
-        f64 Fab_a   = dW_3d(rab, h_a);
-        f64 Fab_b   = dW_3d(rab, h_b);
-        f64 vx = vxa - hs.vx[b], vy = vya - hs.vy[b], vz = vza - hs.vz[b];
-        f64 inv = inv_sat_positive(rab);
-        f64 rx = dx * inv, ry = dy * inv, rz = dz * inv;
-        f64 v_ab_r_ab     = vx * rx + vy * ry + vz * rz;
-        f64 abs_v_ab_r_ab = fabs(v_ab_r_ab);
-        // varying AV: alpha_a, alpha_b per particle (NodeUpdateDerivsVaryingAlphaAV.cpp:95-96)
-        const f64 alpha_b = hs.alpha ? hs.alpha[b] : p.alpha_AV;
-        f64 vsig_a  = alpha_a * cs_a + p.beta_AV * abs_v_ab_r_ab;
-        f64 vsig_b  = alpha_b * cs_b + p.beta_AV * abs_v_ab_r_ab;
-        f64 rho_avg = (rho_a + rho_b) * 0.5;
-        f64 abs_dp  = fabs(P_a - P_b);
-        f64 vsig_u  = sqrt(abs_dp / rho_avg);
-        f64 qa_ab   = fmax(-f64(0.5) * rho_a * vsig_a * v_ab_r_ab, f64(0));
-        f64 qb_ab   = fmax(-f64(0.5) * rho_b * vsig_b * v_ab_r_ab, f64(0));
-        f64 AV_P_a  = P_a + qa_ab;
-        f64 AV_P_b  = P_b + qb_ab;
-        f64 sub_fact_a = rho_a_sq * omega_a;
-        f64 ca = AV_P_a * inv_sat_zero(sub_fact_a);
-        f64 cb;
-        if (PRE) {
-            cb = AV_P_b * hs.inv_sub[b];
-        } else {
-            f64 sub_fact_b = (rho_b * rho_b) * hs.omega[b];
-            cb = AV_P_b * inv_sat_zero(sub_fact_b);
+    float sig_low = -1.f;     // a lower bound of the largest |v.u|
+    u32 sig_n     = 0;        // candidates kept
+    u32 sig_k[kSigCandidates];
+    float sig_up[kSigCandidates];
+    bool any_pair = false;
+    u32 k         = k0;
+    while (true) {
+        D4 B0;
+        f64 rab2  = 0;
+        u32 b     = a;
+        bool have = false;
+        while (k < k1) {
+            b  = ent[k++];
+            B0 = ldd4(rec, N, 0, b);
+            const float r2  = cut.r2(B0.x, B0.y, B0.z);
+            const float hb  = cut32(B0.w); // NaN bounds decide nothing
+            const float tm  = hb < 1e18f ? fmaxf(cut.thr, 4.f * hb * hb) : __int_as_float(0x7fc00000);
+            if (r2 > tm * cut.hi) continue;
+            if (b == a && !plain_row) {
+                any_pair = true;
+                continue;
+            }
+            const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+            rab2 = dx * dx + dy * dy + dz * dz;
+            if (!(r2 < tm * cut.lo) && rab2 > A.p.w * A.p.w * Rker2 && rab2 > B0.w * B0.w * Rker2)
+                continue;
+            have = true;
+            break;
         }
-        f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
-        f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
-        f64 mb = -p.pmass;
-        fx += mb * (ca * nax + cb * nbx);
-        fy += mb * (ca * nay + cb * nby);
-        fz += mb * (ca * naz + cb * nbz);
-        f64 dotvg = vx * nax + vy * nay + vz * naz;
-        tdu += AV_P_a * (omega_a_rho_a_inv * rho_a_inv) * p.pmass * dotvg;
-        f64 Fa = Fab_a * omega_a_rho_a_inv;
-        f64 Fb = Fab_b / (PRE ? hs.rho_om[b] : rho_b * hs.omega[b]);
-        tdu += p.pmass * p.alpha_u * vsig_u * (u_a - u_b) * f64(0.5) * (Fa + Fb);
-        if (VSIG) {
-            // separate v_sig kernel of the reference: r_hat = dr / r, zero below 1e-9,
-            // alpha = 1, beta = 2 fixed
-            f64 ux = dx / rab, uy = dy / rab, uz = dz / rab;
-            if (rab < 1e-9) ux = uy = uz = 0;
-            f64 vr = vx * ux + vy * uy + vz * uz;
-            f64 vs = 1.0 * cs_a + 2.0 * fabs(vr);
-            vsig_max = fmax(vsig_max, vs);
+        if (!__any_sync(0xffffffffu, have)) break;
+        if (!have) continue;
+        any_pair    = true;
+        const D4 B1 = ldd4(rec, N, 1, b), B2 = ldd4(rec, N, 2, b), B3 = ldd4(rec, N, 3, b),
+                 B4 = ldd4(rec, N, 4, b);
+        const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+        bool bad      = plain_row;
+        const Root r  = root64(rab2, bad);
+        const f64 rab = root_value(r);
+        f64 inv       = root_reciprocal(r, bad);
+        if (bits64(rab) < bits64(1e-9)) inv = 0;
+        const Denominator HB{B0.w, B3.w, low_float(B4.z)}, HB4{B4.x, B4.y, high_float(B4.z)},
+            RB{B3.y, B3.z, low_float(B4.w)};
+        const f64 Fab_a = divide_by(kNorm3d * lean_m4_df(divide_by(rab, A.H, bad)), A.H4, bad);
+        const f64 Fab_b = divide_by(kNorm3d * lean_m4_df(divide_by(rab, HB, bad)), HB4, bad);
+        const f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+        const f64 rx = dx * inv, ry = dy * inv, rz = dz * inv;
+        Pair64 o;
+        o.vr             = vx * rx + vy * ry + vz * rz;
+        const f64 bv     = p.beta_AV * fabs(o.vr);
+        const f64 vsig_a = A.e.y + bv;
+        const f64 vsig_b = B2.y + bv;
+        const f64 dp     = fabs(A.e.x - B2.x);
+        f64 vsig_u       = 0;
+        {
+            bool odd       = false;
+            const f64 sum  = A.rho + B3.x;
+            const f64 q    = quotient64(dp, half(sum, odd), odd);
+            const Root ru  = root64(q, odd);
+            const bool eq  = bits64(dp) == 0; // sqrt(0 / rho) = 0
+            vsig_u         = eq ? 0.0 : root_value(ru);
+            bad |= eq ? !(hi64(sum) - 0x00100000u < 0x7FE00000u) : odd;
         }
+        const f64 AV_P_a = A.e.x + positive(A.e.z * vsig_a * o.vr);
+        const f64 AV_P_b = B2.x + positive(B2.z * vsig_b * o.vr);
+        const f64 ca = AV_P_a * A.e.w, cb = AV_P_b * B2.w;
+        const f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
+        const f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
+        const f64 mb = -p.pmass;
+        o.fx = mb * (ca * nax + cb * nbx);
+        o.fy = mb * (ca * nay + cb * nby);
+        o.fz = mb * (ca * naz + cb * nbz);
+        o.t1 = AV_P_a * A.c_heat * p.pmass * (vx * nax + vy * nay + vz * naz);
+        const f64 Fa = Fab_a * A.inv_rho_om;
+        const f64 Fb = divide_by(Fab_b, RB, bad);
+        o.t2 = half(p.pmass * p.alpha_u * vsig_u * (A.v.w - B1.w), bad) * (Fa + Fb);
+        if (bad) force_pair_plain(A, B0, B1, B2, B3, p, o);
+        fx += o.fx;
+        fy += o.fy;
+        fz += o.fz;
+        tdu += o.t1;
+        tdu += o.t2;
+        // a pair at rest adds 0 to the maximum
+        if (VSIG && ((bits64(vx) | bits64(vy) | bits64(vz)) << 1) != 0) {
+            const float vf = fabsf(cut32(vx)) + fabsf(cut32(vy)) + fabsf(cut32(vz));
+            const float w  = fabsf(cut32(o.vr)), slack = 3e-7f * w + 1e-14f * vf;
+            // NaN or out of the float range: always a candidate
+            const float up = w + slack < 1e37f ? w + slack : __int_as_float(0x7f800000);
+            if (up >= sig_low) {
+                if (sig_n < kSigCandidates) {
+                    sig_k[sig_n]  = k - 1;
+                    sig_up[sig_n] = up;
+                }
+                sig_n++;
+                if (w - slack > sig_low) {
+                    sig_low = w - slack;
+                    // forget the candidates it overtakes
+                    u32 m = 0;
+                    for (u32 i = 0; i < min(sig_n, kSigCandidates); i++)
+                        if (sig_up[i] >= sig_low) {
+                            sig_k[m]    = sig_k[i];
+                            sig_up[m++] = sig_up[i];
+                        }
+                    if (sig_n <= kSigCandidates) sig_n = m;
+                }
+            }
+        }
+    }
+    vsig_max = 0;
+    if (VSIG && any_pair) {
+        f64 vr       = 0;
+        const bool few = sig_n <= kSigCandidates;
+        const u32 n    = few ? sig_n : k1 - k0;
+        for (u32 i = 0; i < n; i++) {
+            const u32 b = ent[few ? sig_k[i] : k0 + i];
+            const D4 B0 = ldd4(rec, N, 0, b);
+            if (!few) {
+                const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+                const f64 d2 = dx * dx + dy * dy + dz * dz;
+                if (d2 > A.p.w * A.p.w * Rker2 && d2 > B0.w * B0.w * Rker2) continue;
+            }
+            vr = fmax(vr, sig_speed_plain(A, B0, ldd4(rec, N, 1, b)));
+        }
+        vsig_max = fmax(vsig_max, 1.0 * cs_a + 2.0 * vr);
     }
 }
 
 // module form: reference CSR, outputs a, du (and vsig) by row
-__global__ void __launch_bounds__(128) k_derivs(RowSpace rs, HydroSpace hs, DerivParams p,
+__global__ void __launch_bounds__(128) k_derivs(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+                                                const f64 *__restrict__ cs, DerivParams p,
                                                 f64 *__restrict__ ax, f64 *__restrict__ ay,
                                                 f64 *__restrict__ az, f64 *__restrict__ du,
                                                 f64 *__restrict__ vsig) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rs.n) return;
-    u32 a  = rs.row_rank ? rs.row_rank[t] : t;
-    u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    u32 a = 0, k0 = 0, k1 = 0;
+    if (t < rs.n) {
+        a  = rs.row_rank ? rs.row_rank[t] : t;
+        k0 = rs.off[t];
+        k1 = k0 + rs.cnt[t];
+    }
     f64 fx, fy, fz, tdu, vm;
-    if (vsig) derivs_row<true>(rs, hs, a, k0, k1, p, fx, fy, fz, tdu, vm);
-    else derivs_row<false>(rs, hs, a, k0, k1, p, fx, fy, fz, tdu, vm);
+    if (vsig) derivs_row<true>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
+    else derivs_row<false>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
+    if (t >= rs.n) return;
     ax[t] = fx;
     ay[t] = fy;
     az[t] = fz;
@@ -319,19 +612,23 @@ __global__ void __launch_bounds__(128) k_derivs(RowSpace rs, HydroSpace hs, Deri
 }
 
 // pipeline form: derivatives + v_sig + leapfrog corrector + CFL, outputs to the
-// caller's local arrays.  Neighbour velocities come from the rank-ordered copy
+// caller's local arrays.  Neighbour velocities come from the staged records
 // taken before the corrector, so correcting the caller's v here is race-free.
-template<bool PRE>
-__global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, HydroSpace hs, DerivParams p,
+__global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+                                                     const f64 *__restrict__ cs, DerivParams p,
                                                      LocalFields lf, Scalars *sc) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
     u64 ev2 = 0, dtm = ~0ull;
     f64 v2  = 0;
+    u32 a = 0, k0 = 0, k1 = 0;
     if (t < rs.n) {
-        u32 a  = rs.row_rank[t];
-        u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
-        f64 fx, fy, fz, tdu, vm;
-        derivs_row<true, PRE>(rs, hs, a, k0, k1, p, fx, fy, fz, tdu, vm);
+        a  = rs.row_rank[t];
+        k0 = rs.off[t];
+        k1 = k0 + rs.cnt[t];
+    }
+    f64 fx, fy, fz, tdu, vm;
+    derivs_row<true>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
+    if (t < rs.n) {
         u32 i  = rs.row_local[t];
         size_t iv = (size_t) i * lf.vs;
         if (p.ext.x) {
@@ -356,7 +653,7 @@ __global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, HydroSpace hs,
         ev2       = f64_to_ordered(ix * ix + iy * iy + iz * iz);
         v2        = nvx * nvx + nvy * nvy + nvz * nvz;
         // CFL with the new acceleration
-        f64 h_a  = hs.h[a];
+        f64 h_a  = rec[4 * (size_t) a + 3];
         f64 dt   = __longlong_as_double(0x7ff0000000000000ll);
         f64 dt_c = p.C_cour * h_a / vm;
         dt       = fmin(dt, dt_c);
@@ -369,8 +666,8 @@ __global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, HydroSpace hs,
     dtm = block_reduce(dtm, OpMinU64{}, ~0ull);
     v2  = block_reduce(v2, OpAddF64{}, 0.0);
     if (threadIdx.x == 0) {
-        atomicMax((unsigned long long *) &sc->epsv2_max, (unsigned long long) ev2);
-        atomicMin((unsigned long long *) &sc->dt_min, (unsigned long long) dtm);
+        raise_u64(&sc->epsv2_max, ev2);
+        lower_u64(&sc->dt_min, dtm);
         atomicAdd(&sc->sum_v2, v2);
     }
 }
@@ -515,38 +812,74 @@ __device__ __forceinline__ void mul33(const f64 a[3][3], const f64 b[3][3], f64 
         for (int j = 0; j < 3; j++) c[i][j] = (a[i][0] * b[0][j] + a[i][1] * b[1][j]) + a[i][2] * b[2][j];
 }
 
-__global__ void __launch_bounds__(128) k_velgrad64(RowSpace rs, HydroSpace hs,
-                                                   const f64 *__restrict__ axr,
-                                                   const f64 *__restrict__ ayr,
-                                                   const f64 *__restrict__ azr, f64 pmass,
+// the pair's e = r / |r| (zero below 1e-9) and F = dW(|r|, h_a) with the plain operators
+__device__ __noinline__ void gradient_pair_plain(const f64 r[3], f64 rab2, f64 h_a, f64 e[3], f64 &F) {
+    const f64 rab = sqrt(rab2);
+    for (int c = 0; c < 3; c++) e[c] = (rab < 1e-9) ? 0.0 : r[c] / rab;
+    F = dW_3d(rab, h_a);
+}
+
+// Bound by the FP64 pipe like the loops above and arranged like them.  Pairs beyond 2 h_a
+// (inside the neighbour's support only) have F = 0 and add zeros, so those that the FP32
+// test finds outside are not evaluated.  acc: records {ax, ay, az, -} of the last evaluation.
+__global__ void __launch_bounds__(128) k_velgrad64(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+                                                   const f64 *__restrict__ acc, f64 pmass,
                                                    f64 *__restrict__ divv, f64 *__restrict__ cx,
                                                    f64 *__restrict__ cy, f64 *__restrict__ cz,
                                                    u32 cvs, f64 *__restrict__ dtdivv) {
     u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rs.n) return;
-    const u32 a  = rs.row_rank[t];
-    const u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
+    u32 a = 0, k0 = 0, k1 = 0;
+    if (t < rs.n) {
+        a  = rs.row_rank[t];
+        k0 = rs.off[t];
+        k1 = k0 + rs.cnt[t];
+    }
     const f64 Rker2 = kRkern * kRkern;
-    const f64 h_a   = hs.h[a];
-    const f64 xa[3] = {rs.x[a], rs.y[a], rs.z[a]};
-    const f64 va[3] = {hs.vx[a], hs.vy[a], hs.vz[a]};
-    const f64 aa[3] = {axr[a], ayr[a], azr[a]};
-    const f64 rho_a = rho_h(pmass, h_a);
-    const f64 inv_rho_omega_a = 1. / (hs.omega[a] * rho_a);
+    const D4 A0 = ldd4(rec, N, 0, a), A1 = ldd4(rec, N, 1, a), A3 = ldd4(rec, N, 3, a),
+             A4 = ldd4(rec, N, 4, a), Aa = ldd4(acc, N, 0, a);
+    const f64 h_a = A0.w;
+    const Denominator H{h_a, A3.w, low_float(A4.z)}, H4{A4.x, A4.y, high_float(A4.z)};
+    const f64 inv_rho_omega_a = 1. / A3.y; // 1 / (Omega rho)
+    const RowCut cut(A0.x, A0.y, A0.z, h_a);
+    const bool plain_row = !(fabs(A1.x) + fabs(A1.y) + fabs(A1.z) + fabs(Aa.x) + fabs(Aa.y) + fabs(Aa.z) < 1e300)
+                           || !(H.lo == H.lo) || !(H4.lo == H4.lo);
     f64 sdiv = 0, sc[3] = {0, 0, 0};
     f64 R[3][3] = {}, Dv[3][3] = {}, Da[3][3] = {};
-    for (u32 k = k0; k < k1; k++) {
-        const u32 b    = rs.ent[k];
-        const f64 r[3] = {xa[0] - rs.x[b], xa[1] - rs.y[b], xa[2] - rs.z[b]};
-        const f64 rab2 = (r[0] * r[0] + r[1] * r[1]) + r[2] * r[2];
-        const f64 h_b  = hs.h[b];
-        if (rab2 > h_a * h_a * Rker2 && rab2 > h_b * h_b * Rker2) continue;
-        const f64 rab  = sqrt(rab2);
-        const f64 v[3] = {va[0] - hs.vx[b], va[1] - hs.vy[b], va[2] - hs.vz[b]};
-        const f64 w[3] = {aa[0] - axr[b], aa[1] - ayr[b], aa[2] - azr[b]};
-        f64 e[3] = {r[0] / rab, r[1] / rab, r[2] / rab};
-        if (rab < 1e-9) e[0] = e[1] = e[2] = 0;
-        const f64 F    = dW_3d(rab, h_a);
+    u32 k = k0;
+    while (true) {
+        f64 r[3]  = {0, 0, 0}, rab2 = 0;
+        u32 b     = a;
+        bool have = false;
+        while (k < k1) {
+            b           = rs.ent[k++];
+            const D4 B0 = ldd4(rec, N, 0, b);
+            const float r2 = cut.r2(B0.x, B0.y, B0.z);
+            if (!plain_row && (r2 > cut.thr * cut.hi || b == a)) continue;
+            r[0] = A0.x - B0.x;
+            r[1] = A0.y - B0.y;
+            r[2] = A0.z - B0.z;
+            rab2 = (r[0] * r[0] + r[1] * r[1]) + r[2] * r[2];
+            if (!(r2 < cut.thr * cut.lo) && rab2 > h_a * h_a * Rker2 && rab2 > B0.w * B0.w * Rker2)
+                continue;
+            have = true;
+            break;
+        }
+        if (!__any_sync(0xffffffffu, have)) break;
+        if (!have) continue;
+        const D4 B1 = ldd4(rec, N, 1, b), Ba = ldd4(acc, N, 0, b);
+        const f64 v[3] = {A1.x - B1.x, A1.y - B1.y, A1.z - B1.z};
+        const f64 w[3] = {Aa.x - Ba.x, Aa.y - Ba.y, Aa.z - Ba.z};
+        bool bad        = plain_row;
+        const Root root = root64(rab2, bad);
+        const f64 rab   = root_value(root);
+        Denominator D{rab, 0, 0.f};
+        root_reciprocal(root, bad, D.y, D.lo);
+        bad |= bits64(rab) < bits64(1e-9);
+        f64 e[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) e[c] = divide_by(r[c], D, bad);
+        f64 F = divide_by(kNorm3d * lean_m4_df(divide_by(rab, H, bad)), H4, bad);
+        if (bad) gradient_pair_plain(r, rab2, h_a, e, F);
         const f64 g[3] = {F * e[0], F * e[1], F * e[2]};
         sdiv  = sdiv + pmass * ((v[0] * g[0] + v[1] * g[1]) + v[2] * g[2]);
         sc[0] = sc[0] + pmass * (v[1] * g[2] - v[2] * g[1]);
@@ -562,6 +895,7 @@ __global__ void __launch_bounds__(128) k_velgrad64(RowSpace rs, HydroSpace hs,
                 Da[j][i] = Da[j][i] - w[i] * mg[j];
             }
     }
+    if (t >= rs.n) return;
     const u32 i = rs.row_local[t];
     divv[i]     = -inv_rho_omega_a * sdiv;
     cx[(size_t) i * cvs] = -inv_rho_omega_a * sc[0];
@@ -633,14 +967,16 @@ __global__ void k_mm97(u32 n, const f64 *__restrict__ divv, const f64 *__restric
     alpha_new[i]    = (f64) ((na < alpha_max) ? na : alpha_max);
 }
 
-__global__ void k_gather_merged(const u32 *__restrict__ sort_index, u32 N, u32 n_local,
-                                const u32 *__restrict__ ghost_src, const f64 *__restrict__ src,
-                                u32 stride, f64 *__restrict__ dst) {
+// accelerations of the last evaluation in rank order (ghosts copy their source), one
+// 32-byte record per rank
+__global__ void k_gather_acc(const u32 *__restrict__ sort_index, u32 N, u32 n_local,
+                             const u32 *__restrict__ ghost_src, LocalFields lf,
+                             f64 *__restrict__ acc) {
     u32 r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= N) return;
-    u32 id  = sort_index[r];
-    u32 s   = id < n_local ? id : ghost_src[id - n_local];
-    dst[r]  = src[(size_t) s * stride];
+    const u32 id    = sort_index[r];
+    const size_t iv = (size_t) (id < n_local ? id : ghost_src[id - n_local]) * lf.vs;
+    std4(acc, N, 0, r, lf.ax[iv], lf.ay[iv], lf.az[iv], 0.0);
 }
 
 __global__ void k_rank_to_local(u32 n, const u32 *__restrict__ row_rank,
@@ -678,14 +1014,14 @@ __global__ void k_fill(u32 n, f64 *__restrict__ dst, f64 v) {
 cudaError_t h_iterate64(Ctx &c, const RowSpace &rs, const f64 *h_old, f64 *h_new, f64 *eps,
                         f64 pmass, f64 hev, f64 hevi, u32 iters, f64 eps_p) {
     ProfScope ps(c, kProfHIter, rs.n);
-    { k_h_iterate<<<div_up(rs.n, 256), 256, 0, c.stream>>>(rs, h_old, h_new, eps, pmass, hev, hevi,
+    { k_h_iterate<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, h_old, h_new, eps, pmass, hev, hevi,
                                                          iters, eps_p, c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t omega64(Ctx &c, const RowSpace &rs, const f64 *h_row, f64 pmass, f64 *out,
                     const u32 *out_index) {
     ProfScope ps(c, kProfOmega, rs.n);
-    { k_omega<<<div_up(rs.n, 256), 256, 0, c.stream>>>(rs, h_row, pmass, out, out_index); GBSPH_COUNTED; }
+    { k_omega<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, h_row, pmass, out, out_index); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t eos64(Ctx &c, u32 n, const f64 *h, const f64 *u, f64 pmass, f64 gamma, f64 *P, f64 *cs) {
@@ -693,14 +1029,21 @@ cudaError_t eos64(Ctx &c, u32 n, const f64 *h, const f64 *u, f64 pmass, f64 gamm
     return cudaGetLastError();
 }
 cudaError_t gather_eos64(Ctx &c, u32 N, u32 n_local, const LocalFields &lf, const f64 *omega_local,
-                         f64 pmass, const EosParams &eos) {
+                         f64 pmass, const EosParams &eos, f64 alpha_AV) {
+    cudaError_t e;
+    if ((e = c.scs.ensure(sizeof(f64) * (size_t) N, c.stream)) != cudaSuccess) return e;
+    if ((e = c.rec64.ensure(sizeof(f64) * 20 * (size_t) N, c.stream)) != cudaSuccess) return e;
     ProfScope ps(c, kProfGatherEos, N);
     { k_gather_eos<<<div_up(N, 256), 256, 0, c.stream>>>(
         c.sort_index.as<u32>(), N, n_local, c.ghost_src.as<u32>(), lf.h, lf.u, lf.vx, lf.vy, lf.vz,
-        lf.vs, omega_local, pmass, eos, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
-        c.sh2.as<f64>(), c.su.as<f64>(), c.svx.as<f64>(), c.svy.as<f64>(), c.svz.as<f64>(),
-        c.som.as<f64>(), c.sP.as<f64>(), c.scs.as<f64>(), c.srho.as<f64>(), c.sinv.as<f64>(),
-        c.srom.as<f64>()); GBSPH_COUNTED; }
+        lf.vs, omega_local, pmass, eos, alpha_AV, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
+        c.scs.as<f64>(), c.rec64.as<f64>()); GBSPH_COUNTED; }
+    return cudaGetLastError();
+}
+cudaError_t stage_alpha64(Ctx &c, u32 N, u32 n_local, const f64 *alpha_local) {
+    { k_stage_alpha64<<<div_up(N, 256), 256, 0, c.stream>>>(c.sort_index.as<u32>(), N, n_local,
+                                                           c.ghost_src.as<u32>(), alpha_local,
+                                                           c.scs.as<f64>(), c.rec64.as<f64>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t eos_lp07(Ctx &c, u32 n, const f64 *x, const f64 *y, const f64 *z, u32 vs, const f64 *h,
@@ -710,20 +1053,24 @@ cudaError_t eos_lp07(Ctx &c, u32 n, const f64 *x, const f64 *y, const f64 *z, u3
 }
 cudaError_t derivs64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, f64 pmass, f64 alpha_u,
                      f64 alpha_AV, f64 beta_AV, f64 *ax, f64 *ay, f64 *az, f64 *du, f64 *vsig) {
-    DerivParams p{pmass, alpha_u, alpha_AV, beta_AV, 0, 0, 0, ExtAccel{nullptr, nullptr, nullptr}};
-    { k_derivs<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, hs, p, ax, ay, az, du, vsig); GBSPH_COUNTED; }
+    DerivParams p{pmass, alpha_u, beta_AV, 0, 0, 0, ExtAccel{nullptr, nullptr, nullptr}};
+    // the caller's merged arrays hold c.n_obj entries
+    const u32 N   = c.n_obj;
+    cudaError_t e = c.rec64.ensure(sizeof(f64) * 20 * (size_t) N, c.stream);
+    if (e != cudaSuccess) return e;
+    { k_stage_modules<<<div_up(N, 256), 256, 0, c.stream>>>(N, rs.x, rs.y, rs.z, hs, pmass, alpha_AV,
+                                                           c.rec64.as<f64>()); GBSPH_COUNTED; }
+    { k_derivs<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, hs.cs, p, ax, ay, az,
+                                                       du, vsig); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
-cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, f64 pmass, f64 alpha_u,
-                          f64 alpha_AV, f64 beta_AV, f64 hdt, f64 C_cour, f64 C_force,
-                          const LocalFields &lf, const ExtAccel &ext) {
-    DerivParams p{pmass, alpha_u, alpha_AV, beta_AV, hdt, C_cour, C_force, ext};
+cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, u32 N, f64 pmass, f64 alpha_u, f64 beta_AV,
+                          f64 hdt, f64 C_cour, f64 C_force, const LocalFields &lf,
+                          const ExtAccel &ext) {
+    DerivParams p{pmass, alpha_u, beta_AV, hdt, C_cour, C_force, ext};
     ProfScope ps(c, kProfDerivs, rs.n);
-    if (hs.rho && hs.inv_sub && hs.rho_om) {
-        k_derivs_step<true><<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, hs, p, lf, c.d_scalars.as<Scalars>()); GBSPH_COUNTED;
-    } else {
-        k_derivs_step<false><<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, hs, p, lf, c.d_scalars.as<Scalars>()); GBSPH_COUNTED;
-    }
+    { k_derivs_step<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.scs.as<f64>(), p,
+                                                            lf, c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 // leapfrog corrector (integrators.cpp:88-120): v += dt/2 (a_new - a_old), u likewise;
@@ -797,12 +1144,16 @@ cudaError_t predict64(Ctx &c, const LocalFields &lf, u32 n, f64 dt, int periodic
                                                    ext_z); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
-cudaError_t velgrad64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, const f64 *ax,
-                      const f64 *ay, const f64 *az, f64 pmass, f64 *divv, f64 *cx, f64 *cy,
-                      f64 *cz, u32 cvs, f64 *dtdivv) {
+cudaError_t velgrad64(Ctx &c, const RowSpace &rs, u32 N, u32 n_local, const LocalFields &lf, f64 pmass,
+                      f64 *divv, f64 *cx, f64 *cy, f64 *cz, u32 cvs, f64 *dtdivv) {
+    cudaError_t e = c.av_arank.ensure(sizeof(f64) * 4 * (size_t) N, c.stream);
+    if (e != cudaSuccess) return e;
     ProfScope ps(c, kProfVelGrad, rs.n);
-    { k_velgrad64<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, hs, ax, ay, az, pmass, divv, cx, cy,
-                                                         cz, cvs, dtdivv); GBSPH_COUNTED; }
+    { k_gather_acc<<<div_up(N, 256), 256, 0, c.stream>>>(c.sort_index.as<u32>(), N, n_local,
+                                                        c.ghost_src.as<u32>(), lf,
+                                                        c.av_arank.as<f64>()); GBSPH_COUNTED; }
+    { k_velgrad64<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.av_arank.as<f64>(),
+                                                         pmass, divv, cx, cy, cz, cvs, dtdivv); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t cd10_update(Ctx &c, u32 n, const f64 *divv, const f64 *cx, const f64 *cy,
@@ -837,12 +1188,6 @@ cudaError_t conservation64(Ctx &c, const LocalFields &lf, u32 n, f64 pmass, f64 
     const u32 nb = 1024;
     { k_cons_partial<<<nb, kConsBlock, 0, c.stream>>>(lf, n, scratch); GBSPH_COUNTED; }
     { k_cons_final<<<1, 32, 0, c.stream>>>(scratch, nb, pmass, out_dev); GBSPH_COUNTED; }
-    return cudaGetLastError();
-}
-cudaError_t gather_merged64(Ctx &c, u32 N, u32 n_local, const f64 *src, u32 stride, f64 *dst) {
-    { k_gather_merged<<<div_up(N, 256), 256, 0, c.stream>>>(c.sort_index.as<u32>(), N, n_local,
-                                                           c.ghost_src.as<u32>(), src, stride,
-                                                           dst); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t rank_to_local64(Ctx &c, u32 n, const f64 *src_rank, f64 *dst) {

@@ -23,15 +23,9 @@ struct RowSpace {
     const f64 *x, *y, *z;
 };
 
-// Hydro fields in the same index space as the CSR entries.  alpha (optional): the
-// per-particle viscosity of the varying-AV form, else the constant alpha_AV.
+// The module form's hydro fields in the same index space as the CSR entries.
 struct HydroSpace {
     const f64 *h, *u, *vx, *vy, *vz, *omega, *P, *cs;
-    const f64 *alpha;
-    // optional per-particle factors of the FP64 pair loop, computed once by the staging
-    // pass with the pair loop's own expressions (so the same bits): rho_h(m, h),
-    // inv_sat_zero(rho^2 Omega) and rho Omega
-    const f64 *rho, *inv_sub, *rho_om;
 };
 
 // Equation of state of the step: adiabatic (P = (gamma - 1) rho u) or locally
@@ -67,15 +61,20 @@ cudaError_t h_iterate64(Ctx &c, const RowSpace &rs, const f64 *h_old, f64 *h_new
 cudaError_t omega64(Ctx &c, const RowSpace &rs, const f64 *h_row, f64 pmass, f64 *out,
                     const u32 *out_index);
 cudaError_t eos64(Ctx &c, u32 n, const f64 *h, const f64 *u, f64 pmass, f64 gamma, f64 *P, f64 *cs);
+// the corrector's EOS and the FP64 pair loops' records of merged ranks 0..N-1 (c.rec64,
+// c.scs); with a varying viscosity alpha_AV is 1 and stage_alpha64 multiplies the updated
+// per-particle alpha in
 cudaError_t gather_eos64(Ctx &c, u32 N, u32 n_local, const LocalFields &lf, const f64 *omega_local,
-                         f64 pmass, const EosParams &eos);
+                         f64 pmass, const EosParams &eos, f64 alpha_AV);
+cudaError_t stage_alpha64(Ctx &c, u32 N, u32 n_local, const f64 *alpha_local);
 cudaError_t eos_lp07(Ctx &c, u32 n, const f64 *x, const f64 *y, const f64 *z, u32 vs, const f64 *h,
                      f64 pmass, f64 cs0, f64 r0, f64 q, f64 *P, f64 *cs);
 cudaError_t derivs64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, f64 pmass, f64 alpha_u,
                      f64 alpha_AV, f64 beta_AV, f64 *ax, f64 *ay, f64 *az, f64 *du, f64 *vsig);
-cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, f64 pmass, f64 alpha_u,
-                          f64 alpha_AV, f64 beta_AV, f64 hdt, f64 C_cour, f64 C_force,
-                          const LocalFields &lf, const ExtAccel &ext);
+// after gather_eos64 (and stage_alpha64)
+cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, u32 N, f64 pmass, f64 alpha_u, f64 beta_AV,
+                          f64 hdt, f64 C_cour, f64 C_force, const LocalFields &lf,
+                          const ExtAccel &ext);
 // mGM != 0: the central point-mass acceleration (-M G) r / |r|^3 at the drifted
 // positions, before the wrap, into ext_out (AddForceCentralGravPotential.cpp:37-48)
 cudaError_t predict64(Ctx &c, const LocalFields &lf, u32 n, f64 dt, int periodic, const f64 *bmin,
@@ -86,11 +85,10 @@ cudaError_t kdk_correct64(Ctx &c, const LocalFields &lf, u32 n, const f64 *aox, 
 cudaError_t cfl64(Ctx &c, u32 n, const f64 *h, const f64 *vsig, const f64 *ax, const f64 *ay,
                   const f64 *az, u32 avs, f64 C_cour, f64 C_force, f64 *dt_part);
 // varying (Cullen & Dehnen 2010) viscosity, sph64.cu:
-// div v, curl v, d(div v)/dt per pipeline row from rank-ordered fields (hs: h, v, omega;
-// ax..az: the accelerations of the last evaluation), outputs by local id
-cudaError_t velgrad64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, const f64 *ax,
-                      const f64 *ay, const f64 *az, f64 pmass, f64 *divv, f64 *cx, f64 *cy,
-                      f64 *cz, u32 cvs, f64 *dtdivv);
+// div v, curl v, d(div v)/dt per pipeline row after gather_eos64 (lf: the accelerations of
+// the last evaluation), outputs by local id
+cudaError_t velgrad64(Ctx &c, const RowSpace &rs, u32 N, u32 n_local, const LocalFields &lf, f64 pmass,
+                      f64 *divv, f64 *cx, f64 *cy, f64 *cz, u32 cvs, f64 *dtdivv);
 // the switch update of n local particles (UpdateViscosity.cpp:170-215)
 cudaError_t cd10_update(Ctx &c, u32 n, const f64 *divv, const f64 *cx, const f64 *cy,
                         const f64 *cz, u32 cvs, const f64 *dtdivv, const f64 *cs, const f64 *h,
@@ -104,8 +102,6 @@ cudaError_t conservation64(Ctx &c, const LocalFields &lf, u32 n, f64 pmass, f64 
 cudaError_t mm97_update(Ctx &c, u32 n, const f64 *divv, const f64 *cs, const f64 *h,
                         const f64 *alpha, f64 dt, f64 sigma_decay, f64 alpha_min, f64 alpha_max,
                         f64 *alpha_new, bool fp32 = false);
-// dst[r] = src[(merged id of rank r) -> local source] * stride, r < N (ghosts copy their source)
-cudaError_t gather_merged64(Ctx &c, u32 N, u32 n_local, const f64 *src, u32 stride, f64 *dst);
 // dst[row_local[t]] = src[row_rank[t]] for the n pipeline rows
 cudaError_t rank_to_local64(Ctx &c, u32 n, const f64 *src_rank, f64 *dst);
 cudaError_t scatter_rows(Ctx &c, u32 n, const f64 *src, f64 *dst);
