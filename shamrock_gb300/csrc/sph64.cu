@@ -18,6 +18,8 @@
 #include "lean64.cuh"
 #include "sph_kernels.cuh"
 
+#include <algorithm>
+
 namespace gbsph {
 
 namespace {
@@ -62,8 +64,8 @@ __device__ __forceinline__ f64 quarter(f64 v) { return from64(bits64(v) - (2ull 
 __device__ __forceinline__ f64 lean_m4_f(f64 q) {
     f64 t1 = 2 - q;
     f64 t2 = 1 - q;
-    t1     = t1 * t1 * t1;
-    t2     = t2 * t2 * t2;
+    t1     = mul64i(mul64i(t1, t1), t1);
+    t2     = mul64i(mul64i(t2, t2), t2);
     t1     = quarter(t1); // not zero below q = 2
     const u32 hq = hi64(q);
     const f64 t  = t1 - t2;
@@ -72,8 +74,8 @@ __device__ __forceinline__ f64 lean_m4_f(f64 q) {
 __device__ __forceinline__ f64 lean_m4_df(f64 q) {
     const u32 hq  = hi64(q);
     const bool in = hq < 0x3FF00000u;
-    const f64 t = 3 * q, u = t - 3;
-    const f64 s = (in ? 9. / 4. : -3. / 4.) * q * q;
+    const f64 t = mul64i(3.0, q), u = t - 3;
+    const f64 s = mul64i(mul64i(in ? 9. / 4. : -3. / 4., q), q);
     const f64 v = (in ? -t : u) + s;
     return hq < 0x40000000u ? v : 0.0;
 }
@@ -101,6 +103,12 @@ struct RowCut {
     }
 };
 
+// r^2 of a pair inside the band (a call, so that the walk executes its FP64 for those alone)
+__device__ __noinline__ f64 pair_r2(f64 xa, f64 ya, f64 za, f64 xb, f64 yb, f64 zb) {
+    const f64 dx = xa - xb, dy = ya - yb, dz = za - zb;
+    return dx * dx + dy * dy + dz * dz;
+}
+
 // ---------------------------------------------------------------- density sums
 // The pair terms of one row at h_a, with the plain operators
 __device__ __noinline__ void density_pair_plain(f64 rab2, f64 h_a, f64 &w, f64 &dw) {
@@ -125,33 +133,33 @@ __device__ __forceinline__ void density_sums(const RowSpace &rs, u32 a, u32 k0, 
     sumdWdh  = 0;
     u32 k    = k0;
     while (true) {
-        f64 rab2  = 0;
+        f64 xb = 0, yb = 0, zb = 0;
         bool have = false;
         while (k < k1) {
-            const u32 b  = rs.ent[k++];
-            const f64 xb = rs.x[b], yb = rs.y[b], zb = rs.z[b];
+            const u32 b = rs.ent[k++];
+            xb = rs.x[b], yb = rs.y[b], zb = rs.z[b];
             const float r2 = cut.r2(xb, yb, zb);
             if (r2 > cut.thr * cut.hi) continue;
-            const f64 dx = xa - xb, dy = ya - yb, dz = za - zb;
-            rab2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 < cut.thr * cut.lo) && rab2 > dint) continue;
+            if (!(r2 < cut.thr * cut.lo) && pair_r2(xa, ya, za, xb, yb, zb) > dint) continue;
             have = true;
             break;
         }
         if (!__any_sync(0xffffffffu, have)) break;
         if (!have) continue;
+        const f64 dx = xa - xb, dy = ya - yb, dz = za - zb;
+        const f64 rab2 = mul64i(dx, dx) + mul64i(dy, dy) + mul64i(dz, dz);
         bool bad     = false;
         const Root r = root64(rab2, bad);
-        const bool zero = (bits64(rab2) << 1) == 0;
+        const bool zero = zero64(bits64(rab2));
         bad             = bad && !zero;
         const f64 rab = zero ? 0.0 : root_value(r);
         const f64 q   = divide_by(rab, H, bad);
         const f64 f = lean_m4_f(q), df = lean_m4_df(q);
-        f64 w  = divide_by(kNorm3d * f, H3, bad);
-        f64 dw = divide_by(-(kNorm3d) * (3 * f + q * df), H4, bad);
+        f64 w  = divide_by(mul64i(kNorm3d, f), H3, bad);
+        f64 dw = divide_by(mul64i(-(kNorm3d), mul64i(3.0, f) + mul64i(q, df)), H4, bad);
         if (bad) density_pair_plain(rab2, h_a, w, dw);
-        rho_sum += pmass * w;
-        sumdWdh += pmass * dw;
+        rho_sum += mul64i(pmass, w);
+        sumdWdh += mul64i(pmass, dw);
     }
 }
 
@@ -159,7 +167,7 @@ __device__ __forceinline__ void density_sums(const RowSpace &rs, u32 a, u32 k0, 
 // particle: a particle's update reads only its own h, so it iterates until its own
 // eps <= eps_p (1e-6 in the reference), becomes -1, or the iteration cap is reached).
 // The rows of a warp iterate together until the last of them is done.
-__global__ void __launch_bounds__(128) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
+__global__ void __launch_bounds__(128, 8) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
                                                    f64 *__restrict__ h_new, f64 *__restrict__ eps,
                                                    f64 pmass, f64 h_evol_max, f64 h_evol_iter_max,
                                                    u32 iters, f64 eps_p, Scalars *sc) {
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(128) k_h_iterate(RowSpace rs, const f64 *__res
     }
 }
 
-__global__ void __launch_bounds__(128) k_omega(RowSpace rs, const f64 *__restrict__ h_row,
+__global__ void __launch_bounds__(128, 6) k_omega(RowSpace rs, const f64 *__restrict__ h_row,
                                                f64 pmass, f64 *__restrict__ omega_out,
                                                const u32 *__restrict__ out_index) {
     const u32 t      = blockIdx.x * blockDim.x + threadIdx.x;
@@ -359,20 +367,39 @@ struct DerivParams {
     ExtAccel ext;        // external acceleration added to the hydro one (may be null)
 };
 
-// One row's particle, as the pair loop keeps it
+// One row's particle as the pair loop keeps it, in shared memory: four lanes share a row
+// and the loop has no registers to spare (a stride of 25 doubles keeps the eight rows of a
+// warp in different banks)
 struct Row64 {
-    D4 p, v, e; // records 0, 1, 2
+    struct Vec4 {
+        f64 x, y, z, w;
+        __device__ __forceinline__ void operator=(const D4 &d) { x = d.x, y = d.y, z = d.z, w = d.w; }
+    };
+    Vec4 p, v, e; // records 0, 1, 2
     f64 rho, inv_rho_om, c_heat; // rho, 1 / (Omega rho), that times 1 / rho
-    Denominator H, H4;
+    f64 yH, h4, yH4;             // Denominator of h and of h^4
+    float loH, loH4;
+    f64 pad[6];
+    __device__ __forceinline__ Denominator H() const { return Denominator{p.w, yH, loH}; }
+    __device__ __forceinline__ Denominator H4() const { return Denominator{h4, yH4, loH4}; }
 };
-// the pair's contributions and v.r_hat of the forces
+static_assert(sizeof(Row64) == 25 * 8, "Row64 stride");
+
+// the pair's contributions: force, the two du/dt terms, and v.r_hat of the forces
 struct Pair64 {
     f64 fx, fy, fz, t1, t2, vr;
 };
 
+// a pair outside both supports (the exact test, a call for the pairs inside the band)
+__device__ __noinline__ bool beyond_both(f64 xa, f64 ya, f64 za, f64 ha, f64 xb, f64 yb, f64 zb, f64 hb) {
+    const f64 Rker2 = kRkern * kRkern;
+    const f64 r2    = pair_r2(xa, ya, za, xb, yb, zb);
+    return r2 > ha * ha * Rker2 && r2 > hb * hb * Rker2;
+}
+
 // v / 2 where that is exact
 __device__ __forceinline__ f64 half(f64 v, bool &bad) {
-    const bool zero = (bits64(v) << 1) == 0;
+    const bool zero = zero64(bits64(v));
     bad |= !zero && (hi64(v) & 0x7FFFFFFFu) - 0x00200000u >= 0x7FD00000u;
     return zero ? v : from64(bits64(v) - (1ull << 52));
 }
@@ -381,256 +408,343 @@ __device__ __forceinline__ f64 positive(f64 v) {
     return bits64(v) - 1ull < 0x7FF0000000000000ull ? v : 0.0;
 }
 
-// The pair terms with the plain operators (UpdateDerivs.cpp:176-271)
-__device__ __noinline__ void force_pair_plain(const Row64 &A, const D4 &B0, const D4 &B1,
-                                              const D4 &B2, const D4 &B3, const DerivParams &p,
-                                              Pair64 &o) {
-    const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+// (Inlined: ptxas 13.0.88 crashes on these two as calls beside the warp votes of the loop.)
+// The pair terms with the plain operators (UpdateDerivs.cpp:176-271), from the records of a
+// and b
+__device__ __forceinline__ void force_pair_plain(const f64 *__restrict__ rec, size_t N, u32 a, u32 b,
+                                              const DerivParams &p, Pair64 &o) {
+    const D4 A0 = ldd4(rec, N, 0, a), A1 = ldd4(rec, N, 1, a), A2 = ldd4(rec, N, 2, a),
+             A3 = ldd4(rec, N, 3, a);
+    const D4 B0 = ldd4(rec, N, 0, b), B1 = ldd4(rec, N, 1, b), B2 = ldd4(rec, N, 2, b),
+             B3 = ldd4(rec, N, 3, b);
+    const f64 dx = A0.x - B0.x, dy = A0.y - B0.y, dz = A0.z - B0.z;
     const f64 rab = sqrt(dx * dx + dy * dy + dz * dz);
-    f64 Fab_a   = dW_3d(rab, A.p.w);
+    f64 Fab_a   = dW_3d(rab, A0.w);
     f64 Fab_b   = dW_3d(rab, B0.w);
-    f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+    f64 vx = A1.x - B1.x, vy = A1.y - B1.y, vz = A1.z - B1.z;
     f64 inv = inv_sat_positive(rab);
     f64 rx = dx * inv, ry = dy * inv, rz = dz * inv;
     f64 vr      = vx * rx + vy * ry + vz * rz;
     f64 bv      = p.beta_AV * fabs(vr);
-    f64 vsig_a  = A.e.y + bv;
+    f64 vsig_a  = A2.y + bv;
     f64 vsig_b  = B2.y + bv;
-    f64 rho_avg = (A.rho + B3.x) * 0.5;
-    f64 vsig_u  = sqrt(fabs(A.e.x - B2.x) / rho_avg);
-    f64 AV_P_a  = A.e.x + fmax(A.e.z * vsig_a * vr, f64(0));
+    f64 rho_avg = (A3.x + B3.x) * 0.5;
+    f64 vsig_u  = sqrt(fabs(A2.x - B2.x) / rho_avg);
+    f64 AV_P_a  = A2.x + fmax(A2.z * vsig_a * vr, f64(0));
     f64 AV_P_b  = B2.x + fmax(B2.z * vsig_b * vr, f64(0));
-    f64 ca = AV_P_a * A.e.w, cb = AV_P_b * B2.w;
+    f64 ca = AV_P_a * A2.w, cb = AV_P_b * B2.w;
     f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
     f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
     f64 mb = -p.pmass;
     o.fx = mb * (ca * nax + cb * nbx);
     o.fy = mb * (ca * nay + cb * nby);
     o.fz = mb * (ca * naz + cb * nbz);
-    o.t1 = AV_P_a * A.c_heat * p.pmass * (vx * nax + vy * nay + vz * naz);
-    f64 Fa = Fab_a * A.inv_rho_om;
+    const f64 inv_rho_om = 1 / A3.y;
+    o.t1 = AV_P_a * (inv_rho_om * (1. / A3.x)) * p.pmass * (vx * nax + vy * nay + vz * naz);
+    f64 Fa = Fab_a * inv_rho_om;
     f64 Fb = Fab_b / B3.y;
-    o.t2 = p.pmass * p.alpha_u * vsig_u * (A.v.w - B1.w) * f64(0.5) * (Fa + Fb);
+    o.t2 = p.pmass * p.alpha_u * vsig_u * (A1.w - B1.w) * f64(0.5) * (Fa + Fb);
     o.vr = vr;
 }
 
 // v.r_hat of the reference's separate v_sig kernel: r_hat = dr / r, zero below 1e-9
-__device__ __noinline__ f64 sig_speed_plain(const Row64 &A, const D4 &B0, const D4 &B1) {
-    const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
+__device__ __forceinline__ f64 sig_speed_plain(const f64 *__restrict__ rec, size_t N, u32 a, u32 b) {
+    const D4 A0 = ldd4(rec, N, 0, a), A1 = ldd4(rec, N, 1, a);
+    const D4 B0 = ldd4(rec, N, 0, b), B1 = ldd4(rec, N, 1, b);
+    const f64 dx = A0.x - B0.x, dy = A0.y - B0.y, dz = A0.z - B0.z;
     const f64 rab = sqrt(dx * dx + dy * dy + dz * dz);
-    const f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+    const f64 vx = A1.x - B1.x, vy = A1.y - B1.y, vz = A1.z - B1.z;
     f64 ux = dx / rab, uy = dy / rab, uz = dz / rab;
     if (rab < 1e-9) ux = uy = uz = 0;
     return fabs(vx * ux + vy * uy + vz * uz);
 }
 
-// The FP64 pair loop, called by all 32 lanes of a warp (no row: k0 = k1).  It is bound by
-// the FP64 pipe, so as in density_sums a lane first walks to its next pair inside either
-// support in FP32, then all lanes evaluate a pair together from the staged records with the
-// quotients, roots and reciprocals of lean64.cuh: 112 FP64 instructions per pair instead of
-// about 215, none for the quarter of the cached pairs outside both supports and no
-// divergence between the pieces of M4.  The particle itself adds zeros and is skipped
-// unless a field of the row is not finite.
+// The in-support pairs of the rows of a warp, four lanes per row: the quad tests its next
+// four entries in FP32 and queues those inside in entry order until four are there (or the
+// row is done); lane j then holds the j-th.
+struct QuadWalk {
+    u32 k, k1, n, j, q, shift;
+    u32 (*queue)[8];
+    __device__ __forceinline__ QuadWalk(u32 (*queue_)[8], u32 k0, u32 k1_) : k(k0), k1(k1_), n(0), queue(queue_) {
+        const u32 lane = threadIdx.x & 31u;
+        j = lane & 3u, q = lane >> 2, shift = lane & ~3u;
+    }
+    // inside(entry index) for the lane's candidate; false when the warp has no pairs left.
+    // take: pairs of this round; the lane has one (entry index at) if j < take.
+    template<class Inside>
+    __device__ __forceinline__ bool next(Inside &&inside, u32 &take, u32 &at) {
+        while (true) {
+            const bool need = n < 4 && k < k1;
+            if (!__any_sync(0xffffffffu, need)) break;
+            bool in      = false;
+            const u32 kk = k + j;
+            if (need) {
+                if (kk < k1) in = inside(kk);
+                k += 4;
+            }
+            const u32 bits = (__ballot_sync(0xffffffffu, in) >> shift) & 15u;
+            if (in) queue[q][n + __popc(bits & ((1u << j) - 1u))] = kk;
+            n += __popc(bits);
+        }
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, n > 0)) return false;
+        take           = min(n, 4u);
+        at             = queue[q][j];
+        const u32 rest = queue[q][4 + j];
+        __syncwarp();
+        queue[q][j] = rest;
+        n -= take;
+        return true;
+    }
+};
+
+// The FP64 pair loop, called by all 32 lanes of a warp, four to a row (no row: k0 = k1).
+// It is bound by the FP64 pipe (two lanes per clock and SM), so
+//  - a quad first walks to its next pairs inside either support in FP32 and its lanes then
+//    evaluate four of them together: none of the work goes to the quarter of the cached
+//    pairs outside both supports, the pieces of M4 do not diverge and rows of different
+//    lengths leave few lanes idle;
+//  - quotients, roots and reciprocals are those of lean64.cuh, 33 of the 51 products run on
+//    the integer pipes (mul64i; all of them there leaves the FP64 pipe waiting for the
+//    other instructions: 2.04 ms against 1.75), and the neighbour's factors are staged;
+//  - lane c adds component c (x, y, z, du/dt) of the four pairs in entry order.
+// About 95 FP64 instructions per pair, where the plain operators take about 215: 5.12 ->
+// 1.75 ms per launch at 131,072 particles of the jittered lattice.  The
+// particle itself adds zeros and is skipped unless a field of the row is not finite.
 // The v_sig maximum, max over the pairs of c_s + 2 |v.u| with u = dr / r: rounding is
 // monotonic, so that of the largest |v.u|, which differs from the forces' v.r_hat = v.(dr
 // (1/r)) by a few units in the last place of |v|.  The loop keeps the pairs whose |v.r_hat|
 // could be the largest within that margin and evaluates the three quotients for those only
-// (every pair of the row where more than kSigCandidates are that close).
-constexpr u32 kSigCandidates = 12;
+// (every pair of the row where more than kSigCandidates of a lane are that close).
+constexpr u32 kSigCandidates = 8;
+struct Warp64 {
+    Row64 row[8];
+    f64 x[8][4][6]; // [quad][pair]{fx, fy, fz, t1, t2, 0}
+    u32 queue[8][8];
+};
 
 template<bool VSIG>
-__device__ __forceinline__ void derivs_row(const u32 *__restrict__ ent, const f64 *__restrict__ rec,
-                                           size_t N, u32 a, u32 k0, u32 k1, f64 cs_a,
-                                           const DerivParams &p, f64 &fx, f64 &fy, f64 &fz,
-                                           f64 &tdu, f64 &vsig_max) {
-    const f64 Rker2 = kRkern * kRkern;
-    Row64 A;
+__device__ __forceinline__ void derivs_row(Warp64 &W, const u32 *__restrict__ ent,
+                                           const f64 *__restrict__ rec, size_t N, u32 a, u32 k0,
+                                           u32 k1, f64 cs_a, const DerivParams &p, f64 &sum,
+                                           f64 &vsig_max) {
+    QuadWalk walk(W.queue, k0, k1);
+    const u32 j = walk.j, q = walk.q;
+    Row64 &A    = W.row[q];
     bool plain_row;
     {
-        A.p = ldd4(rec, N, 0, a), A.v = ldd4(rec, N, 1, a), A.e = ldd4(rec, N, 2, a);
-        const D4 c = ldd4(rec, N, 3, a), d = ldd4(rec, N, 4, a);
-        A.rho        = c.x;
-        A.inv_rho_om = 1 / c.y;
-        A.c_heat     = A.inv_rho_om * (1. / A.rho);
-        A.H          = Denominator{A.p.w, c.w, low_float(d.z)};
-        A.H4         = Denominator{d.x, d.y, high_float(d.z)};
+        const D4 r0 = ldd4(rec, N, 0, a), r1 = ldd4(rec, N, 1, a), r2 = ldd4(rec, N, 2, a),
+                 r3 = ldd4(rec, N, 3, a), r4 = ldd4(rec, N, 4, a);
+        const f64 iro = 1 / r3.y, heat = iro * (1. / r3.x);
         // a sum is finite only if its terms are (or cancel infinities, which gives NaN)
-        const f64 all = fabs(A.v.x) + fabs(A.v.y) + fabs(A.v.z) + fabs(A.v.w) + fabs(A.e.x)
-                        + fabs(A.e.y) + fabs(A.e.z) + fabs(A.e.w) + fabs(A.c_heat);
-        plain_row = !(all < 1e300) || !(A.H.lo == A.H.lo) || !(A.H4.lo == A.H4.lo);
+        const f64 all = fabs(r1.x) + fabs(r1.y) + fabs(r1.z) + fabs(r1.w) + fabs(r2.x)
+                        + fabs(r2.y) + fabs(r2.z) + fabs(r2.w) + fabs(heat);
+        const float lo = low_float(r4.z), lo4 = high_float(r4.z);
+        plain_row = !(all < 1e300) || !(lo == lo) || !(lo4 == lo4);
+        __syncwarp();
+        if (j == 0) {
+            A.p = r0, A.v = r1, A.e = r2;
+            A.rho = r3.x, A.inv_rho_om = iro, A.c_heat = heat;
+            A.yH = r3.w, A.h4 = r4.x, A.yH4 = r4.y;
+            A.loH = lo, A.loH4 = lo4;
+        }
+        W.x[q][j][5] = 0;
+        __syncwarp();
     }
     const RowCut cut(A.p.x, A.p.y, A.p.z, A.p.w);
-    fx = fy = fz = tdu = 0;
-    float sig_low = -1.f;     // a lower bound of the largest |v.u|
-    u32 sig_n     = 0;        // candidates kept
-    u32 sig_k[kSigCandidates];
+    sum = 0;
+    float sig_low = -1.f; // a lower bound of the lane's largest |v.u|
+    u32 sig_n     = 0;    // candidates kept
+    u32 sig_b[kSigCandidates];
     float sig_up[kSigCandidates];
     bool any_pair = false;
-    u32 k         = k0;
-    while (true) {
-        D4 B0;
-        f64 rab2  = 0;
-        u32 b     = a;
-        bool have = false;
-        while (k < k1) {
-            b  = ent[k++];
-            B0 = ldd4(rec, N, 0, b);
-            const float r2  = cut.r2(B0.x, B0.y, B0.z);
-            const float hb  = cut32(B0.w); // NaN bounds decide nothing
-            const float tm  = hb < 1e18f ? fmaxf(cut.thr, 4.f * hb * hb) : __int_as_float(0x7fc00000);
-            if (r2 > tm * cut.hi) continue;
-            if (b == a && !plain_row) {
-                any_pair = true;
-                continue;
-            }
+    u32 take, at;
+    auto inside = [&](u32 kk) {
+        const u32 b = ent[kk];
+        const D4 B  = ldd4(rec, N, 0, b);
+        const float r2 = cut.r2(B.x, B.y, B.z);
+        const float hb = cut32(B.w); // NaN bounds decide nothing
+        const float tm = hb < 1e18f ? fmaxf(cut.thr, 4.f * hb * hb) : __int_as_float(0x7fc00000);
+        if (r2 > tm * cut.hi) return false;
+        if (b == a && !plain_row) {
+            any_pair = true;
+            return false;
+        }
+        return r2 < tm * cut.lo || !beyond_both(A.p.x, A.p.y, A.p.z, A.p.w, B.x, B.y, B.z, B.w);
+    };
+    while (walk.next(inside, take, at)) {
+        Pair64 o{0, 0, 0, 0, 0, 0};
+        if (j < take) {
+            any_pair    = true;
+            const u32 b = ent[at];
+            const D4 B0 = ldd4(rec, N, 0, b), B1 = ldd4(rec, N, 1, b), B2 = ldd4(rec, N, 2, b),
+                     B3 = ldd4(rec, N, 3, b), B4 = ldd4(rec, N, 4, b);
             const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
-            rab2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 < tm * cut.lo) && rab2 > A.p.w * A.p.w * Rker2 && rab2 > B0.w * B0.w * Rker2)
-                continue;
-            have = true;
-            break;
-        }
-        if (!__any_sync(0xffffffffu, have)) break;
-        if (!have) continue;
-        any_pair    = true;
-        const D4 B1 = ldd4(rec, N, 1, b), B2 = ldd4(rec, N, 2, b), B3 = ldd4(rec, N, 3, b),
-                 B4 = ldd4(rec, N, 4, b);
-        const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
-        bool bad      = plain_row;
-        const Root r  = root64(rab2, bad);
-        const f64 rab = root_value(r);
-        f64 inv       = root_reciprocal(r, bad);
-        if (bits64(rab) < bits64(1e-9)) inv = 0;
-        const Denominator HB{B0.w, B3.w, low_float(B4.z)}, HB4{B4.x, B4.y, high_float(B4.z)},
-            RB{B3.y, B3.z, low_float(B4.w)};
-        const f64 Fab_a = divide_by(kNorm3d * lean_m4_df(divide_by(rab, A.H, bad)), A.H4, bad);
-        const f64 Fab_b = divide_by(kNorm3d * lean_m4_df(divide_by(rab, HB, bad)), HB4, bad);
-        const f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
-        const f64 rx = dx * inv, ry = dy * inv, rz = dz * inv;
-        Pair64 o;
-        o.vr             = vx * rx + vy * ry + vz * rz;
-        const f64 bv     = p.beta_AV * fabs(o.vr);
-        const f64 vsig_a = A.e.y + bv;
-        const f64 vsig_b = B2.y + bv;
-        const f64 dp     = fabs(A.e.x - B2.x);
-        f64 vsig_u       = 0;
-        {
-            bool odd       = false;
-            const f64 sum  = A.rho + B3.x;
-            const f64 q    = quotient64(dp, half(sum, odd), odd);
-            const Root ru  = root64(q, odd);
-            const bool eq  = bits64(dp) == 0; // sqrt(0 / rho) = 0
-            vsig_u         = eq ? 0.0 : root_value(ru);
-            bad |= eq ? !(hi64(sum) - 0x00100000u < 0x7FE00000u) : odd;
-        }
-        const f64 AV_P_a = A.e.x + positive(A.e.z * vsig_a * o.vr);
-        const f64 AV_P_b = B2.x + positive(B2.z * vsig_b * o.vr);
-        const f64 ca = AV_P_a * A.e.w, cb = AV_P_b * B2.w;
-        const f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
-        const f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
-        const f64 mb = -p.pmass;
-        o.fx = mb * (ca * nax + cb * nbx);
-        o.fy = mb * (ca * nay + cb * nby);
-        o.fz = mb * (ca * naz + cb * nbz);
-        o.t1 = AV_P_a * A.c_heat * p.pmass * (vx * nax + vy * nay + vz * naz);
-        const f64 Fa = Fab_a * A.inv_rho_om;
-        const f64 Fb = divide_by(Fab_b, RB, bad);
-        o.t2 = half(p.pmass * p.alpha_u * vsig_u * (A.v.w - B1.w), bad) * (Fa + Fb);
-        if (bad) force_pair_plain(A, B0, B1, B2, B3, p, o);
-        fx += o.fx;
-        fy += o.fy;
-        fz += o.fz;
-        tdu += o.t1;
-        tdu += o.t2;
-        // a pair at rest adds 0 to the maximum
-        if (VSIG && ((bits64(vx) | bits64(vy) | bits64(vz)) << 1) != 0) {
-            const float vf = fabsf(cut32(vx)) + fabsf(cut32(vy)) + fabsf(cut32(vz));
-            const float w  = fabsf(cut32(o.vr)), slack = 3e-7f * w + 1e-14f * vf;
-            // NaN or out of the float range: always a candidate
-            const float up = w + slack < 1e37f ? w + slack : __int_as_float(0x7f800000);
-            if (up >= sig_low) {
-                if (sig_n < kSigCandidates) {
-                    sig_k[sig_n]  = k - 1;
-                    sig_up[sig_n] = up;
-                }
-                sig_n++;
-                if (w - slack > sig_low) {
-                    sig_low = w - slack;
-                    // forget the candidates it overtakes
-                    u32 m = 0;
-                    for (u32 i = 0; i < min(sig_n, kSigCandidates); i++)
-                        if (sig_up[i] >= sig_low) {
-                            sig_k[m]    = sig_k[i];
-                            sig_up[m++] = sig_up[i];
+            const f64 rab2 = mul64i(dx, dx) + mul64i(dy, dy) + mul64i(dz, dz);
+            bool bad       = plain_row;
+            const Root r   = root64(rab2, bad);
+            const f64 rab  = root_value(r);
+            f64 inv        = root_reciprocal(r, bad);
+            if (bits64(rab) < bits64(1e-9)) inv = 0;
+            const f64 Fab_a = divide_by(mul64i(kNorm3d, lean_m4_df(divide_by(rab, A.H(), bad))), A.H4(), bad);
+            const f64 qb    = divide_by(rab, Denominator{B0.w, B3.w, low_float(B4.z)}, bad);
+            const f64 Fab_b = divide_by(mul64i(kNorm3d, lean_m4_df(qb)),
+                                        Denominator{B4.x, B4.y, high_float(B4.z)}, bad);
+            const f64 vx = A.v.x - B1.x, vy = A.v.y - B1.y, vz = A.v.z - B1.z;
+            const f64 rx = mul64i(dx, inv), ry = mul64i(dy, inv), rz = mul64i(dz, inv);
+            o.vr             = mul64i(vx, rx) + mul64i(vy, ry) + mul64i(vz, rz);
+            const f64 bv     = mul64i(p.beta_AV, fabs(o.vr));
+            const f64 vsig_a = A.e.y + bv;
+            const f64 vsig_b = B2.y + bv;
+            const f64 dp     = fabs(A.e.x - B2.x);
+            f64 vsig_u       = 0;
+            {
+                bool odd      = false;
+                const f64 rr  = A.rho + B3.x;
+                const f64 qu  = quotient64(dp, half(rr, odd), odd);
+                const Root ru = root64(qu, odd);
+                const bool eq = zero64(bits64(dp)); // sqrt(0 / rho) = 0
+                vsig_u        = eq ? 0.0 : root_value(ru);
+                bad |= eq ? !(hi64(rr) - 0x00100000u < 0x7FE00000u) : odd;
+            }
+            const f64 AV_P_a = A.e.x + positive(mul64i(mul64i(A.e.z, vsig_a), o.vr));
+            const f64 AV_P_b = B2.x + positive(mul64i(mul64i(B2.z, vsig_b), o.vr));
+            const f64 ca = mul64i(AV_P_a, A.e.w), cb = mul64i(AV_P_b, B2.w);
+            const f64 nax = rx * Fab_a, nay = ry * Fab_a, naz = rz * Fab_a;
+            const f64 nbx = rx * Fab_b, nby = ry * Fab_b, nbz = rz * Fab_b;
+            const f64 mb = -p.pmass;
+            o.fx = mb * (ca * nax + cb * nbx);
+            o.fy = mb * (ca * nay + cb * nby);
+            o.fz = mb * (ca * naz + cb * nbz);
+            o.t1 = mul64i(mul64i(mul64i(AV_P_a, A.c_heat), p.pmass),
+                          vx * nax + vy * nay + vz * naz);
+            const f64 Fa = mul64i(Fab_a, A.inv_rho_om);
+            const f64 Fb = divide_by(Fab_b, Denominator{B3.y, B3.z, low_float(B4.w)}, bad);
+            o.t2 = mul64i(half(mul64i(mul64i(p.pmass * p.alpha_u, vsig_u), A.v.w - B1.w), bad), Fa + Fb);
+            if (bad) force_pair_plain(rec, N, a, b, p, o);
+            // a pair at rest adds 0 to the v_sig maximum
+            if (VSIG && !zero64(bits64(vx) | bits64(vy) | bits64(vz))) {
+                const float vf = fabsf(cut32(vx)) + fabsf(cut32(vy)) + fabsf(cut32(vz));
+                const float w  = fabsf(cut32(o.vr)), slack = 3e-7f * w + 1e-14f * vf;
+                // NaN or out of the float range: always a candidate
+                const float up = w + slack < 1e37f ? w + slack : __int_as_float(0x7f800000);
+                if (up >= sig_low) {
+                    if (w - slack > sig_low) {
+                        sig_low = w - slack;
+                        // forget the candidates it overtakes
+                        if (sig_n <= kSigCandidates) {
+                            u32 m = 0;
+                            for (u32 i = 0; i < sig_n; i++)
+                                if (sig_up[i] >= sig_low) {
+                                    sig_b[m]    = sig_b[i];
+                                    sig_up[m++] = sig_up[i];
+                                }
+                            sig_n = m;
                         }
-                    if (sig_n <= kSigCandidates) sig_n = m;
+                    }
+                    if (sig_n < kSigCandidates) {
+                        sig_b[sig_n]  = b;
+                        sig_up[sig_n] = up;
+                    }
+                    sig_n++;
                 }
             }
         }
+        f64 *x = W.x[q][j];
+        x[0] = o.fx, x[1] = o.fy, x[2] = o.fz, x[3] = o.t1, x[4] = o.t2;
+        __syncwarp();
+#pragma unroll
+        for (u32 s = 0; s < 4; s++) {
+            sum += W.x[q][s][j];
+            sum += W.x[q][s][j == 3 ? 4 : 5];
+        }
+        __syncwarp();
     }
     vsig_max = 0;
-    if (VSIG && any_pair) {
-        f64 vr       = 0;
-        const bool few = sig_n <= kSigCandidates;
-        const u32 n    = few ? sig_n : k1 - k0;
-        for (u32 i = 0; i < n; i++) {
-            const u32 b = ent[few ? sig_k[i] : k0 + i];
-            const D4 B0 = ldd4(rec, N, 0, b);
-            if (!few) {
-                const f64 dx = A.p.x - B0.x, dy = A.p.y - B0.y, dz = A.p.z - B0.z;
-                const f64 d2 = dx * dx + dy * dy + dz * dz;
-                if (d2 > A.p.w * A.p.w * Rker2 && d2 > B0.w * B0.w * Rker2) continue;
+    if (VSIG) {
+        auto quad_max = [](float v) {
+            v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+            return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        };
+        const float low = quad_max(sig_low);
+        f64 vr          = 0;
+        if (__any_sync(0xffffffffu, sig_n > kSigCandidates)) {
+            for (u32 k = k0; k < k1; k++) {
+                const u32 b = ent[k];
+                const D4 B  = ldd4(rec, N, 0, b);
+                if (!beyond_both(A.p.x, A.p.y, A.p.z, A.p.w, B.x, B.y, B.z, B.w))
+                    vr = fmax(vr, sig_speed_plain(rec, N, a, b));
             }
-            vr = fmax(vr, sig_speed_plain(A, B0, ldd4(rec, N, 1, b)));
+        } else {
+            // each lane steps to its next candidate, then all evaluate one
+            for (u32 i = 0; true; i++) {
+                while (i < sig_n && !(sig_up[i] >= low)) i++;
+                if (!__any_sync(0xffffffffu, i < sig_n)) break;
+                if (i < sig_n) vr = fmax(vr, sig_speed_plain(rec, N, a, sig_b[i]));
+            }
         }
-        vsig_max = fmax(vsig_max, 1.0 * cs_a + 2.0 * vr);
+        vr = fmax(vr, __shfl_xor_sync(0xffffffffu, vr, 1));
+        vr = fmax(vr, __shfl_xor_sync(0xffffffffu, vr, 2));
+        const u32 any = (__ballot_sync(0xffffffffu, any_pair) >> walk.shift) & 15u;
+        if (any) vsig_max = fmax(0.0, 1.0 * cs_a + 2.0 * vr);
     }
 }
 
 // module form: reference CSR, outputs a, du (and vsig) by row
-__global__ void __launch_bounds__(128) k_derivs(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+template<bool VSIG>
+__global__ void __launch_bounds__(128, 4) k_derivs(RowSpace rs, const f64 *__restrict__ rec, u32 N,
                                                 const f64 *__restrict__ cs, DerivParams p,
                                                 f64 *__restrict__ ax, f64 *__restrict__ ay,
                                                 f64 *__restrict__ az, f64 *__restrict__ du,
                                                 f64 *__restrict__ vsig) {
-    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ Warp64 W[4];
+    const u32 t = (blockIdx.x * 128 + threadIdx.x) >> 2, j = threadIdx.x & 3u;
     u32 a = 0, k0 = 0, k1 = 0;
     if (t < rs.n) {
         a  = rs.row_rank ? rs.row_rank[t] : t;
         k0 = rs.off[t];
         k1 = k0 + rs.cnt[t];
     }
-    f64 fx, fy, fz, tdu, vm;
-    if (vsig) derivs_row<true>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
-    else derivs_row<false>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
+    f64 sum, vm;
+    derivs_row<VSIG>(W[threadIdx.x >> 5], rs.ent, rec, N, a, k0, k1, cs[a], p, sum, vm);
     if (t >= rs.n) return;
-    ax[t] = fx;
-    ay[t] = fy;
-    az[t] = fz;
-    du[t] = tdu;
-    if (vsig) vsig[t] = vm;
+    (j == 0 ? ax : j == 1 ? ay : j == 2 ? az : du)[t] = sum;
+    if (VSIG && j == 0) vsig[t] = vm;
 }
 
-// pipeline form: derivatives + v_sig + leapfrog corrector + CFL, outputs to the
-// caller's local arrays.  Neighbour velocities come from the staged records
-// taken before the corrector, so correcting the caller's v here is race-free.
-__global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, const f64 *__restrict__ rec, u32 N,
-                                                     const f64 *__restrict__ cs, DerivParams p,
-                                                     LocalFields lf, Scalars *sc) {
-    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 ev2 = 0, dtm = ~0ull;
-    f64 v2  = 0;
+// pipeline form: the sums by rank, {fx, fy, fz, du | v_sig maximum}
+__global__ void __launch_bounds__(128, 4) k_derivs_sums64(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+                                                       const f64 *__restrict__ cs, DerivParams p,
+                                                       f64 *__restrict__ sums, f64 *__restrict__ vmax) {
+    __shared__ Warp64 W[4];
+    const u32 t = (blockIdx.x * 128 + threadIdx.x) >> 2, j = threadIdx.x & 3u;
     u32 a = 0, k0 = 0, k1 = 0;
     if (t < rs.n) {
         a  = rs.row_rank[t];
         k0 = rs.off[t];
         k1 = k0 + rs.cnt[t];
     }
-    f64 fx, fy, fz, tdu, vm;
-    derivs_row<true>(rs.ent, rec, N, a, k0, k1, cs[a], p, fx, fy, fz, tdu, vm);
-    if (t < rs.n) {
-        u32 i  = rs.row_local[t];
-        size_t iv = (size_t) i * lf.vs;
+    f64 sum, vm;
+    derivs_row<true>(W[threadIdx.x >> 5], rs.ent, rec, N, a, k0, k1, cs[a], p, sum, vm);
+    if (t >= rs.n) return;
+    sums[4 * (size_t) a + j] = sum;
+    if (j == 0) vmax[a] = vm;
+}
+
+// leapfrog corrector + CFL from the sums, in the caller's order
+__global__ void __launch_bounds__(256) k_correct64(u32 n, const u32 *__restrict__ rank_of,
+                                                   const f64 *__restrict__ sums,
+                                                   const f64 *__restrict__ vmax, DerivParams p,
+                                                   LocalFields lf, Scalars *sc) {
+    u64 ev2 = 0, dtm = ~0ull;
+    f64 v2  = 0;
+    for (u32 i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const u32 r  = rank_of[i];
+        const D4 S   = ldd4(sums, 0, 0, r);
+        const f64 vm = vmax[r];
+        f64 fx = S.x, fy = S.y, fz = S.z;
+        const f64 tdu   = S.w;
+        const size_t iv = (size_t) i * lf.vs;
         if (p.ext.x) {
             // axyz += axyz_ext (ExternalForces.cpp:342-359)
             fx = fx + p.ext.x[i];
@@ -650,17 +764,19 @@ __global__ void __launch_bounds__(128) k_derivs_step(RowSpace rs, const f64 *__r
         lf.vz[iv] = nvz;
         f64 iu    = p.hdt * (tdu - odu);
         lf.u[i]   = lf.u[i] + iu;
-        ev2       = f64_to_ordered(ix * ix + iy * iy + iz * iz);
-        v2        = nvx * nvx + nvy * nvy + nvz * nvz;
+        const u64 e = f64_to_ordered(ix * ix + iy * iy + iz * iz);
+        ev2         = e > ev2 ? e : ev2;
+        v2 += nvx * nvx + nvy * nvy + nvz * nvz;
         // CFL with the new acceleration
-        f64 h_a  = rec[4 * (size_t) a + 3];
+        f64 h_a  = lf.h[i];
         f64 dt   = __longlong_as_double(0x7ff0000000000000ll);
         f64 dt_c = p.C_cour * h_a / vm;
         dt       = fmin(dt, dt_c);
         f64 abs_a = sqrt(fx * fx + fy * fy + fz * fz);
         f64 dt_f  = p.C_force * sqrt(h_a / abs_a);
         dt        = fmin(dt, dt_f);
-        dtm       = f64_to_ordered(dt);
+        const u64 d = f64_to_ordered(dt);
+        dtm         = d < dtm ? d : dtm;
     }
     ev2 = block_reduce(ev2, OpMaxU64{}, 0ull);
     dtm = block_reduce(dtm, OpMinU64{}, ~0ull);
@@ -819,83 +935,124 @@ __device__ __noinline__ void gradient_pair_plain(const f64 r[3], f64 rab2, f64 h
     F = dW_3d(rab, h_a);
 }
 
-// Bound by the FP64 pipe like the loops above and arranged like them.  Pairs beyond 2 h_a
+// Bound by the FP64 pipe like the loop above and arranged like it.  Pairs beyond 2 h_a
 // (inside the neighbour's support only) have F = 0 and add zeros, so those that the FP32
-// test finds outside are not evaluated.  acc: records {ax, ay, az, -} of the last evaluation.
-__global__ void __launch_bounds__(128) k_velgrad64(RowSpace rs, const f64 *__restrict__ rec, u32 N,
+// test finds outside are not evaluated.  Each lane of a quad evaluates a pair; lane 0 then
+// adds R, lane 1 Dv, lane 2 Da (the same nine products with r, v or w) and lane 3 div and
+// curl, in entry order, and lane 0 collects them.  acc: records {ax, ay, az, -} of the last
+// evaluation.
+constexpr int kVgTerms = 19; // {r, v, w (9), curl terms (3), div term, 0 | m g (3), -1}, padded
+struct WarpVg64 {
+    f64 z[8][4][kVgTerms]; // [quad][pair]
+    u32 queue[8][8];
+};
+
+__global__ void __launch_bounds__(128, 4) k_velgrad64(RowSpace rs, const f64 *__restrict__ rec, u32 N,
                                                    const f64 *__restrict__ acc, f64 pmass,
                                                    f64 *__restrict__ divv, f64 *__restrict__ cx,
                                                    f64 *__restrict__ cy, f64 *__restrict__ cz,
                                                    u32 cvs, f64 *__restrict__ dtdivv) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ WarpVg64 Ws[4];
+    WarpVg64 &W = Ws[threadIdx.x >> 5];
+    const u32 t = (blockIdx.x * 128 + threadIdx.x) >> 2;
     u32 a = 0, k0 = 0, k1 = 0;
     if (t < rs.n) {
         a  = rs.row_rank[t];
         k0 = rs.off[t];
         k1 = k0 + rs.cnt[t];
     }
-    const f64 Rker2 = kRkern * kRkern;
+    QuadWalk walk(W.queue, k0, k1);
+    const u32 j = walk.j, q = walk.q;
     const D4 A0 = ldd4(rec, N, 0, a), A1 = ldd4(rec, N, 1, a), A3 = ldd4(rec, N, 3, a),
              A4 = ldd4(rec, N, 4, a), Aa = ldd4(acc, N, 0, a);
     const f64 h_a = A0.w;
     const Denominator H{h_a, A3.w, low_float(A4.z)}, H4{A4.x, A4.y, high_float(A4.z)};
-    const f64 inv_rho_omega_a = 1. / A3.y; // 1 / (Omega rho)
     const RowCut cut(A0.x, A0.y, A0.z, h_a);
     const bool plain_row = !(fabs(A1.x) + fabs(A1.y) + fabs(A1.z) + fabs(Aa.x) + fabs(Aa.y) + fabs(Aa.z) < 1e300)
                            || !(H.lo == H.lo) || !(H4.lo == H4.lo);
-    f64 sdiv = 0, sc[3] = {0, 0, 0};
-    f64 R[3][3] = {}, Dv[3][3] = {}, Da[3][3] = {};
-    u32 k = k0;
-    while (true) {
-        f64 r[3]  = {0, 0, 0}, rab2 = 0;
-        u32 b     = a;
-        bool have = false;
-        while (k < k1) {
-            b           = rs.ent[k++];
-            const D4 B0 = ldd4(rec, N, 0, b);
-            const float r2 = cut.r2(B0.x, B0.y, B0.z);
-            if (!plain_row && (r2 > cut.thr * cut.hi || b == a)) continue;
-            r[0] = A0.x - B0.x;
-            r[1] = A0.y - B0.y;
-            r[2] = A0.z - B0.z;
-            rab2 = (r[0] * r[0] + r[1] * r[1]) + r[2] * r[2];
-            if (!(r2 < cut.thr * cut.lo) && rab2 > h_a * h_a * Rker2 && rab2 > B0.w * B0.w * Rker2)
-                continue;
-            have = true;
-            break;
+    f64 S[8] = {};
+    W.z[q][j][13] = 0.0;
+    W.z[q][j][17] = -1.0;
+    auto inside = [&](u32 kk) {
+        const u32 b    = rs.ent[kk];
+        const D4 B     = ldd4(rec, N, 0, b);
+        const float r2 = cut.r2(B.x, B.y, B.z);
+        if (!plain_row && (r2 > cut.thr * cut.hi || b == a)) return false;
+        return r2 < cut.thr * cut.lo || !beyond_both(A0.x, A0.y, A0.z, A0.w, B.x, B.y, B.z, B.w);
+    };
+    u32 take, at;
+    while (walk.next(inside, take, at)) {
+        f64 r[3] = {0, 0, 0}, v[3] = {0, 0, 0}, w[3] = {0, 0, 0}, mg[3] = {0, 0, 0}, cu[3] = {0, 0, 0}, dv = 0;
+        if (j < take) {
+            const u32 b = rs.ent[at];
+            const D4 B0 = ldd4(rec, N, 0, b), B1 = ldd4(rec, N, 1, b), Ba = ldd4(acc, N, 0, b);
+            r[0] = A0.x - B0.x, r[1] = A0.y - B0.y, r[2] = A0.z - B0.z;
+            v[0] = A1.x - B1.x, v[1] = A1.y - B1.y, v[2] = A1.z - B1.z;
+            w[0] = Aa.x - Ba.x, w[1] = Aa.y - Ba.y, w[2] = Aa.z - Ba.z;
+            const f64 rab2  = (mul64i(r[0], r[0]) + mul64i(r[1], r[1])) + mul64i(r[2], r[2]);
+            bool bad        = plain_row;
+            const Root root = root64(rab2, bad);
+            const f64 rab   = root_value(root);
+            Denominator D{rab, 0, 0.f};
+            root_reciprocal(root, bad, D.y, D.lo);
+            bad |= bits64(rab) < bits64(1e-9);
+            f64 e[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) e[c] = divide_by(r[c], D, bad);
+            f64 F = divide_by(mul64i(kNorm3d, lean_m4_df(divide_by(rab, H, bad))), H4, bad);
+            if (bad) gradient_pair_plain(r, rab2, h_a, e, F);
+            const f64 g[3] = {mul64i(F, e[0]), mul64i(F, e[1]), mul64i(F, e[2])};
+            dv    = mul64i(pmass, (mul64i(v[0], g[0]) + mul64i(v[1], g[1])) + mul64i(v[2], g[2]));
+            cu[0] = mul64i(pmass, mul64i(v[1], g[2]) - mul64i(v[2], g[1]));
+            cu[1] = mul64i(pmass, mul64i(v[2], g[0]) - mul64i(v[0], g[2]));
+            cu[2] = mul64i(pmass, mul64i(v[0], g[1]) - mul64i(v[1], g[0]));
+#pragma unroll
+            for (int c = 0; c < 3; c++) mg[c] = mul64i(g[c], pmass);
         }
-        if (!__any_sync(0xffffffffu, have)) break;
-        if (!have) continue;
-        const D4 B1 = ldd4(rec, N, 1, b), Ba = ldd4(acc, N, 0, b);
-        const f64 v[3] = {A1.x - B1.x, A1.y - B1.y, A1.z - B1.z};
-        const f64 w[3] = {Aa.x - Ba.x, Aa.y - Ba.y, Aa.z - Ba.z};
-        bool bad        = plain_row;
-        const Root root = root64(rab2, bad);
-        const f64 rab   = root_value(root);
-        Denominator D{rab, 0, 0.f};
-        root_reciprocal(root, bad, D.y, D.lo);
-        bad |= bits64(rab) < bits64(1e-9);
-        f64 e[3];
+        f64 *z = W.z[q][j];
 #pragma unroll
-        for (int c = 0; c < 3; c++) e[c] = divide_by(r[c], D, bad);
-        f64 F = divide_by(kNorm3d * lean_m4_df(divide_by(rab, H, bad)), H4, bad);
-        if (bad) gradient_pair_plain(r, rab2, h_a, e, F);
-        const f64 g[3] = {F * e[0], F * e[1], F * e[2]};
-        sdiv  = sdiv + pmass * ((v[0] * g[0] + v[1] * g[1]) + v[2] * g[2]);
-        sc[0] = sc[0] + pmass * (v[1] * g[2] - v[2] * g[1]);
-        sc[1] = sc[1] + pmass * (v[2] * g[0] - v[0] * g[2]);
-        sc[2] = sc[2] + pmass * (v[0] * g[1] - v[1] * g[0]);
-        const f64 mg[3] = {g[0] * pmass, g[1] * pmass, g[2] * pmass};
+        for (int c = 0; c < 3; c++) {
+            z[c]      = r[c];
+            z[3 + c]  = v[c];
+            z[6 + c]  = w[c];
+            z[9 + c]  = cu[c];
+            z[14 + c] = mg[c];
+        }
+        z[12] = dv;
+        __syncwarp();
+        // S = S - u (m g): lanes 0-2 the entries (i, jj) of their matrix but the last, lane 3
+        // the three last ones and the curl and div terms (times -1)
+        for (u32 s = 0; s < take; s++) {
+            const f64 *zs = W.z[q][s];
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                R[i][j]  = R[i][j] - r[i] * mg[j];
-                Dv[j][i] = Dv[j][i] - v[i] * mg[j];
-                Da[j][i] = Da[j][i] - w[i] * mg[j];
+            for (int m = 0; m < 8; m++) {
+                const f64 u  = zs[j < 3 ? 3 * j + m / 3 : (m < 3 ? 3 * m + 2 : 6 + m)];
+                const f64 gg = zs[j < 3 ? 14 + m % 3 : (m < 3 ? 16 : 17)];
+                S[m]         = S[m] - mul64i(u, gg);
             }
+        }
+        __syncwarp();
     }
-    if (t >= rs.n) return;
+    // the quad's sums through shared memory to its first lane
+    f64 *out = &W.z[q][0][0];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 8; m++) out[8 * j + m] = S[m];
+    __syncwarp();
+    if (t >= rs.n || j != 0) return;
+    const f64 inv_rho_omega_a = 1. / A3.y; // 1 / (Omega rho)
+    f64 R[3][3], Dv[3][3], Da[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int jj = 0; jj < 3; jj++) {
+            const int m = 3 * i + jj;
+            R[i][jj]    = out[m < 8 ? m : 24];
+            Dv[jj][i]   = out[m < 8 ? 8 + m : 25];
+            Da[jj][i]   = out[m < 8 ? 16 + m : 26];
+        }
+    const f64 sc[3] = {out[27], out[28], out[29]};
+    const f64 sdiv  = out[30];
     const u32 i = rs.row_local[t];
     divv[i]     = -inv_rho_omega_a * sdiv;
     cx[(size_t) i * cvs] = -inv_rho_omega_a * sc[0];
@@ -1060,8 +1217,9 @@ cudaError_t derivs64(Ctx &c, const RowSpace &rs, const HydroSpace &hs, f64 pmass
     if (e != cudaSuccess) return e;
     { k_stage_modules<<<div_up(N, 256), 256, 0, c.stream>>>(N, rs.x, rs.y, rs.z, hs, pmass, alpha_AV,
                                                            c.rec64.as<f64>()); GBSPH_COUNTED; }
-    { k_derivs<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, hs.cs, p, ax, ay, az,
-                                                       du, vsig); GBSPH_COUNTED; }
+    auto kern = vsig ? k_derivs<true> : k_derivs<false>;
+    { kern<<<div_up(rs.n, 32), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, hs.cs, p, ax, ay, az, du,
+                                                  vsig); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, u32 N, f64 pmass, f64 alpha_u, f64 beta_AV,
@@ -1069,8 +1227,13 @@ cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, u32 N, f64 pmass, f64 alph
                           const ExtAccel &ext) {
     DerivParams p{pmass, alpha_u, beta_AV, hdt, C_cour, C_force, ext};
     ProfScope ps(c, kProfDerivs, rs.n);
-    { k_derivs_step<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.scs.as<f64>(), p,
-                                                            lf, c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
+    cudaError_t e = c.f_sums.ensure(sizeof(f64) * 5 * (size_t) N, c.stream);
+    if (e != cudaSuccess) return e;
+    f64 *sums = c.f_sums.as<f64>(), *vmax = sums + 4 * (size_t) N;
+    { k_derivs_sums64<<<div_up(rs.n, 32), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.scs.as<f64>(), p,
+                                                             sums, vmax); GBSPH_COUNTED; }
+    { k_correct64<<<std::min(div_up(rs.n, 256), 6 * c.sms), 256, 0, c.stream>>>(
+        rs.n, c.rank_of.as<u32>(), sums, vmax, p, lf, c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 // leapfrog corrector (integrators.cpp:88-120): v += dt/2 (a_new - a_old), u likewise;
@@ -1152,7 +1315,7 @@ cudaError_t velgrad64(Ctx &c, const RowSpace &rs, u32 N, u32 n_local, const Loca
     { k_gather_acc<<<div_up(N, 256), 256, 0, c.stream>>>(c.sort_index.as<u32>(), N, n_local,
                                                         c.ghost_src.as<u32>(), lf,
                                                         c.av_arank.as<f64>()); GBSPH_COUNTED; }
-    { k_velgrad64<<<div_up(rs.n, 128), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.av_arank.as<f64>(),
+    { k_velgrad64<<<div_up(rs.n, 32), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.av_arank.as<f64>(),
                                                          pmass, divv, cx, cy, cz, cvs, dtdivv); GBSPH_COUNTED; }
     return cudaGetLastError();
 }

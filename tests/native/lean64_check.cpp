@@ -45,6 +45,8 @@ static void all(double a, double b) {
     bad = false;
     const double q = divide_by(a, denominator(b), bad);
     expect(q, a / b, bad);
+    expect(mul64i(a, b), a * b, false);
+    expect(mul64i(-a, b), -a * b, false);
     const float c = cut32(a);
     if (std::fabs(a) >= 1.2e-38 && std::fabs(a) < 3.4e38) {
         checks++;
