@@ -69,7 +69,7 @@ Ctx::~Ctx() {
                       &offsets, &reduc, &reduced, &radix_k, &radix_v, &radix_hist, &radix_off, &lchild, &rchild, &lflag, &rflag, &endrange,
                       &parent, &boxes, &visit, &fboxes, &fpairs, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
                       &row_local, &row_flags, &row_offsets, &leaf_cnt, &leaf_off, &leaf_ent,
-                      &owner, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
+                      &leaf_head, &next_row, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
                       &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &scs, &rec64,
                       &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
                       &h_old_row, &eps_row, &omega_local, &a_old, &du_old, &hnew_row, &omega_row,
@@ -406,12 +406,10 @@ int gbsph_neighbour_cache(gbsph_ctx *ctx, uint32_t n_local, double htol, uint32_
     REQUIRE_ARG(precision == GBSPH_FP64 || precision == GBSPH_MIXED, "unknown precision");
     CU(cudaMemsetAsync(c.d_scalars.p, 0, sizeof(Scalars), c.stream));
     CU(build_rows(c, n_local));
-    if (precision == GBSPH_MIXED) {
-        CU(stage_positions_mixed(c, c.n_obj, htol));
-        CU(neigh_cache_build(c, htol, mixed_positions(c)));
-    } else {
-        CU(neigh_cache_build(c, htol));
-    }
+    // both precisions pre-test the pairs in FP32 (exact FP64 test inside the rounding band):
+    // the cache is the same
+    CU(stage_positions_mixed(c, c.n_obj, htol));
+    CU(neigh_cache_build(c, htol, mixed_positions(c)));
     CU(cudaStreamSynchronize(c.stream));
     return GBSPH_OK;
 }

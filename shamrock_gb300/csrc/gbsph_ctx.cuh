@@ -134,7 +134,7 @@ struct Ctx {
     u32 row_seen = 0;              // largest stage-2 row of the last build
     u64 slot_budget = 0;            // bytes of one-pass slots allowed (0: library default)
     DevBuf leaf_cnt, leaf_off, leaf_ent; // stage 1 (leaf ids)
-    DevBuf owner;                        // per row: leaf index
+    DevBuf leaf_head, next_row;          // the rows each leaf owns, linked
     DevBuf leaf_thr;                     // per leaf: FP32 bits of max thr over its owned rows
     DevBuf csr_cnt, csr_off, csr_ent;    // stage 2, per row, entries are ranks
     u32 n_local = 0;
@@ -212,9 +212,9 @@ cudaError_t sync_scalars(Ctx &c);            // copy Scalars to pinned host, wai
 
 // neigh.cu
 cudaError_t build_rows(Ctx &c, u32 n_local);
-// P: optional FP32 position records (2 float4 per rank: hi + 1/h, lo + fl32(thr));
-// when given, candidate pairs are pre-tested in FP32 (same resulting cache).
-cudaError_t neigh_cache_build(Ctx &c, f64 h_tolerance, const float4 *P = nullptr);
+// P: FP32 position records (2 float4 per rank: hi + 1/h, lo + fl32(thr)): candidate pairs
+// are pre-tested in FP32 and decided in FP64 inside the rounding band.
+cudaError_t neigh_cache_build(Ctx &c, f64 h_tolerance, const float4 *P);
 cudaError_t tree_query(Ctx &c, const f64 *qx, const f64 *qy, const f64 *qz, u32 nq, int mode,
                        f64 s, u32 *counts, u32 *offsets, u32 *out, bool fill);
 

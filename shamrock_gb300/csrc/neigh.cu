@@ -16,6 +16,7 @@
 #include "gbsph_ctx.cuh"
 #include "split64.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <type_traits>
@@ -317,7 +318,8 @@ __global__ void k_rows(const u32 *__restrict__ sort_index, const u8 *__restrict_
 // i.e. the last leaf the reference's left-first DFS reports (NeighbourCache.cpp:419-443).
 // Right-first traversal over the child-pair records (the first leaf reached is the
 // largest); containment is decided in FP32 outside a rounding band, else in FP64.
-// leaf_thr (optional): per leaf, the FP32 bits (rounded up) of the largest pair-test
+// The rows of a leaf are linked: head[leaf], then next_row[row] (their order does not matter).
+// leaf_thr: per leaf, the FP32 bits (rounded up) of the largest pair-test
 // threshold thr_a = ((h_a htol)^2) R^2 over the rows it owns, 0 for a leaf owning none.
 // The exact containment test inside the FP32 band compares the doubles' ordered bit
 // patterns with integer operations (the FP64 pipe is scarce on GB300; particles lie on
@@ -332,8 +334,8 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
                                                const NodePairF *__restrict__ rec,
                                                const u32 *__restrict__ row_rank, u32 n_rows,
                                                const f64 *__restrict__ sx, const f64 *__restrict__ sy,
-                                               const f64 *__restrict__ sz, u32 *__restrict__ owner,
-                                               u32 *__restrict__ flags, const f64 *__restrict__ sh,
+                                               const f64 *__restrict__ sz, u32 *__restrict__ head,
+                                               u32 *__restrict__ next_row, u32 *__restrict__ flags, const f64 *__restrict__ sh,
                                                float h_tol_up, u32 *__restrict__ leaf_thr) {
     u32 row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n_rows) return;
@@ -380,16 +382,16 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         if (cr) stack[top++] = ri;
     }
     if (found == kNone) {
-        atomicOr(flags, kFlagOwnerMissing);
+        atomicOr(flags, kFlagOwnerMissing); // the build stops at its next sync
         found = 0;
-    } else if (leaf_thr) {
+    } else {
         // an FP32 upper bound of thr_a = fl64(fl64(h htol)^2 R^2): every factor rounded up
         // (a float at or above a real number is at or above its nearest double)
         const float rint = __fmul_ru(__double2float_ru(sh[r]), h_tol_up);
         const float thr  = __fmul_ru(__fmul_ru(rint, rint), (float) (kRkern * kRkern));
         atomicMax(&leaf_thr[found], __float_as_uint(thr));
     }
-    owner[row] = found;
+    next_row[row] = atomicExch(&head[found], row);
 }
 
 // ---- stage 2 (NeighbourCache.cpp:492-591)
@@ -399,102 +401,176 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // overflows so the host reruns the two-pass build.  Either way every row starts on a
 // 16-byte boundary, so readers may fetch entries four at a time.
 //
-// F32: the pair test is r^2 <= max(thr_a, thr_b), thr = ((h htol)^2) R^2 in FP64.  r^2
-// is estimated in FP32 from hi/lo-split positions (relative error below ~3e-7) and
-// compared with the FP32 rounding of max(thr_a, thr_b) carried in the position record;
-// outside a +-1e-5 relative band the answer is certain, inside it the exact FP64 test
-// decides.  The cache is therefore identical to the FP64 one.
+// The pair test is r^2 <= max(thr_a, thr_b), thr = ((h htol)^2) R^2 in FP64.  r^2 is
+// estimated in FP32 and compared with the FP32 rounding of max(thr_a, thr_b) carried in the
+// position records; outside a +-1e-5 relative band the answer is certain, inside it the
+// exact FP64 test decides, so the cache is the FP64 one.
+//
+// A warp walks one leaf: the rows that the leaf owns share its candidates, so the warp
+// expands the leaf's rank runs once, loads each candidate's record once, coalesced, and
+// keeps its position relative to the leaf in shared memory; a row is then tested against 32
+// candidates at a time and the accepted lanes are placed by a ballot, in rank order.  Bound
+// by instruction issue (about 60 a row and 32 candidates); a thread per row loads a record
+// per candidate and row, 10 L1 wavefronts a request, its lanes diverge over runs of
+// different lengths, and a state of 2,048 particles runs on 64 warps: 104 -> 18 us there,
+// 131,072 particles 181 -> 138 us, 1,048,576 1000 -> 875 us, disc 1146 -> 916 us,
+// homogeneous 8.5 M 5.57 -> 5.36 ms.  Relative positions are rounded to FP32:
+// with S the largest of the rows' own, r^2 / thr of a pair near the threshold errs by at
+// most 2.1e-7 (2 S / sqrt(thr) + 2), and the hi/lo records themselves by 2.5e-14 M /
+// sqrt(thr) for coordinates of size M; a row for which these do not stay well inside the
+// band takes the FP64 test for every candidate.
 enum CacheMode { kCount = 0, kFill = 1, kOnePass = 2 };
 
-template<int MODE, bool F32>
-__global__ void __launch_bounds__(256) k_part_cache(
-    const u32 *__restrict__ row_rank, u32 n_rows, const u32 *__restrict__ owner,
-    const u32 *__restrict__ leaf_cnt, const u32 *__restrict__ leaf_off,
-    const uint2 *__restrict__ leaf_ent, const float4 *__restrict__ P,
-    const f64 *__restrict__ sx, const f64 *__restrict__ sy, const f64 *__restrict__ sz,
-    const f64 *__restrict__ sh, f64 h_tol, u32 *__restrict__ cnt, u32 *__restrict__ off,
-    u32 *__restrict__ ent, Scalars *sc, u32 cap) {
-    u32 row = blockIdx.x * blockDim.x + threadIdx.x;
-    u32 c   = 0;
-    if (row < n_rows) {
-        u32 ra     = row_rank[row];
-        f64 xa     = sx[ra], ya = sy[ra], za = sz[ra];
-        f64 rint_a = __dmul_rn(sh[ra], h_tol);
-        f64 thr_a  = __dmul_rn(__dmul_rn(rint_a, rint_a), kRkern * kRkern);
-        float4 Aa = make_float4(0, 0, 0, 0), Ba = Aa;
-        if (F32) {
-            F8 pa = ldg256(&P[2 * (size_t) ra]);
-            Aa    = pa.a;
-            Ba    = pa.b;
-        }
-        const float lo_f = 1.f - 1e-5f, hi_f = 1.f + 1e-5f;
-        u32 leaf = owner[row];
-        u32 k0 = leaf_off[leaf], k1 = k0 + leaf_cnt[leaf];
-        u32 w = (MODE == kFill) ? off[row] : ((MODE == kOnePass) ? row * cap : 0);
-        // one flat loop over the row's candidates (rows of a warp with different owner
-        // leaves then stay converged); the next range is fetched one range ahead
-        uint2 g  = (k0 < k1) ? leaf_ent[k0] : make_uint2(0, 0);
-        u32 k    = k0 + 1;
-        uint2 gn = (k < k1) ? leaf_ent[k] : g;
-        u32 rb   = g.x;
-        bool more = true;
-        while (true) {
-            while (rb >= g.y) {
-                if (k >= k1) {
-                    more = false;
-                    break;
-                }
-                g  = gn;
-                rb = g.x;
-                k++;
-                if (k < k1) gn = leaf_ent[k];
+// the exact test (NeighbourCache.cpp:492-591); a call, as few candidates need it
+__device__ __noinline__ bool pair_inside(const f64 *__restrict__ sx, const f64 *__restrict__ sy,
+                                         const f64 *__restrict__ sz, const f64 *__restrict__ sh,
+                                         f64 h_tol, u32 a, u32 b) {
+    const f64 dx = __dsub_rn(sx[a], sx[b]), dy = __dsub_rn(sy[a], sy[b]), dz = __dsub_rn(sz[a], sz[b]);
+    const f64 rab2   = dot3_rn(dx, dy, dz);
+    const f64 rint_a = __dmul_rn(sh[a], h_tol), rint_b = __dmul_rn(sh[b], h_tol);
+    const f64 thr_a  = __dmul_rn(__dmul_rn(rint_a, rint_a), kRkern * kRkern);
+    const f64 thr_b  = __dmul_rn(__dmul_rn(rint_b, rint_b), kRkern * kRkern);
+    return !(rab2 > thr_a && rab2 > thr_b);
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+constexpr u32 kCandBlock = 256; // candidates of a leaf held at a time
+
+template<int MODE>
+__global__ void __launch_bounds__(256, 5) k_part_cache(
+    u32 L, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
+    const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
+    const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
+    const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
+    const f64 *__restrict__ sz, const f64 *__restrict__ sh, f64 h_tol, u32 *__restrict__ cnt,
+    u32 *__restrict__ off, u32 *__restrict__ ent, Scalars *sc, u32 cap) {
+    __shared__ float4 s_cand[8][kCandBlock];
+    __shared__ u32 s_id[8][kCandBlock];
+    const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const u32 below = (1u << lane) - 1u, upto = below | (1u << lane);
+    constexpr u32 kAll = 0xffffffffu;
+    float4 *cand = s_cand[wid];
+    u32 *ids     = s_id[wid];
+    const float lo_f = 1.f - 1e-5f, band = (1.f + 1e-5f) / (1.f - 1e-5f);
+    u32 c_max = 0;
+    u64 c_sum = 0;
+    for (u32 l = blockIdx.x * 8 + wid; l < L; l += gridDim.x * 8) {
+        u32 cur      = head[l];
+        const u32 k0 = leaf_off[l], nk = leaf_cnt[l];
+        while (cur != kNone) {
+            // the next 32 rows at most, a lane each
+            u32 row = kNone, m = 0;
+            while (m < 32 && cur != kNone) {
+                if (lane == m) row = cur;
+                cur = next_row[cur];
+                m++;
             }
-            if (!more) break;
+            u32 ra = 0, w = 0, c = 0;
+            float4 Ph = make_float4(0, 0, 0, 0), Pl = Ph;
+            if (lane < m) {
+                ra           = row_rank[row];
+                const F8 rec = ldg256(&P[2 * (size_t) ra]);
+                Ph = rec.a, Pl = rec.b;
+                w = (MODE == kFill) ? off[row] : ((MODE == kOnePass) ? row * cap : 0);
+            }
+            const float ox = __shfl_sync(kAll, Ph.x, 0), oy = __shfl_sync(kAll, Ph.y, 0),
+                        oz = __shfl_sync(kAll, Ph.z, 0);
+            const float xa = __fadd_rn(__fsub_rn(Ph.x, ox), Pl.x), ya = __fadd_rn(__fsub_rn(Ph.y, oy), Pl.y),
+                        za = __fadd_rn(__fsub_rn(Ph.z, oz), Pl.z), thr = Pl.w;
+            float tlo; // the lower end of the band; NaN: decide in FP64
             {
-                int decided = -1;
-                if (F32) {
-                    F8 pb = ldg256(&P[2 * (size_t) rb]);
-                    const float4 Ab = pb.a, Bb = pb.b;
-                    float dx = __fadd_rn(__fsub_rn(Aa.x, Ab.x), __fsub_rn(Ba.x, Bb.x));
-                    float dy = __fadd_rn(__fsub_rn(Aa.y, Ab.y), __fsub_rn(Ba.y, Bb.y));
-                    float dz = __fadd_rn(__fsub_rn(Aa.z, Ab.z), __fsub_rn(Ba.z, Bb.z));
-                    float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                    float tm = fmaxf(Ba.w, Bb.w);
-                    decided  = (r2 < tm * lo_f) ? 1 : ((r2 > tm * hi_f) ? 0 : -1);
+                const float mine = lane < m ? fmaxf(fmaxf(fabsf(xa), fabsf(ya)), fabsf(za)) : 0.f;
+                const float S    = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(mine)));
+                const float M    = fmaxf(fmaxf(fabsf(Ph.x), fabsf(Ph.y)), fabsf(Ph.z));
+                // 2 S / sqrt(thr) + 2 <= 24 and M / sqrt(thr) <= 1e8
+                const bool ok = S * S <= 121.f * thr && M * M <= 1e16f * thr && thr > 1e-30f;
+                tlo           = ok ? thr * lo_f : __int_as_float(0x7fc00000);
+            }
+            for (u32 kb = 0; kb < nk; kb += 32) {
+                const uint2 run = kb + lane < nk ? leaf_ent[k0 + kb + lane] : make_uint2(0, 0);
+                const u32 len   = run.y - run.x;
+                u32 end         = len;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const u32 v = __shfl_up_sync(kAll, end, o);
+                    if (lane >= o) end += v;
                 }
-                bool in;
-                if (decided >= 0) {
-                    in = decided == 1;
-                } else {
-                    f64 dx = __dsub_rn(xa, sx[rb]), dy = __dsub_rn(ya, sy[rb]),
-                        dz = __dsub_rn(za, sz[rb]);
-                    f64 rab2   = dot3_rn(dx, dy, dz);
-                    f64 rint_b = __dmul_rn(sh[rb], h_tol);
-                    f64 thr_b  = __dmul_rn(__dmul_rn(rint_b, rint_b), kRkern * kRkern);
-                    in = !(rab2 > thr_a && rab2 > thr_b);
-                }
-                if (in) {
-                    if (MODE == kFill) ent[w + c] = rb;
-                    if (MODE == kOnePass && c < cap) ent[w + c] = rb;
-                    c++;
+                const u32 total = __shfl_sync(kAll, end, 31), start = end - len;
+                for (u32 t0 = 0; t0 < total; t0 += kCandBlock) {
+                    const u32 nb = min(kCandBlock, total - t0);
+                    __syncwarp();
+                    for (u32 t = t0; t < t0 + nb; t += 32) {
+                        // slot t + lane lies in the last run that starts at or before it
+                        const u32 d    = start - t;
+                        const u32 here = __reduce_or_sync(kAll, len && d < 32 ? 1u << d : 0u);
+                        const u32 past = __popc(__ballot_sync(kAll, len && start < t));
+                        const u32 j    = past + __popc(here & upto) - 1;
+                        const u32 b    = __shfl_sync(kAll, run.x - start, j) + t + lane;
+                        // (slots past the end: far away)
+                        float4 q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
+                        if (t + lane < total) {
+                            const F8 rec = ldg256(&P[2 * (size_t) b]);
+                            q = make_float4(__fadd_rn(__fsub_rn(rec.a.x, ox), rec.b.x),
+                                            __fadd_rn(__fsub_rn(rec.a.y, oy), rec.b.y),
+                                            __fadd_rn(__fsub_rn(rec.a.z, oz), rec.b.z), rec.b.w * lo_f);
+                        }
+                        cand[t - t0 + lane] = q;
+                        ids[t - t0 + lane]  = t + lane < total ? b : kNone;
+                    }
+                    __syncwarp();
+                    for (u32 r = 0; r < m; r++) {
+                        const float x = __shfl_sync(kAll, xa, r), y = __shfl_sync(kAll, ya, r),
+                                    z = __shfl_sync(kAll, za, r);
+                        // rows decided in FP64 alone: no candidate is certain
+                        const float ta = __shfl_sync(kAll, tlo, r);
+                        const u32 rr   = __shfl_sync(kAll, ra, r);
+                        u32 *out       = ent + __shfl_sync(kAll, w, r);
+                        u32 cr         = __shfl_sync(kAll, c, r);
+#pragma unroll 1
+                        for (u32 t = 0; t < nb; t += 32) {
+                            const float4 q = cand[t + lane];
+                            const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
+                            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+                            const float tm = max_nan(ta, q.w);
+                            const bool sure = r2 < tm, open = !sure & !(r2 > tm * band);
+                            u32 bits        = __ballot_sync(kAll, sure);
+                            if (__any_sync(kAll, open)) {
+                                const u32 b = open ? ids[t + lane] : kNone;
+                                bits |= __ballot_sync(kAll, b != kNone && pair_inside(sx, sy, sz, sh, h_tol, rr, b));
+                            }
+                            const u32 at   = cr + __popc(bits & below);
+                            if (MODE != kCount && (bits >> lane & 1u) && (MODE == kFill || at < cap))
+                                out[at] = ids[t + lane];
+                            cr += __popc(bits);
+                        }
+                        if (lane == r) c = cr;
+                    }
                 }
             }
-            rb++;
-        }
-        if (MODE != kFill) cnt[row] = c;
-        if (MODE == kCount) off[row] = (c + 3u) & ~3u;
-        if (MODE == kOnePass) {
-            off[row] = w;
-            if (c > cap) atomicOr(&sc->flags, kFlagCsrCap);
+            if (lane < m) {
+                if (MODE != kFill) cnt[row] = c;
+                if (MODE == kCount) off[row] = (c + 3u) & ~3u;
+                if (MODE == kOnePass) {
+                    off[row] = w;
+                    if (c > cap) atomicOr(&sc->flags, kFlagCsrCap);
+                }
+                c_max = max(c_max, c);
+                c_sum += c;
+            }
         }
     }
     // the largest row of the build (sizes the slots of the next one)
     {
-        u64 m = block_reduce((u64) c, OpMaxU64{}, 0ull);
-        if (threadIdx.x == 0 && m) atomicMax(&sc->row_cnt_max, (u32) m);
+        u64 mx = block_reduce((u64) c_max, OpMaxU64{}, 0ull);
+        if (threadIdx.x == 0 && mx) raise_u32(&sc->row_cnt_max, (u32) mx);
     }
     if (MODE != kCount) {
-        u64 tot = block_reduce((u64) c, OpAddU64{}, 0ull);
+        u64 tot = block_reduce(c_sum, OpAddU64{}, 0ull);
         if (threadIdx.x == 0) atomicAdd((unsigned long long *) &sc->csr_entries, (unsigned long long) tot);
     }
 }
@@ -613,14 +689,16 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // Owner leaves first: they also record, per leaf, the largest threshold of the rows
     // it owns, which lets stage 1 drop leaves that no owned row can pair with (and skip
     // leaves that own no row); the cache is unchanged.
-    if ((e = c.owner.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
+    if ((e = c.next_row.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
+    if ((e = c.leaf_head.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(c.leaf_head.p, 0xff, sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = c.leaf_thr.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(c.leaf_thr.p, 0, sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     u32 *leaf_thr = c.leaf_thr.as<u32>();
     if (n) {
         ProfScope ps(c, kProfOwner, n);
         { k_owner<<<div_up(n, 128), 128, 0, s>>>(t, fb, rec, c.row_rank.as<u32>(), n, c.sx.as<f64>(),
-                                               c.sy.as<f64>(), c.sz.as<f64>(), c.owner.as<u32>(),
+                                               c.sy.as<f64>(), c.sz.as<f64>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(),
                                                &dsc->flags, c.sh.as<f64>(), up_f32(h_tol), leaf_thr); GBSPH_COUNTED; }
     }
     auto stage1 = [&]() -> cudaError_t {
@@ -682,21 +760,17 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     if (one_pass)
         if ((e = c.csr_ent.ensure(sizeof(u32) * ((size_t) n * c.row_cap + 4), s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(&dsc->csr_entries, 0, sizeof(u64), s)) != cudaSuccess) return e;
-    // launch helper for the stage-2 kernel family
+    // launch helper for the stage-2 kernel family: a warp per leaf, in four times the five
+    // blocks that an SM holds (41 KB of candidates each; with one such grid the leaves'
+    // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics
+    // on the totals, 10 ns each, take longer than the build)
     auto part = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
-        if (P) {
-            { k_part_cache<MODE, true><<<div_up(n, 256), 256, 0, s>>>(
-                c.row_rank.as<u32>(), n, c.owner.as<u32>(), c.leaf_cnt.as<u32>(),
-                c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
-                c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap); GBSPH_COUNTED; }
-        } else {
-            { k_part_cache<MODE, false><<<div_up(n, 256), 256, 0, s>>>(
-                c.row_rank.as<u32>(), n, c.owner.as<u32>(), c.leaf_cnt.as<u32>(),
-                c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), nullptr,
-                c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off,
-                ent, dsc, c.row_cap); GBSPH_COUNTED; }
-        }
+        const u32 blocks   = std::min(div_up(L, 8), 20 * c.sms);
+        { k_part_cache<MODE><<<blocks, 256, 0, s>>>(
+            L, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
+            c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
+            c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap); GBSPH_COUNTED; }
     };
     using OnePass = std::integral_constant<int, kOnePass>;
     using Count   = std::integral_constant<int, kCount>;
