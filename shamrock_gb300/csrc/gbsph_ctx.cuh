@@ -119,7 +119,7 @@ struct Ctx {
     u32 n_obj = 0, morton_count = 0, leaf_count = 0;
     DevBuf keys, sort_index, flags_a, flags_b, offsets, reduc, reduced;
     DevBuf radix_k, radix_v, radix_hist, radix_off; // radix sort ping-pong and digit tables
-    DevBuf lchild, rchild, lflag, rflag, endrange, parent, boxes, visit, fboxes, fpairs;
+    DevBuf lchild, rchild, lflag, rflag, endrange, parent, boxes, visit, fboxes, fpairs, wboxes;
     bool has_rint = false;
 
     // ---- rank-ordered copies of merged fields

@@ -88,8 +88,8 @@ struct RangeWriter {
     u32 base, cap, c;
     uint2 cur;
     bool open;
-    __device__ RangeWriter(uint2 *o, const u32 *rd, u32 b, u32 cp)
-        : out(o), reduc(rd), base(b), cap(cp), c(0), open(false) {}
+    __device__ RangeWriter(uint2 *o, const u32 *rd, u32 b, u32 cp, bool writes = true)
+        : out(writes ? o : nullptr), reduc(rd), base(b), cap(cp), c(0), open(false) {}
     __device__ __forceinline__ void add(u32 r0, u32 r1) {
         if (open && cur.y == r0) {
             cur.y = r1;
@@ -289,6 +289,170 @@ __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *
     w.flush();
     const u32 c = w.c;
     if (!ok) atomicOr(&sc->flags, kFlagStackOverflow);
+    if (c > cap) {
+        atomicOr(&sc->flags, kFlagLeafCap);
+        atomicMax(&sc->leaf_cnt_max, c);
+    }
+    cnt[l] = c;
+    off[l] = base;
+}
+
+// ---- an 8-ary hierarchy over the leaves in Morton order for stage 1
+// Level 0 are the leaves' FP32 boxes, node i of level m + 1 bounds the nodes 8 i .. 8 i + 7 of
+// level m (boxes united, the largest interaction radius).  The criterion grows with the
+// boxes and radii (rounding is monotonic), so every leaf that passes lies below nodes that
+// pass, whatever the hierarchy; this one needs no pointers, its eight children are 256
+// consecutive bytes, and eight lanes test them together.
+constexpr int kWideLevels = 9; // 8^8 leaves, then the top nodes are walked in eights
+struct WideTree {
+    const NodeBoxF *level[kWideLevels];
+    u32 n[kWideLevels];
+    int top;
+};
+
+__device__ __forceinline__ float min8(float v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float max8(float v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// three levels above n nodes: 512 of them to 64, 8 and 1 per block
+__global__ void __launch_bounds__(512) k_wide_levels(const NodeBoxF *__restrict__ in, u32 n,
+                                                     NodeBoxF *__restrict__ l1,
+                                                     NodeBoxF *__restrict__ l2,
+                                                     NodeBoxF *__restrict__ l3) {
+    __shared__ NodeBoxF s1[64], s2[32];
+    const float big = 3.0e38f;
+    NodeBoxF none;
+    none.lo = make_float4(big, big, big, 0.f);
+    none.hi = make_float4(-big, -big, -big, 0.f);
+    const u32 t = threadIdx.x, i = blockIdx.x * 512 + t;
+    auto unite = [](NodeBoxF v) {
+        v.lo = make_float4(min8(v.lo.x), min8(v.lo.y), min8(v.lo.z), max8(v.lo.w));
+        v.hi = make_float4(max8(v.hi.x), max8(v.hi.y), max8(v.hi.z), 0.f);
+        return v;
+    };
+    NodeBoxF v = unite(i < n ? in[i] : none);
+    const u32 n1 = (n + 7) / 8, n2 = (n1 + 7) / 8, n3 = (n2 + 7) / 8;
+    if ((t & 7) == 0) {
+        const u32 o = blockIdx.x * 64 + t / 8;
+        s1[t / 8]   = v;
+        if (o < n1) l1[o] = v;
+    }
+    __syncthreads();
+    if (t < 64) {
+        v = unite(s1[t]);
+        if ((t & 7) == 0) {
+            const u32 o = blockIdx.x * 8 + t / 8;
+            s2[t / 8]   = v;
+            if (l2 && o < n2) l2[o] = v;
+        }
+    }
+    __syncthreads();
+    if (t < 32) {
+        v = unite(t < 8 ? s2[t] : none);
+        if (t == 0 && l3 && blockIdx.x < n3) l3[blockIdx.x] = v;
+    }
+}
+
+// Stage 1 for few leaves: eight lanes walk the hierarchy for one leaf, testing a node's eight children per
+// step; the children that pass are a byte of a 64-bit mask per level, so the next node in
+// ascending order is its lowest bit and the walk needs no stack.  Inner nodes pass unless
+// no owned row can pair with anything below them; leaves are decided as in LeafCrit too.
+// Twice the instructions per leaf of k_leaf_lists (the eights of leaves follow the Morton
+// curve, so their boxes are looser than the tree's), but a quarter of its dependent loads
+// and eight times its warps.
+// A leaf owning no row gets an empty list, and a candidate leaf that no owned row can pair
+// with is dropped (leaf_thr, see k_owner; the cache is unchanged).
+__global__ void __launch_bounds__(128) k_leaf_lists_wide(TreeView t, const NodeBoxF *__restrict__ fb,
+                                                         WideTree wt, u32 *__restrict__ cnt,
+                                                         u32 *__restrict__ off,
+                                                         uint2 *__restrict__ ent, u32 cap, Scalars *sc,
+                                                         const u32 *__restrict__ leaf_thr) {
+    const u32 g = threadIdx.x & 7u, shift = threadIdx.x & 24u;
+    const u32 l = (blockIdx.x * 128 + threadIdx.x) / 8;
+    const u32 base = l * cap;
+    const u32 tb   = l < t.L ? leaf_thr[l] : 0; // 0: no row is owned by this leaf
+    const float thr_own = __uint_as_float(tb);
+    LazyLeafCrit crit(t, l < t.L ? l : 0);
+    const F8 fa = ldg256(&wt.level[0][l < t.L ? l : 0]), fr = ldg256(&fb[0]);
+    const float4 alo = fa.a, ahi = fa.b, rlo = fr.a, rhi = fr.b;
+    float M = fmaxf(fmaxf(fmaxf(fabsf(rlo.x), fabsf(rlo.y)), fmaxf(fabsf(rlo.z), fabsf(rhi.x))),
+                    fmaxf(fabsf(rhi.y), fabsf(rhi.z)));
+    float band_abs = 1e-6f * M;
+    // Every row owned by this leaf lies in its box, so a pair (a, b) with b below a node has
+    // r_ab at least the Euclidean gap D between the boxes.  With thr_own >= thr_a of every
+    // owned row and (r_node R)^2 >= thr_b, D^2 > max of the two makes every pair test below
+    // the node fail.  The FP32 gaps are shrunk by the rounding band and the bound carries a
+    // 1e-5 margin, so the skip is certain.
+    auto apart = [&](const float4 &nlo, const float4 &nhi) -> bool {
+        float gx = fmaxf(fmaxf(nlo.x - ahi.x, alo.x - nhi.x) - band_abs, 0.f);
+        float gy = fmaxf(fmaxf(nlo.y - ahi.y, alo.y - nhi.y) - band_abs, 0.f);
+        float gz = fmaxf(fmaxf(nlo.z - ahi.z, alo.z - nhi.z) - band_abs, 0.f);
+        float d2 = gx * gx + gy * gy + gz * gz;
+        float tb2 = fmaxf(thr_own, nlo.w * nlo.w * 1.000001f);
+        return d2 > tb2 * 1.00001f;
+    };
+    // the criterion of the reference for a leaf, in FP64 inside the rounding band
+    auto leaf_passes = [&](u32 leaf, const float4 &nlo, const float4 &nhi) -> bool {
+        float sx = fmaxf(nlo.x - ahi.x, alo.x - nhi.x);
+        float sy = fmaxf(nlo.y - ahi.y, alo.y - nhi.y);
+        float sz = fmaxf(nlo.z - ahi.z, alo.z - nhi.z);
+        float sm = fmaxf(fmaxf(sx, sy), sz);
+        float R  = fmaxf(nlo.w, alo.w);
+        float band = band_abs + 1e-6f * R;
+        if (sm < R - band) return true;
+        if (sm > R + band) return false;
+        return crit(t.off() + leaf);
+    };
+    RangeWriter w(ent, t.reduc, base, cap, g == 0);
+    // the node whose children are tested next: index i at level m (m = top + 1: the i-th eight
+    // of the top level); pend: children still to visit, byte m - 1 for those at level m
+    u32 i = 0, root = 0;
+    const u32 roots = (wt.n[wt.top] + 7) / 8;
+    int m    = wt.top + 1;
+    u64 pend = 0;
+    bool run = tb != 0;
+    while (__any_sync(0xffffffffu, run)) {
+        const u32 child = 8 * i + g;
+        bool pass       = false;
+        if (run && child < wt.n[m - 1]) {
+            const F8 nb = ldg256(&wt.level[m - 1][child]);
+            pass = !apart(nb.a, nb.b);
+            if (m == 1 && pass) pass = leaf_passes(child, nb.a, nb.b);
+        }
+        u32 bits = (__ballot_sync(0xffffffffu, pass) >> shift) & 0xffu;
+        if (!run) continue;
+        if (m == 1) {
+            while (bits) { // runs of consecutive leaves
+                const u32 s = __ffs(bits) - 1, e = __ffs(~(bits >> s)) - 1;
+                w.add(8 * i + s, 8 * i + s + e);
+                bits &= ~(((1u << e) - 1u) << s);
+            }
+        } else {
+            pend |= (u64) bits << (8 * (m - 2));
+        }
+        if (pend) {
+            const int p = __ffsll((long long) pend) - 1;
+            const int at = p / 8 + 1;                // level of the pending child
+            i    = 8 * (i >> (3 * (at + 1 - m))) + (u32) (p & 7);
+            m    = at;
+            pend &= pend - 1;
+        } else {
+            root++;
+            i   = root;
+            m   = wt.top + 1;
+            run = root < roots;
+        }
+    }
+    if (l >= t.L || g != 0) return;
+    w.flush();
+    const u32 c = w.c;
     if (c > cap) {
         atomicOr(&sc->flags, kFlagLeafCap);
         atomicMax(&sc->leaf_cnt_max, c);
@@ -686,6 +850,32 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     const NodeBoxF *fb = c.fboxes.as<NodeBoxF>();
     const NodePairF *rec = c.fpairs.as<NodePairF>();
     if (L > 1) { k_node_pairs<<<div_up(L - 1, 256), 256, 0, s>>>(t, fb, c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
+    // Stage 1 on the 8-ary hierarchy (built here, three levels per launch) while a thread per
+    // leaf would leave an SM fewer than 512 threads: the binary walk is a chain of dependent
+    // loads, 113 us for 1,399 leaves and 219 us for 35,981 against 36 and 139 us; from about
+    // 100,000 leaves on its throughput wins (245,000 leaves: 0.58 against 0.80 ms).
+    const bool wide = L <= 512 * c.sms;
+    WideTree wt{};
+    wt.level[0] = fb + (L - 1);
+    wt.n[0]     = L;
+    size_t wide_nodes = 0;
+    while (wide && wt.top + 1 < kWideLevels && wt.n[wt.top] > 8) {
+        wt.n[wt.top + 1] = (wt.n[wt.top] + 7) / 8;
+        wt.top++;
+        wide_nodes += wt.n[wt.top];
+    }
+    if ((e = c.wboxes.ensure(sizeof(NodeBoxF) * (wide_nodes + 1), s)) != cudaSuccess) return e;
+    {
+        NodeBoxF *at = c.wboxes.as<NodeBoxF>();
+        for (int m = 1; m <= wt.top; m++) {
+            wt.level[m] = at;
+            at += wt.n[m];
+        }
+        auto lv = [&](int m) { return m <= wt.top ? const_cast<NodeBoxF *>(wt.level[m]) : nullptr; };
+        for (int m = 0; m < wt.top; m += 3) {
+            { k_wide_levels<<<div_up(wt.n[m], 512), 512, 0, s>>>(wt.level[m], wt.n[m], lv(m + 1), lv(m + 2), lv(m + 3)); GBSPH_COUNTED; }
+        }
+    }
     // Owner leaves first: they also record, per leaf, the largest threshold of the rows
     // it owns, which lets stage 1 drop leaves that no owned row can pair with (and skip
     // leaves that own no row); the cache is unchanged.
@@ -705,8 +895,13 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         cudaError_t err = c.leaf_ent.ensure(sizeof(uint2) * ((size_t) L * c.leaf_cap + 1), s);
         if (err != cudaSuccess) return err;
         ProfScope ps(c, kProfStage1, L);
-        { k_leaf_lists<<<div_up(L, 128), 128, 0, s>>>(t, fb, rec, c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(),
-                                                    c.leaf_ent.as<uint2>(), c.leaf_cap, dsc, leaf_thr); GBSPH_COUNTED; }
+        if (wide) {
+            k_leaf_lists_wide<<<div_up(L, 16), 128, 0, s>>>(t, fb, wt, c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(),
+                                                           c.leaf_ent.as<uint2>(), c.leaf_cap, dsc, leaf_thr); GBSPH_COUNTED;
+        } else {
+            k_leaf_lists<<<div_up(L, 128), 128, 0, s>>>(t, fb, rec, c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(),
+                                                       c.leaf_ent.as<uint2>(), c.leaf_cap, dsc, leaf_thr); GBSPH_COUNTED;
+        }
         return cudaGetLastError();
     };
     if (s1_one_pass) {
