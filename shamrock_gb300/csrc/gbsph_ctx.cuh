@@ -153,7 +153,7 @@ struct Ctx {
     DevBuf rec64; // FP64 pair-loop records, 20 doubles per merged particle (sph64.cu)
     // mixed precision staging (rank order); f_comp: the compensated tier's extra records
     DevBuf f_pos, f_anchor, f_aux0, f_aux1, f_aux2, f_comp;
-    DevBuf f_sums; // pair sums of the mixed derivatives, by rank
+    DevBuf f_sums; // pair sums of the derivatives, by rank (see sums_buffer)
     // error-controlled mixed precision: the tier the next step starts in (1 FP32 pair
     // arithmetic, 2 compensated) and the start state a step is recomputed from
     u32 guard_tier = 1;
@@ -182,6 +182,18 @@ struct Ctx {
 
     ~Ctx();
 };
+
+// Room for the derivatives' pair sums: the stage-1 lists, which only the cache build before
+// them reads, or a buffer of its own where those are too small.
+inline cudaError_t sums_buffer(Ctx &c, size_t bytes, void **p) {
+    if (c.leaf_ent.size >= bytes) {
+        *p = c.leaf_ent.p;
+        return cudaSuccess;
+    }
+    cudaError_t e = c.f_sums.ensure(bytes, c.stream);
+    *p            = c.f_sums.p;
+    return e;
+}
 
 // ------------------------------------------------------------------ profiling
 int prof_begin(Ctx &c, int kind, u64 units);

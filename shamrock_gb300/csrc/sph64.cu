@@ -1227,9 +1227,10 @@ cudaError_t derivs_step64(Ctx &c, const RowSpace &rs, u32 N, f64 pmass, f64 alph
                           const ExtAccel &ext) {
     DerivParams p{pmass, alpha_u, beta_AV, hdt, C_cour, C_force, ext};
     ProfScope ps(c, kProfDerivs, rs.n);
-    cudaError_t e = c.f_sums.ensure(sizeof(f64) * 5 * (size_t) N, c.stream);
+    void *room    = nullptr;
+    cudaError_t e = sums_buffer(c, sizeof(f64) * 5 * (size_t) N, &room);
     if (e != cudaSuccess) return e;
-    f64 *sums = c.f_sums.as<f64>(), *vmax = sums + 4 * (size_t) N;
+    f64 *sums = (f64 *) room, *vmax = sums + 4 * (size_t) N;
     { k_derivs_sums64<<<div_up(rs.n, 32), 128, 0, c.stream>>>(rs, c.rec64.as<f64>(), N, c.scs.as<f64>(), p,
                                                              sums, vmax); GBSPH_COUNTED; }
     { k_correct64<<<std::min(div_up(rs.n, 256), 6 * c.sms), 256, 0, c.stream>>>(

@@ -944,8 +944,9 @@ cudaError_t derivs_step_mixed(Ctx &c, const RowSpace &rs, f64 pmass, f64 alpha_u
     const float *cs_rank = varying_av ? c.f_aux2.as<float>() : nullptr;
     ProfScope ps(c, kProfDerivs, rs.n);
     cudaError_t e;
-    if ((e = c.f_sums.ensure(2 * sizeof(float4) * (size_t) c.n_obj, c.stream)) != cudaSuccess) return e;
-    float4 *sums = c.f_sums.as<float4>();
+    void *room = nullptr;
+    if ((e = sums_buffer(c, 2 * sizeof(float4) * (size_t) c.n_obj, &room)) != cudaSuccess) return e;
+    float4 *sums = (float4 *) room;
     auto kern    = cond ? k_derivs_sums_mixed<true> : k_derivs_sums_mixed<false>;
     { kern<<<div_up(rs.n, 32), 128, 0, c.stream>>>(rs, ms, p, cs_rank, sums); GBSPH_COUNTED; }
     auto corr = cond ? k_correct_mixed<true> : k_correct_mixed<false>;
