@@ -16,6 +16,7 @@ struct BBox {
     f64 lo[3];
     f64 hi[3];
     f64 fact[3];
+    f64 inv[3]; // 1 / fact, 0 outside the middle of the range (see grid_cell)
 };
 
 // Small device-side reduction results, read back through pinned memory.

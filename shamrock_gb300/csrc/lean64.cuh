@@ -261,4 +261,30 @@ GBSPH_HD double mul64i(double a, double b) {
     return from64(m + ((uint64_t) (e - 1u) << 52) + ((uint64_t) ((ah ^ bh) & 0x80000000u) << 32));
 }
 
+// The Morton grid cell of a coordinate: min(trunc(RN((clamp(p, lo, hi) - lo) / step)), top),
+// inv = 1 / step (0: step is not a normal number in the middle of the range).  The quotient
+// comes from one FMA that adds 2^28: it leaves the cell above bit 24 of the significand and
+// 24 fraction bits below, in error by less than 0.6 of the last, so a fraction other than
+// zero proves the cell (the correctly rounded quotient lies in the same cell); a zero
+// fraction, infinities and NaN take the quotient itself.  Two FP64 instructions instead of
+// about 25 with the clamps and the division.
+static GBSPH_HD_RARE uint32_t grid_cell_plain(double p, double lo, double hi, double step, uint32_t top) {
+    const double r = fmin(fmax(p, lo), hi);
+    const double q = (r - lo) / step;
+    if (!(q > 0.)) return 0u;
+    return q < (double) top ? (uint32_t) q : top;
+}
+GBSPH_HD uint32_t grid_cell(double p, double lo, double hi, double step, double inv, uint32_t top) {
+    const double d    = p - lo;
+    const uint64_t tb = bits64(fma64(d, inv, 268435456.0));
+    const int32_t th  = (int32_t) (uint32_t) (tb >> 32);
+    const uint32_t tl = (uint32_t) tb;
+    if ((tl & 0xFFFFFFu) == 0u || (hi64(d) & 0x7FF00000u) == 0x7FF00000u)
+        return grid_cell_plain(p, lo, hi, step, top);
+    if (th < 0x41B00000) return 0u;   // below 2^28: left of the box
+    if (th >= 0x41C00000) return top; // at 2^29 and above
+    const uint32_t cell = ((uint32_t) (th - 0x41B00000) << 8) | (tl >> 24);
+    return cell < top ? cell : top;
+}
+
 } // namespace gbsph

@@ -488,12 +488,6 @@ __global__ void k_rows(const u32 *__restrict__ sort_index, const u8 *__restrict_
 // The exact containment test inside the FP32 band compares the doubles' ordered bit
 // patterns with integer operations (the FP64 pipe is scarce on GB300; particles lie on
 // their own leaf's faces, so the band is met often).
-__device__ __forceinline__ long long ord64(f64 v) {
-    long long b = __double_as_longlong(v);
-    if (b == (long long) 0x8000000000000000ull) b = 0; // -0 orders as +0
-    return b < 0 ? (b ^ 0x7fffffffffffffffll) : b;
-}
-
 __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__restrict__ fb,
                                                const NodePairF *__restrict__ rec,
                                                const u32 *__restrict__ row_rank, u32 n_rows,

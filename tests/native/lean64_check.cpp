@@ -54,6 +54,37 @@ static void all(double a, double b) {
     }
 }
 
+// the cell equals the clamped division's, and half the coordinates sit on cell faces or next
+// to them, on the box's faces or beyond
+static void cells(std::mt19937_64 &g, long n) {
+    std::uniform_real_distribution<double> u(-0.1, 1.1);
+    for (const uint32_t count : {1024u, 2097152u})
+        for (long b = 0; b < 64; b++) {
+            const double lo   = b % 8 == 0 ? 0.0 : (b % 8 == 1 ? -0.5 : std::ldexp(u(g) - 0.5, (int) (b % 40) - 20));
+            const double size = b % 16 < 2 ? 1.0 : (b == 17 ? 0.0 : (b == 18 ? 1e-320 : std::ldexp(1 + std::fabs(u(g)), (int) (b * 5 % 61) - 30)));
+            const double hi = lo + size, step = (hi - lo) / (double) count;
+            const double inv = step > 1e-300 && step < 1e300 ? 1.0 / step : 0.0;
+            std::vector<double> ps = {lo, hi, std::nextafter(lo, -1e308), std::nextafter(hi, 1e308), -0.0, 1e308, -1e308,
+                                      std::numeric_limits<double>::infinity(), -std::numeric_limits<double>::infinity(),
+                                      std::numeric_limits<double>::quiet_NaN(), lo + 1e6 * size, hi - 1e9 * size};
+            for (long i = 0; i < n / 128; i++) {
+                double p = lo + u(g) * (hi - lo);
+                if (i % 2) p = lo + (double) (g() % count) * step;
+                if (i % 4 == 3) p = std::nextafter(p, i % 8 == 3 ? 1e308 : -1e308);
+                ps.push_back(p);
+            }
+            for (double p : ps) {
+                const double r = std::fmin(std::fmax(p, lo), hi), q = (r - lo) / step;
+                const uint32_t want = !(q > 0) ? 0u : (q >= (double) (count - 1) ? count - 1 : (uint32_t) q);
+                checks++;
+                if (grid_cell(p, lo, hi, step, inv, count - 1) != want) {
+                    if (wrong < 5) std::printf("cell of %a in [%a, %a], %u\n", p, lo, hi, count);
+                    wrong++;
+                }
+            }
+        }
+}
+
 int main(int argc, char **argv) {
     const long n = argc > 1 ? std::atol(argv[1]) : 1000000;
     std::mt19937_64 g(7);
@@ -80,6 +111,7 @@ int main(int argc, char **argv) {
         all(std::ldexp(a, ea), std::ldexp(b, eb));
     }
     const double share = (double) reported / (double) (checks - before);
+    cells(g, n);
     std::printf("checks %ld wrong %ld reported %.3g edges reported %ld\n", checks, wrong, share, edges_reported);
     return wrong == 0 && share < 0.05 ? 0 : 1;
 }
