@@ -100,40 +100,87 @@ __device__ __forceinline__ void cmpx(K &a, K &b, u32 &va, u32 &vb, bool reverse)
     }
 }
 
+// The tile of the shared-memory passes.  A thread holds the elements that differ in up to
+// four neighbouring index bits, the lowest of them bit 0, 4 or 8; with the low four bits
+// exchanged with the next four (an XOR, so the places of a group follow from one) 16
+// consecutive lanes always meet all 16 pairs of banks.
+__device__ __forceinline__ u32 tile_place(u32 i) { return i ^ ((i >> 4) & 15u); }
 template<class K, int TILE>
-__global__ void __launch_bounds__(512) k_bitonic_smem(K *__restrict__ keys, u32 *__restrict__ vals,
-                                                      u32 tile, u32 length_lo, u32 length_hi,
-                                                      u32 inc_start) {
-    __shared__ K sk[TILE];
-    __shared__ u32 sv[TILE];
-    u32 base = blockIdx.x * tile;
-    for (u32 k = threadIdx.x; k < tile; k += blockDim.x) {
-        sk[k] = keys[base + k];
-        sv[k] = vals[base + k];
+struct SortTile {
+    K k[TILE];
+    u32 v[TILE];
+    __device__ __forceinline__ void get(u32 p, K &a, u32 &b) const { a = k[p], b = v[p]; }
+    __device__ __forceinline__ void put(u32 p, K a, u32 b) { k[p] = a, v[p] = b; }
+};
+template<int TILE>
+struct SortTile<u32, TILE> {
+    uint2 kv[TILE];
+    __device__ __forceinline__ void get(u32 p, u32 &a, u32 &b) const {
+        const uint2 e = kv[p];
+        a = e.x, b = e.y;
+    }
+    __device__ __forceinline__ void put(u32 p, u32 a, u32 b) { kv[p] = make_uint2(a, b); }
+};
+
+// the stages of increments S / 2 ... 1 among S elements in registers
+template<class K, int S>
+__device__ __forceinline__ void reg_stages(K (&x)[S], u32 (&v)[S], bool reverse) {
+#pragma unroll
+    for (int d = S / 2; d >= 1; d >>= 1)
+#pragma unroll
+        for (int k = 0; k < S; k++)
+            if ((k & d) == 0) cmpx(x[k], x[k + d], v[k], v[k + d], reverse);
+}
+
+// BITS consecutive stages (increments 2^(bit + BITS - 1) ... 2^bit) of one merge step;
+// from: where the first of a merge's rounds finds the elements, null once they are in s
+template<class K, int TILE, int BITS>
+__device__ __forceinline__ void tile_round(SortTile<K, TILE> &s, u32 tile, u32 base, u32 dir, int bit,
+                                           const K *from_k = nullptr, const u32 *from_v = nullptr) {
+    constexpr int S = 1 << BITS;
+    for (u32 g = threadIdx.x; g < tile >> BITS; g += blockDim.x) {
+        const u32 i = ((g >> bit) << (bit + BITS)) | (g & ((1u << bit) - 1u)), p = tile_place(i);
+        K x[S];
+        u32 v[S];
+#pragma unroll
+        for (int k = 0; k < S; k++) {
+            if (from_k) x[k] = from_k[base + i + ((u32) k << bit)], v[k] = from_v[base + i + ((u32) k << bit)];
+            else s.get(p ^ tile_place((u32) k << bit), x[k], v[k]);
+        }
+        reg_stages<K, S>(x, v, (dir & (base + i)) == 0);
+#pragma unroll
+        for (int k = 0; k < S; k++) s.put(p ^ tile_place((u32) k << bit), x[k], v[k]);
     }
     __syncthreads();
-    for (u32 length = length_lo; length < length_hi; length <<= 1) {
-        u32 dir = length << 1;
-        for (u32 inc = (length == length_lo) ? inc_start : length; inc > 0; inc >>= 1) {
-            for (u32 j = threadIdx.x; j < tile / 2; j += blockDim.x) {
-                u32 low = j & (inc - 1);
-                u32 i   = (j << 1) - low;
-                bool reverse = (dir & (base + i)) == 0;
-                K a = sk[i], b = sk[i + inc];
-                u32 va = sv[i], vb = sv[i + inc];
-                cmpx(a, b, va, vb, reverse);
-                sk[i]       = a;
-                sk[i + inc] = b;
-                sv[i]       = va;
-                sv[i + inc] = vb;
-            }
-            __syncthreads();
+}
+
+// The stages within tiles, up to four at a time in registers.  MERGE: the last
+// log2(TILE) stages of one merge step, else all steps of lengths below `tile`.  Bound by
+// issue and shared memory about alike: a pair costs about six instructions a stage, and the
+// tile is read and written once for four.  2^22 keys, all launches: 624 us with a stage at a
+// time in shared memory, 398 with three in registers, 208 with four.
+template<class K, int TILE, bool MERGE>
+__global__ void __launch_bounds__(256) k_bitonic_smem(K *__restrict__ keys, u32 *__restrict__ vals,
+                                                      u32 tile, u32 length) {
+    __shared__ SortTile<K, TILE> s;
+    constexpr int kBits = TILE == 4096 ? 12 : 11, kTop = kBits - 8;
+    const u32 base = blockIdx.x * tile;
+    if (MERGE) {
+        tile_round<K, TILE, kTop>(s, TILE, base, length << 1, 8, keys, vals);
+        tile_round<K, TILE, 4>(s, TILE, base, length << 1, 4);
+        tile_round<K, TILE, 4>(s, TILE, base, length << 1, 0);
+    } else {
+        for (u32 k = threadIdx.x; k < tile; k += 256) s.put(tile_place(k), keys[base + k], vals[base + k]);
+        __syncthreads();
+        for (u32 len = 1; len < tile; len <<= 1) {
+            int left = 32 - __clz(len); // stages of the step
+            if (left % 4 == 1) tile_round<K, TILE, 1>(s, tile, base, len << 1, left - 1);
+            if (left % 4 == 2) tile_round<K, TILE, 2>(s, tile, base, len << 1, left - 2);
+            if (left % 4 == 3) tile_round<K, TILE, 3>(s, tile, base, len << 1, left - 3);
+            for (left -= left % 4; left > 0; left -= 4) tile_round<K, TILE, 4>(s, tile, base, len << 1, left - 4);
         }
     }
-    for (u32 k = threadIdx.x; k < tile; k += blockDim.x) {
-        keys[base + k] = sk[k];
-        vals[base + k] = sv[k];
-    }
+    for (u32 k = threadIdx.x; k < tile; k += 256) s.get(tile_place(k), keys[base + k], vals[base + k]);
 }
 
 // LEVELS consecutive stages (inc, inc/2, ...) of one merge step in registers,
@@ -174,7 +221,7 @@ cudaError_t bitonic_sort(K *keys, u32 *vals, u32 len, cudaStream_t s) {
     constexpr int TILE = (sizeof(K) == 4) ? 4096 : 2048;
     if (len <= 1) return cudaSuccess;
     u32 tile = len < (u32) TILE ? len : (u32) TILE;
-    { k_bitonic_smem<K, TILE><<<len / tile, 512, 0, s>>>(keys, vals, tile, 1, tile, 1); GBSPH_COUNTED; }
+    { k_bitonic_smem<K, TILE, false><<<len / tile, 256, 0, s>>>(keys, vals, tile, 0); GBSPH_COUNTED; }
     for (u32 length = TILE; length < len; length <<= 1) {
         u32 inc = length;
         while (inc >= (u32) TILE) {
@@ -190,8 +237,7 @@ cudaError_t bitonic_sort(K *keys, u32 *vals, u32 len, cudaStream_t s) {
             }
             inc >>= levels;
         }
-        { k_bitonic_smem<K, TILE><<<len / TILE, 512, 0, s>>>(keys, vals, TILE, length, length << 1,
-                                                          TILE / 2); GBSPH_COUNTED; }
+        { k_bitonic_smem<K, TILE, true><<<len / TILE, 256, 0, s>>>(keys, vals, TILE, length); GBSPH_COUNTED; }
     }
     return cudaGetLastError();
 }
@@ -527,6 +573,14 @@ __global__ void k_bbox_finalize(const Scalars *sc, BBox *bb, u32 val_count) {
     bb->fact[c] = __ddiv_rn(__dsub_rn(hi, lo), (f64) val_count);
 }
 
+// Up to this many keys (padded to a power of two) the network sorts at once.  Where keys are
+// distinct it costs what the radix sort does (2^20: 105 us against 100, and 14 launches
+// against 23; 2^19: 67 against 88; 2^13: 20 us in 3 launches against 68 in 21; at 2^21 192
+// against 119), and where they are not, as in most states that are no lattice, the radix
+// sort's work and the tree passes up to its sync are lost (disc of 1,000,003: 4242 -> 4053 us
+// a step).
+constexpr u32 kNetworkKeys = 1u << 20;
+
 template<class K>
 cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
                             u32 level, f64 htol, u32 morton_count, bool fast_sort) {
@@ -562,9 +616,9 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     Scalars *dsc = c.d_scalars.as<Scalars>();
     u8 *fa = c.flags_a.as<u8>(), *fb = c.flags_b.as<u8>();
     u8 *fin = (level % 2 == 0) ? fa : fb;
-    // The radix sort is tried first when allowed; equal keys (whose order is the
-    // network's) send the build back to the bitonic sort, found at the sync below.
-    const bool radix = fast_sort && std::is_same<K, u32>::value;
+    // For many keys the radix sort is tried first when allowed; equal keys (whose order is
+    // the network's) send the build back to the bitonic sort, found at the sync below.
+    const bool radix = fast_sort && std::is_same<K, u32>::value && P > kNetworkKeys;
     for (int attempt = radix ? 0 : 1; attempt < 2; attempt++) {
         {
             ProfScope ps(c, kProfSort, P);

@@ -1,0 +1,50 @@
+"""Routes that a rule on sizes chooses, on both sides of the rule."""
+import numpy as np
+import pytest
+
+from test_gpu_step import make_pair
+
+pytestmark = pytest.mark.gpu
+
+
+def _lattice_state(nx, ny, nz, ties, seed=0):
+    """A jittered lattice (no two particles in a Morton cell of 1/1024 of the box) and
+    `ties` close pairs that share one."""
+    rng = np.random.default_rng(seed)
+    d = 1.0 / max(nx, ny, nz)
+    pos = np.stack(np.meshgrid(*[(np.arange(k) + 0.5) * d for k in (nx, ny, nz)], indexing="ij"), -1).reshape(-1, 3)
+    pos = pos + 0.1 * d * (rng.random(pos.shape) - 0.5)
+    pick = rng.choice(len(pos), ties, replace=False)
+    pos = np.concatenate([pos, pos[pick] + 1e-7 * rng.standard_normal((ties, 3))])
+    n = len(pos)
+    return dict(pos=pos, vel=np.zeros((n, 3)), h=np.full(n, 1.2 * d), u=np.ones(n), gamma=1.4, pmass=1.0 / n,
+                box_min=(0, 0, 0), box_max=(1, 1, 1))
+
+
+@pytest.mark.parametrize("shape,ties", [((2, 1, 1), 0), ((13, 9, 7), 0), ((13, 9, 7), 5), ((128, 128, 64), 0),
+                                        ((102, 102, 101), 0), ((102, 102, 101), 40)])
+def test_step_sort_is_the_networks(shape, ties):
+    """The permutation after a step equals the bitonic network's over the same keys, by the
+    network itself (up to 2^20 keys), the radix sort, and the radix sort's fall-back."""
+    from shamrock_gb300 import modules as M
+
+    model, _ = make_pair(_lattice_state(*shape, ties), precision="mixed", periodic=False)
+    model.set_next_dt(0.0)
+    model.evolve_once()
+    import ctypes as C
+    import torch
+
+    ctx = model._lib_ctx
+    P, Lc = C.c_uint32(), C.c_uint32()
+    ctx.call("gbsph_tree_counts", C.byref(P), C.byref(Lc))
+    keys = torch.empty(P.value, dtype=torch.int32, device="cuda")
+    perm = torch.empty(P.value, dtype=torch.int32, device="cuda")
+    ctx.call("gbsph_tree_export", C.c_void_p(keys.data_ptr()), C.c_void_p(perm.data_ptr()), *([None] * 11))
+    torch.cuda.synchronize()
+    unsorted = torch.empty_like(keys)
+    unsorted[perm.long()] = keys
+    want_keys, want = M.sort_by_key(ctx, unsorted, key_bits=32)
+    assert torch.equal(keys, want_keys)
+    n = len(model.collect_data()["hpart"])
+    assert torch.equal(perm[:n], want[:n])
+    assert (len(torch.unique(keys[:n])) < n) == (ties > 0)
