@@ -68,7 +68,7 @@ Ctx::~Ctx() {
     DevBuf *bufs[] = {&scan_scratch, &d_scalars, &d_bbox, &keys, &sort_index, &flags_a, &flags_b,
                       &offsets, &reduc, &reduced, &radix_k, &radix_v, &radix_hist, &radix_off, &lchild, &rchild, &lflag, &rflag, &endrange,
                       &parent, &boxes, &visit, &fboxes, &fpairs, &wboxes, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
-                      &row_local, &row_flags, &row_offsets, &leaf_cnt, &leaf_off, &leaf_ent,
+                      &row_local, &leaf_cnt, &leaf_off, &leaf_ent,
                       &leaf_head, &next_row, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
                       &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &scs, &rec64,
                       &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
@@ -100,24 +100,12 @@ __global__ void k_cache_export_entries(u32 n, const u32 *__restrict__ row_local,
     for (u32 k = off[t]; k < off[t] + cnt[t]; k++) out_ent[w++] = sort_index[ent[k]];
 }
 
-struct ScalarsReset {
-    static void eps(Scalars &s) {
-        s.eps_max   = 0;
-        s.eps_min   = ~0ull;
-        s.iters_max = 0;
-    }
-};
-
 __global__ void k_reset_eps(Scalars *sc) {
     sc->eps_max   = 0;
     sc->eps_min   = ~0ull;
     sc->iters_max = 0;
 }
-__global__ void k_reset_corrector(Scalars *sc) {
-    sc->epsv2_max = 0;
-    sc->dt_min    = ~0ull;
-    sc->sum_v2    = 0;
-}
+__global__ void k_reset_corrector(Scalars *sc) { reset_corrector(sc); }
 
 // tape: velocity and energy (SoA) before a corrector evaluation
 __global__ void k_snap_vu(u32 n, const f64 *__restrict__ vx, const f64 *__restrict__ vy,
@@ -305,7 +293,7 @@ int gbsph_morton_codes(gbsph_ctx *ctx, const double *x, const double *y, const d
     ENTER(ctx, stream);
     REQUIRE_ARG(morton_count >= n, "MortonCodeSet: morton_count < cnt_obj");
     REQUIRE_ARG(key_bits == 32 || key_bits == 64, "key_bits must be 32 or 64");
-    CU(set_bbox_host(ctx->c, bmin_host, bmax_host));
+    CU(set_bbox_host(ctx->c, bmin_host, bmax_host, key_bits));
     CU(morton_codes_dev(ctx->c, x, y, z, n, morton_count, key_bits, keys_out));
     return GBSPH_OK;
 }
@@ -330,7 +318,7 @@ int gbsph_build_tree(gbsph_ctx *ctx, const double *x, const double *y, const dou
     REQUIRE_ARG(morton_count == 0 || (morton_count >= n && (morton_count & (morton_count - 1)) == 0),
                 "morton_count must be 0 or a power of two >= n");
     CU(cudaMemsetAsync(ctx->c.d_scalars.p, 0, sizeof(Scalars), ctx->c.stream));
-    CU(set_bbox_host(ctx->c, bmin_host, bmax_host));
+    CU(set_bbox_host(ctx->c, bmin_host, bmax_host, key_bits));
     CU(tree_build(ctx->c, x, y, z, h, n, reduction_level, htol, key_bits, morton_count));
     ctx->c.cache_valid = false;
     CU(cudaStreamSynchronize(ctx->c.stream));
@@ -712,9 +700,8 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         } else {
             c.n_ghost = 0;
         }
-        CU(merge_positions(c, lf.x, lf.y, lf.z, lf.vs, lf.h, n));
+        CU(merge_positions(c, lf.x, lf.y, lf.z, lf.vs, lf.h, n, true));
         u32 N = n + c.n_ghost;
-        CU(bbox_from_merged(c, N));
         CU(tree_build(c, c.mx.as<f64>(), c.my.as<f64>(), c.mz.as<f64>(), c.mh.as<f64>(), N,
                       cfg->tree_reduction_level, cfg->htol_up_coarse, 32, 0, true));
         CU(build_rows(c, n));
@@ -725,11 +712,9 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         rs = RowSpace{n,                  c.row_rank.as<u32>(), c.row_local.as<u32>(),
                       c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>(),
                       c.sx.as<f64>(),      c.sy.as<f64>(),      c.sz.as<f64>()};
-        CU(gather_rows(c, n, c.sh.as<f64>(), c.h_old_row.as<f64>(), c.hnew_row.as<f64>()));
-        CU(fill64(c, n, c.eps_row.as<f64>(), 100.0));
+        CU(h_start(c, n, c.sh.as<f64>(), c.h_old_row.as<f64>(), c.hnew_row.as<f64>(), c.eps_row.as<f64>(), 100.0));
         u32 iters_total = 0;
         if (fused_h) {
-            { k_reset_eps<<<1, 1, 0, s>>>(dsc); GBSPH_COUNTED; }
             if (mixed)
                 CU(h_iterate_mixed(c, rs, c.h_old_row.as<f64>(), c.hnew_row.as<f64>(),
                                    c.eps_row.as<f64>(), cfg->pmass, cfg->htol_up_coarse,
@@ -866,7 +851,6 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
             }
             tape->iters = corr_iters + 1;
         }
-        { k_reset_corrector<<<1, 1, 0, s>>>(dsc); GBSPH_COUNTED; }
         f64 C_cour  = cfg->cfl_cour * ts->cfl_mult;
         f64 C_force = cfg->cfl_force * ts->cfl_mult;
         // the error estimate of the mixed tiers comes from the step's first evaluation

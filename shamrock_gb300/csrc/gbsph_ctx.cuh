@@ -21,8 +21,8 @@ struct BBox {
 
 // Small device-side reduction results, read back through pinned memory.
 struct Scalars {
-    u64 bbox_min[3];   // ordered-u64 min of merged positions
-    u64 bbox_max[3];   // ordered-u64 max
+    u64 bbox_min[3];   // complement of the ordered-u64 min of merged positions
+    u64 bbox_max[3];   // ordered-u64 max; these and hmax are zero between their kernels
     u64 hmax;          // ordered-u64 max of local h
     u64 eps_max;       // ordered-u64 max of eps_h (h iteration)
     u64 eps_min;       // ordered-u64 min of eps_h
@@ -47,7 +47,15 @@ struct Scalars {
     u32 leaf_cnt_max;  // largest stage-1 list among leaves that overflowed their slots
     u32 row_cnt_max;   // largest stage-2 row among rows that overflowed their slots
     u32 dup_keys;      // radix-sorted Morton keys had equal neighbours
+    u32 ticket;        // last-block counter, zero between kernels
 };
+
+// identities of a corrector evaluation's reductions, set by the staging kernel before it
+__device__ __forceinline__ void reset_corrector(Scalars *sc) {
+    sc->epsv2_max = 0;
+    sc->dt_min    = ~0ull;
+    sc->sum_v2    = 0;
+}
 
 enum KernelFlags : u32 {
     kFlagStackOverflow = 1u,
@@ -127,7 +135,6 @@ struct Ctx {
     DevBuf rank_of;            // merged id -> rank
     DevBuf sx, sy, sz, sh;     // positions, h (tree build time)
     DevBuf row_rank, row_local; // local rows in rank order
-    DevBuf row_flags, row_offsets;
 
     // ---- neighbour cache
     u64 leaf_csr_total = 0, csr_total = 0;
@@ -219,8 +226,7 @@ struct ProfScope {
 // kept, so only builds whose sorted padding is never exported may ask for it)
 cudaError_t tree_build(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
                        u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort = false);
-cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax);
-cudaError_t bbox_from_merged(Ctx &c, u32 n); // reduce mx/my/mz -> widened d_bbox
+cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax, int key_bits);
 cudaError_t sync_scalars(Ctx &c);            // copy Scalars to pinned host, wait
 
 // neigh.cu
@@ -234,7 +240,8 @@ cudaError_t tree_query(Ctx &c, const f64 *qx, const f64 *qy, const f64 *qz, u32 
 // ghosts.cu
 cudaError_t periodic_ghosts(Ctx &c, const f64 *x, const f64 *y, const f64 *z, u32 vs,
                             const f64 *h, u32 n, const f64 *bmin, const f64 *bmax, f64 htol);
+// bbox: also set d_bbox to the merged positions' widened box, for 32-bit keys
 cudaError_t merge_positions(Ctx &c, const f64 *x, const f64 *y, const f64 *z, u32 vs,
-                            const f64 *h, u32 n);
+                            const f64 *h, u32 n, bool bbox = false);
 
 } // namespace gbsph

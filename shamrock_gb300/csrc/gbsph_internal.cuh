@@ -152,6 +152,22 @@ __device__ __forceinline__ void raise_u32(u32 *p, u32 v) {
     if (v > __ldcg(p)) atomicMax(p, v);
 }
 
+// True in every thread of the block that comes here last of its grid, after all blocks'
+// writes; the counter is back at zero then.  One atomic a block on one address, so for grids
+// of some hundred blocks.
+__device__ __forceinline__ bool last_block(u32 *ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 inline u32 div_up(u64 a, u64 b) { return (u32) ((a + b - 1) / b); }
 
 // ------------------------------------------------------------------ device buffers
@@ -199,8 +215,5 @@ struct __align__(16) NodeBox {
 // Exclusive prefix sum of n u32 values; writes the grand total to *total_dev.
 cudaError_t scan_exclusive_u32(
     const u32 *in, u32 *out, u32 n, u32 *total_dev, DevBuf &scratch, cudaStream_t s);
-// Exclusive prefix sum of n u8 flags into u32 offsets (+ total).
-cudaError_t scan_exclusive_flags(
-    const u8 *in, u32 *out, u32 n, u32 *total_dev, DevBuf &scratch, cudaStream_t s);
 
 } // namespace gbsph

@@ -13,7 +13,7 @@
 // Rows are local particles in Morton order; entries are ranks, so a row lists its
 // neighbours in exactly the reference order (ascending leaf, then in-leaf order).
 
-#include "gbsph_ctx.cuh"
+#include "compact.cuh"
 #include "split64.cuh"
 
 #include <algorithm>
@@ -183,26 +183,6 @@ __global__ void k_leaf_fill(TreeView t, const u32 *__restrict__ off, uint2 *__re
 // separation s = max(n.lo - a.hi, a.lo - n.hi).  The FP32 estimate of s carries at most
 // ~2e-7 of the largest coordinate M plus 1e-7 relative; outside a band of
 // 1e-6 (M + R) the FP32 answer is certain, inside it the FP64 criterion decides.
-__global__ void k_boxes_f32(const NodeBox *__restrict__ b, u32 T, NodeBoxF *__restrict__ f) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= T) return;
-    NodeBox v = b[i];
-    f[i].lo = make_float4(__double2float_rn(v.lo[0]), __double2float_rn(v.lo[1]),
-                          __double2float_rn(v.lo[2]), __double2float_rn(__dmul_rn(v.rint, kRkern)));
-    f[i].hi = make_float4(__double2float_rn(v.hi[0]), __double2float_rn(v.hi[1]),
-                          __double2float_rn(v.hi[2]), 0.f);
-}
-
-__global__ void k_node_pairs(TreeView t, const NodeBoxF *__restrict__ fb, NodePairF *__restrict__ rec) {
-    u32 n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= t.off()) return; // internal nodes 0 .. L - 2
-    u32 l = t.left(n), r = t.right(n);
-    NodeBoxF bl = fb[l], br = fb[r];
-    bl.hi.w = __uint_as_float(l);
-    br.hi.w = __uint_as_float(r);
-    rec[n]  = NodePairF{bl, br};
-}
-
 // Stage 1 over the child-pair records.  A popped internal node loads both children's
 // boxes in one record and tests them together, pushing those that pass (right, then
 // left, so the left subtree is walked first); a popped leaf has passed and is
@@ -461,22 +441,30 @@ __global__ void __launch_bounds__(128) k_leaf_lists_wide(TreeView t, const NodeB
     off[l] = base;
 }
 
+// what a cache build accumulates into: no owned row, no threshold, no flag, no entry
+__global__ void k_cache_init(u32 L, u32 *__restrict__ head, u32 *__restrict__ leaf_thr, Scalars *sc) {
+    u32 l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l == 0) sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = 0, sc->csr_entries = 0;
+    if (l >= L) return;
+    head[l]     = kNone;
+    leaf_thr[l] = 0;
+}
+
 // ---- rows: local particles in rank order
-__global__ void k_row_flags(const u32 *__restrict__ sort_index, u32 N, u32 n_local,
-                            u8 *__restrict__ flags) {
-    u32 r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= N) return;
-    flags[r] = sort_index[r] < n_local ? 1 : 0;
-}
-__global__ void k_rows(const u32 *__restrict__ sort_index, const u8 *__restrict__ flags,
-                       const u32 *__restrict__ offs, u32 N, u32 *__restrict__ row_rank,
-                       u32 *__restrict__ row_local) {
-    u32 r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= N || !flags[r]) return;
-    u32 row        = offs[r];
-    row_rank[row]  = r;
-    row_local[row] = sort_index[r];
-}
+struct RowFlag {
+    const u32 *sort_index;
+    u32 n_local;
+    __device__ __forceinline__ bool operator()(u32 r) const { return sort_index[r] < n_local; }
+};
+struct RowPlace {
+    const u32 *sort_index;
+    u32 *row_rank, *row_local;
+    __device__ __forceinline__ void operator()(u32 r, u32 row) const {
+        row_rank[row]  = r;
+        row_local[row] = sort_index[r];
+    }
+    __device__ __forceinline__ void end(u32) const {}
+};
 
 // ---- owner leaf: max leaf index whose box contains the point (inclusive bounds),
 // i.e. the last leaf the reference's left-first DFS reports (NeighbourCache.cpp:419-443).
@@ -792,19 +780,12 @@ cudaError_t build_rows(Ctx &c, u32 n_local) {
     cudaStream_t s = c.stream;
     cudaError_t e;
     u32 N = c.n_obj;
-    if ((e = c.row_flags.ensure(N, s)) != cudaSuccess) return e;
-    if ((e = c.row_offsets.ensure(sizeof(u32) * (size_t) N, s)) != cudaSuccess) return e;
     if ((e = c.row_rank.ensure(sizeof(u32) * (size_t) n_local, s)) != cudaSuccess) return e;
     if ((e = c.row_local.ensure(sizeof(u32) * (size_t) n_local, s)) != cudaSuccess) return e;
-    { k_row_flags<<<div_up(N, 256), 256, 0, s>>>(c.sort_index.as<u32>(), N, n_local,
-                                               c.row_flags.as<u8>()); GBSPH_COUNTED; }
-    Scalars *dsc = c.d_scalars.as<Scalars>();
-    if ((e = scan_exclusive_flags(c.row_flags.as<u8>(), c.row_offsets.as<u32>(), N, &dsc->total2,
-                                  c.scan_scratch, s)) != cudaSuccess)
+    const u32 *si = c.sort_index.as<u32>();
+    if ((e = compact(c, RowFlag{si, n_local}, RowPlace{si, c.row_rank.as<u32>(), c.row_local.as<u32>()}, N,
+                     &c.d_scalars.as<Scalars>()->total2)) != cudaSuccess)
         return e;
-    { k_rows<<<div_up(N, 256), 256, 0, s>>>(c.sort_index.as<u32>(), c.row_flags.as<u8>(),
-                                          c.row_offsets.as<u32>(), N, c.row_rank.as<u32>(),
-                                          c.row_local.as<u32>()); GBSPH_COUNTED; }
     c.n_local = n_local;
     return cudaGetLastError();
 }
@@ -824,11 +805,6 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // Stage 1 in one pass into c.leaf_cap slots per leaf; if a leaf has more candidates
     // the pass is rerun with slots that fit, or, past the slot budget, the exact
     // two-pass build runs.
-    // flags, leaf_cnt_max and row_cnt_max are adjacent u32 fields of Scalars
-    static_assert(offsetof(Scalars, leaf_cnt_max) == offsetof(Scalars, flags) + 4 &&
-                      offsetof(Scalars, row_cnt_max) == offsetof(Scalars, flags) + 8,
-                  "Scalars field order");
-    if ((e = cudaMemsetAsync(&dsc->flags, 0, 3 * sizeof(u32), s)) != cudaSuccess) return e;
     if (c.leaf_cap == 0) c.leaf_cap = kLeafCap;
     const u64 budget = c.slot_budget ? c.slot_budget : kMaxSlotBytes;
     auto slots_ok = [&](u64 rows, u32 cap, u64 esize = 4) {
@@ -836,14 +812,9 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     };
     const bool s1_one_pass = slots_ok(L, c.leaf_cap, sizeof(uint2));
     // FP32 node boxes and the child-pair records the traversals read (the FP64 boxes
-    // decide inside the rounding band)
-    const u32 T = 2 * L - 1;
-    if ((e = c.fboxes.ensure(sizeof(NodeBoxF) * (size_t) T, s)) != cudaSuccess) return e;
-    if ((e = c.fpairs.ensure(sizeof(NodePairF) * (size_t) L, s)) != cudaSuccess) return e;
-    { k_boxes_f32<<<div_up(T, 256), 256, 0, s>>>(c.boxes.as<NodeBox>(), T, c.fboxes.as<NodeBoxF>()); GBSPH_COUNTED; }
+    // decide inside the rounding band), made with the boxes
     const NodeBoxF *fb = c.fboxes.as<NodeBoxF>();
     const NodePairF *rec = c.fpairs.as<NodePairF>();
-    if (L > 1) { k_node_pairs<<<div_up(L - 1, 256), 256, 0, s>>>(t, fb, c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
     // Stage 1 on the 8-ary hierarchy (built here, three levels per launch) while a thread per
     // leaf would leave an SM fewer than 512 threads: the binary walk is a chain of dependent
     // loads, 113 us for 1,399 leaves and 219 us for 35,981 against 36 and 139 us; from about
@@ -875,10 +846,9 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // leaves that own no row); the cache is unchanged.
     if ((e = c.next_row.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
     if ((e = c.leaf_head.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(c.leaf_head.p, 0xff, sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = c.leaf_thr.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(c.leaf_thr.p, 0, sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     u32 *leaf_thr = c.leaf_thr.as<u32>();
+    { k_cache_init<<<div_up(L, 256), 256, 0, s>>>(L, c.leaf_head.as<u32>(), leaf_thr, dsc); GBSPH_COUNTED; }
     if (n) {
         ProfScope ps(c, kProfOwner, n);
         { k_owner<<<div_up(n, 128), 128, 0, s>>>(t, fb, rec, c.row_rank.as<u32>(), n, c.sx.as<f64>(),
@@ -948,7 +918,6 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     bool one_pass = slots_fit(c.row_cap);
     if (one_pass)
         if ((e = c.csr_ent.ensure(sizeof(u32) * ((size_t) n * c.row_cap + 4), s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(&dsc->csr_entries, 0, sizeof(u64), s)) != cudaSuccess) return e;
     // launch helper for the stage-2 kernel family: a warp per leaf, in four times the five
     // blocks that an SM holds (41 KB of candidates each; with one such grid the leaves'
     // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics

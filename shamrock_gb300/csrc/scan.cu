@@ -122,9 +122,4 @@ cudaError_t scan_exclusive_u32(
     return scan_impl<u32>(in, out, n, total_dev, scratch, s);
 }
 
-cudaError_t scan_exclusive_flags(
-    const u8 *in, u32 *out, u32 n, u32 *total_dev, DevBuf &scratch, cudaStream_t s) {
-    return scan_impl<u8>(in, out, n, total_dev, scratch, s);
-}
-
 } // namespace gbsph

@@ -291,8 +291,9 @@ __global__ void k_gather_eos(const u32 *__restrict__ sort_index, u32 N, u32 n_lo
                              const f64 *__restrict__ omega, f64 pmass, EosParams eos, f64 alpha_AV,
                              const f64 *__restrict__ sx, const f64 *__restrict__ sy,
                              const f64 *__restrict__ sz, f64 *__restrict__ scs,
-                             f64 *__restrict__ rec) {
+                             f64 *__restrict__ rec, Scalars *sc) {
     u32 r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r == 0) reset_corrector(sc);
     if (r >= N) return;
     u32 id  = sort_index[r];
     u32 src = id < n_local ? id : ghost_src[id - n_local];
@@ -1165,18 +1166,17 @@ __global__ void k_scatter_rows(u32 n, const u32 *__restrict__ row_local, const f
     dst[row_local[t]] = src[t];
 }
 
-__global__ void k_gather_rows(u32 n, const u32 *__restrict__ row_rank, const f64 *__restrict__ src,
-                              f64 *__restrict__ dst, f64 *__restrict__ dst2) {
+// start of the h iteration: both h of a row, its eps, and the reductions' identities
+__global__ void k_h_start(u32 n, const u32 *__restrict__ row_rank, const f64 *__restrict__ h_rank,
+                          f64 *__restrict__ h_old, f64 *__restrict__ h_new, f64 *__restrict__ eps, f64 eps0,
+                          Scalars *sc) {
     u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) sc->eps_max = 0, sc->eps_min = ~0ull, sc->iters_max = 0;
     if (t >= n) return;
-    f64 v  = src[row_rank[t]];
-    dst[t] = v;
-    if (dst2) dst2[t] = v;
-}
-
-__global__ void k_fill(u32 n, f64 *__restrict__ dst, f64 v) {
-    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) dst[t] = v;
+    const f64 v = h_rank[row_rank[t]];
+    h_old[t]    = v;
+    h_new[t]    = v;
+    eps[t]      = eps0;
 }
 
 } // namespace
@@ -1208,7 +1208,7 @@ cudaError_t gather_eos64(Ctx &c, u32 N, u32 n_local, const LocalFields &lf, cons
     { k_gather_eos<<<div_up(N, 256), 256, 0, c.stream>>>(
         c.sort_index.as<u32>(), N, n_local, c.ghost_src.as<u32>(), lf.h, lf.u, lf.vx, lf.vy, lf.vz,
         lf.vs, omega_local, pmass, eos, alpha_AV, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
-        c.scs.as<f64>(), c.rec64.as<f64>()); GBSPH_COUNTED; }
+        c.scs.as<f64>(), c.rec64.as<f64>(), c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 cudaError_t stage_alpha64(Ctx &c, u32 N, u32 n_local, const f64 *alpha_local) {
@@ -1377,12 +1377,9 @@ cudaError_t scatter_rows(Ctx &c, u32 n, const f64 *src, f64 *dst) {
     { k_scatter_rows<<<div_up(n, 256), 256, 0, c.stream>>>(n, c.row_local.as<u32>(), src, dst); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
-cudaError_t gather_rows(Ctx &c, u32 n, const f64 *src_rank, f64 *dst, f64 *dst2) {
-    { k_gather_rows<<<div_up(n, 256), 256, 0, c.stream>>>(n, c.row_rank.as<u32>(), src_rank, dst, dst2); GBSPH_COUNTED; }
-    return cudaGetLastError();
-}
-cudaError_t fill64(Ctx &c, u32 n, f64 *dst, f64 v) {
-    { k_fill<<<div_up(n, 256), 256, 0, c.stream>>>(n, dst, v); GBSPH_COUNTED; }
+cudaError_t h_start(Ctx &c, u32 n, const f64 *h_rank, f64 *h_old, f64 *h_new, f64 *eps, f64 eps0) {
+    { k_h_start<<<div_up(n, 256), 256, 0, c.stream>>>(n, c.row_rank.as<u32>(), h_rank, h_old, h_new, eps, eps0,
+                                                     c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 

@@ -105,7 +105,6 @@ cudaError_t mm97_update(Ctx &c, u32 n, const f64 *divv, const f64 *cs, const f64
 // dst[row_local[t]] = src[row_rank[t]] for the n pipeline rows
 cudaError_t rank_to_local64(Ctx &c, u32 n, const f64 *src_rank, f64 *dst);
 cudaError_t scatter_rows(Ctx &c, u32 n, const f64 *src, f64 *dst);
-cudaError_t gather_rows(Ctx &c, u32 n, const f64 *src_rank, f64 *dst, f64 *dst2);
-cudaError_t fill64(Ctx &c, u32 n, f64 *dst, f64 v);
+cudaError_t h_start(Ctx &c, u32 n, const f64 *h_rank, f64 *h_old, f64 *h_new, f64 *eps, f64 eps0);
 
 } // namespace gbsph

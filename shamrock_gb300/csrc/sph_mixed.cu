@@ -110,8 +110,9 @@ __global__ void k_gather_stage_mixed(const u32 *__restrict__ sort_index, u32 N, 
                                      const f64 *__restrict__ sx, const f64 *__restrict__ sy,
                                      const f64 *__restrict__ sz, float4 *__restrict__ P,
                                      float4 *__restrict__ H, f64 *__restrict__ h_rank,
-                                     StageAV av, float4 *__restrict__ E) {
+                                     StageAV av, float4 *__restrict__ E, Scalars *sc) {
     u32 r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r == 0) reset_corrector(sc);
     if (r >= N) return;
     u32 id  = sort_index[r];
     u32 src = id < n_local ? id : ghost_src[id - n_local];
@@ -1134,7 +1135,7 @@ cudaError_t gather_stage_mixed(Ctx &c, u32 N, u32 n_local, const LocalFields &lf
     { k_gather_stage_mixed<<<div_up(N, 256), 256, 0, c.stream>>>(
         c.sort_index.as<u32>(), N, n_local, c.ghost_src.as<u32>(), lf, omega_local, pmass, se,
         c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(), c.f_pos.as<float4>(),
-        c.f_aux0.as<float4>(), c.sh2.as<f64>(), av, E); GBSPH_COUNTED; }
+        c.f_aux0.as<float4>(), c.sh2.as<f64>(), av, E, c.d_scalars.as<Scalars>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 

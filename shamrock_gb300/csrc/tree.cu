@@ -11,7 +11,7 @@
 // The reference propagates node boxes with tree_depth full sweeps; here one
 // bottom-up pass with arrival counters produces the same exact min/max.
 
-#include "gbsph_ctx.cuh"
+#include "compact.cuh"
 #include "lean64.cuh"
 
 #include <type_traits>
@@ -55,15 +55,6 @@ struct Morton<u64> {
     __device__ static u64 encode(u64 x, u64 y, u64 z) { return expand(x) * 4 + expand(y) * 2 + expand(z); }
     __device__ static int clz(u64 v) { return __clzll((long long) v); }
 };
-
-__global__ void k_bbox_fact(BBox *bb, u32 val_count) {
-    if (threadIdx.x < 3) {
-        int c       = threadIdx.x;
-        bb->fact[c] = __ddiv_rn(__dsub_rn(bb->hi[c], bb->lo[c]), (f64) val_count);
-        const f64 f = bb->fact[c];
-        bb->inv[c]  = f > 1e-300 && f < 1e300 ? __ddiv_rn(1.0, f) : 0.0;
-    }
-}
 
 // 24 bytes read and 8 written a particle; bound by the FP64 pipe until the cell took two FP64
 // instructions a coordinate: 1,048,576 particles 81 -> 24 us, 8.5 M 590 -> 172 us.
@@ -365,30 +356,34 @@ __global__ void k_reduce_iter(const K *__restrict__ m, u32 cnt, const u8 *__rest
     out[i] = (!(delt_0 < delt_m && delt_mm < delt_m) && in[i]) ? 1 : 0;
 }
 
+// the kept split points become the leaves
+struct LeafFlag {
+    const u8 *f;
+    __device__ __forceinline__ bool operator()(u32 i) const { return f[i] != 0; }
+};
 template<class K>
-__global__ void k_compact_leaves(const u8 *__restrict__ flags, const u32 *__restrict__ offs, u32 cnt,
-                                 const K *__restrict__ m, u32 *__restrict__ reduc,
-                                 K *__restrict__ reduced) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cnt) return;
-    if (flags[i]) {
-        u32 o      = offs[i];
+struct LeafPlace {
+    const K *m;
+    u32 *reduc;
+    K *reduced;
+    u32 cnt;
+    __device__ __forceinline__ void operator()(u32 i, u32 o) const {
         reduc[o]   = i;
         reduced[o] = m[i];
     }
-}
-
-__global__ void k_reduc_tail(u32 *reduc, const u32 *L, u32 cnt) {
-    reduc[*L]     = cnt;
-    reduc[*L + 1] = 0;
-}
+    __device__ __forceinline__ void end(u32 L) const {
+        reduc[L]     = cnt;
+        reduc[L + 1] = 0;
+    }
+};
 
 // ---------------------------------------------------------------- Karras
 template<class K>
 __global__ void k_karras(const K *__restrict__ m, u32 L, u32 *__restrict__ lchild,
                          u32 *__restrict__ rchild, u8 *__restrict__ lflag, u8 *__restrict__ rflag,
-                         u32 *__restrict__ endrange, u32 *__restrict__ parent) {
+                         u32 *__restrict__ endrange, u32 *__restrict__ parent, u32 *__restrict__ visit) {
     u32 ui = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ui < L) visit[ui] = 0; // the counters of the pass over the boxes
     if (ui == 0) parent[0] = kNone;
     if (ui + 1 >= L) return;
     i32 i = (i32) ui;
@@ -466,15 +461,18 @@ __device__ __forceinline__ void store_box(NodeBox *b, const BoxKeys &k) {
 }
 
 // One thread per leaf; of two siblings the one that arrives last unites both boxes and goes
-// on up, with its own box in registers.  The links of the parent are fetched beside the
+// on up, with its own box in registers, and writes the FP32 copies and the child-pair records
+// that the neighbour search walks (passes of their own over the boxes otherwise).  The links of the parent are fetched beside the
 // counter, as a level costs the latencies that follow each other (about 1.5 us).
-// 1,048,576 particles 117 -> 94 us, 8.5 M 471 -> 387 us.
+// 1,048,576 particles 117 -> 99 us, 8.5 M 471 -> 446 us, of which the copies and records take 5
+// and 59 (18 and 130 us as passes of their own).
 __global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 *__restrict__ sx,
                                 const f64 *__restrict__ sy, const f64 *__restrict__ sz,
                                 const f64 *__restrict__ sh, f64 htol, const u32 *__restrict__ lchild,
                                 const u32 *__restrict__ rchild, const u8 *__restrict__ lflag,
                                 const u8 *__restrict__ rflag, const u32 *__restrict__ parent,
-                                u32 *__restrict__ visit, NodeBox *__restrict__ boxes) {
+                                u32 *__restrict__ visit, NodeBox *__restrict__ boxes, NodeBoxF *__restrict__ fb,
+                                NodePairF *__restrict__ rec) {
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= L) return;
     const f64 big = 1.7976931348623157e308;
@@ -504,6 +502,12 @@ __global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 
     u32 off  = L - 1;
     u32 node = off + l;
     store_box(&boxes[node], k);
+    NodeBoxF f; // rounding is monotone, so a united box's FP32 copy is the union of the copies
+    f.lo = make_float4(narrow64(ordered_to_f64(k.lo[0])), narrow64(ordered_to_f64(k.lo[1])),
+                       narrow64(ordered_to_f64(k.lo[2])), narrow64(__dmul_rn(ordered_to_f64(k.rint), kRkern)));
+    f.hi = make_float4(narrow64(ordered_to_f64(k.hi[0])), narrow64(ordered_to_f64(k.hi[1])),
+                       narrow64(ordered_to_f64(k.hi[2])), 0.f);
+    fb[node] = f;
     __threadfence();
     u32 p = parent[node];
     while (p != kNone) {
@@ -512,7 +516,9 @@ __global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 
         const u32 up = parent[p];
         if (atomicAdd(&visit[p], 1u) == 0) return;
         __threadfence();
-        const double2 *s = (const double2 *) &boxes[a == node ? b : a];
+        const u32 sib    = a == node ? b : a;
+        const double2 *s = (const double2 *) &boxes[sib];
+        const float4 glo = __ldcg(&fb[sib].lo), ghi = __ldcg(&fb[sib].hi);
         const double2 s0 = __ldcg(s), s1 = __ldcg(s + 1), s2 = __ldcg(s + 2), s3 = __ldcg(s + 3);
         const f64 slo[3] = {s0.x, s0.y, s1.x}, shi[3] = {s2.x, s2.y, s3.x};
 #pragma unroll
@@ -524,53 +530,18 @@ __global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 
         if (is_nan_bits(ordered_to_f64(k.rint))) k.rint = sr;
         else if (!is_nan_bits(s1.y)) max_key(k.rint, sr);
         store_box(&boxes[p], k);
+        NodePairF pair{f, NodeBoxF{glo, ghi}};
+        if (a != node) pair = NodePairF{NodeBoxF{glo, ghi}, f};
+        pair.l.hi.w = __uint_as_float(a);
+        pair.r.hi.w = __uint_as_float(b);
+        rec[p]      = pair;
+        f.lo = make_float4(fminf(f.lo.x, glo.x), fminf(f.lo.y, glo.y), fminf(f.lo.z, glo.z), fmaxf(f.lo.w, glo.w));
+        f.hi = make_float4(fmaxf(f.hi.x, ghi.x), fmaxf(f.hi.y, ghi.y), fmaxf(f.hi.z, ghi.z), 0.f);
+        fb[p] = f;
         __threadfence();
         node = p;
         p    = up;
     }
-}
-
-// ---------------------------------------------------------------- bbox of merged positions
-__global__ void k_bbox_init(Scalars *sc) {
-    if (threadIdx.x < 3) {
-        sc->bbox_min[threadIdx.x] = ~0ull;
-        sc->bbox_max[threadIdx.x] = 0ull;
-    }
-}
-
-__global__ void k_bbox_reduce(const f64 *__restrict__ x, const f64 *__restrict__ y,
-                              const f64 *__restrict__ z, u32 n, Scalars *sc) {
-    u64 mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0, 0, 0};
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        u64 o[3] = {f64_to_ordered(x[i]), f64_to_ordered(y[i]), f64_to_ordered(z[i])};
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            mn[c] = o[c] < mn[c] ? o[c] : mn[c];
-            mx[c] = o[c] > mx[c] ? o[c] : mx[c];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        u64 a = block_reduce(mn[c], OpMinU64{}, ~0ull);
-        u64 b = block_reduce(mx[c], OpMaxU64{}, 0ull);
-        if (threadIdx.x == 0) {
-            atomicMin((unsigned long long *) &sc->bbox_min[c], (unsigned long long) a);
-            atomicMax((unsigned long long *) &sc->bbox_max[c], (unsigned long long) b);
-        }
-    }
-}
-
-// nextafter widening (BuildTrees.cpp:50-55) + Morton grid step
-__global__ void k_bbox_finalize(const Scalars *sc, BBox *bb, u32 val_count) {
-    int c = threadIdx.x;
-    if (c >= 3) return;
-    f64 lo    = ordered_to_f64(sc->bbox_min[c]);
-    f64 hi    = ordered_to_f64(sc->bbox_max[c]);
-    lo        = nextafter(lo, -__longlong_as_double(0x7ff0000000000000ll));
-    hi        = nextafter(hi, __longlong_as_double(0x7ff0000000000000ll));
-    bb->lo[c] = lo;
-    bb->hi[c] = hi;
-    bb->fact[c] = __ddiv_rn(__dsub_rn(hi, lo), (f64) val_count);
 }
 
 // Up to this many keys (padded to a power of two) the network sorts at once.  Where keys are
@@ -601,7 +572,6 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     ENS(c.sort_index, sizeof(u32) * P);
     ENS(c.flags_a, n);
     ENS(c.flags_b, n);
-    ENS(c.offsets, sizeof(u32) * (size_t) n);
     ENS(c.reduc, sizeof(u32) * ((size_t) n + 2));
     ENS(c.reduced, sizeof(K) * (size_t) n);
     ENS(c.rank_of, sizeof(u32) * (size_t) n);
@@ -638,12 +608,9 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
             if (it % 2 == 0) { k_reduce_iter<K><<<div_up(n, T), T, 0, s>>>(keys, n, fb, fa); GBSPH_COUNTED; }
             else { k_reduce_iter<K><<<div_up(n, T), T, 0, s>>>(keys, n, fa, fb); GBSPH_COUNTED; }
         }
-        if ((e = scan_exclusive_flags(fin, c.offsets.as<u32>(), n, &dsc->total, c.scan_scratch, s)) !=
-            cudaSuccess)
+        if ((e = compact(c, LeafFlag{fin}, LeafPlace<K>{keys, c.reduc.as<u32>(), c.reduced.as<K>(), n}, n,
+                         &dsc->total)) != cudaSuccess)
             return e;
-        { k_compact_leaves<K><<<div_up(n, T), T, 0, s>>>(fin, c.offsets.as<u32>(), n, keys,
-                                                       c.reduc.as<u32>(), c.reduced.as<K>()); GBSPH_COUNTED; }
-        { k_reduc_tail<<<1, 1, 0, s>>>(c.reduc.as<u32>(), &dsc->total, n); GBSPH_COUNTED; }
         if (prof_tree >= 0) prof_end(c, prof_tree);
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
         if (attempt == 0 && !c.h_scalars->dup_keys) break;
@@ -661,18 +628,19 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     ENS(c.parent, sizeof(u32) * Tn);
     ENS(c.visit, sizeof(u32) * (I + 1));
     ENS(c.boxes, sizeof(NodeBox) * Tn);
+    ENS(c.fboxes, sizeof(NodeBoxF) * Tn);
+    ENS(c.fpairs, sizeof(NodePairF) * (size_t) L);
 #undef ENS
     { k_karras<K><<<div_up(L, T), T, 0, s>>>(c.reduced.as<K>(), L, c.lchild.as<u32>(),
                                            c.rchild.as<u32>(), c.lflag.as<u8>(), c.rflag.as<u8>(),
-                                           c.endrange.as<u32>(), c.parent.as<u32>()); GBSPH_COUNTED; }
+                                           c.endrange.as<u32>(), c.parent.as<u32>(), c.visit.as<u32>()); GBSPH_COUNTED; }
     { k_permute<<<div_up(n, T), T, 0, s>>>(vals, n, x, y, z, h, c.sx.as<f64>(), c.sy.as<f64>(),
                                          c.sz.as<f64>(), c.sh.as<f64>(), c.rank_of.as<u32>()); GBSPH_COUNTED; }
-    if ((e = cudaMemsetAsync(c.visit.p, 0, sizeof(u32) * (I + 1), s)) != cudaSuccess) return e;
     { k_leaf_boxes_up<<<div_up(L, T), T, 0, s>>>(
         c.reduc.as<u32>(), L, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
         h ? c.sh.as<f64>() : nullptr, htol, c.lchild.as<u32>(), c.rchild.as<u32>(),
         c.lflag.as<u8>(), c.rflag.as<u8>(), c.parent.as<u32>(), c.visit.as<u32>(),
-        c.boxes.as<NodeBox>()); GBSPH_COUNTED; }
+        c.boxes.as<NodeBox>(), c.fboxes.as<NodeBoxF>(), c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 
@@ -685,38 +653,23 @@ cudaError_t sync_scalars(Ctx &c) {
     return cudaStreamSynchronize(c.stream);
 }
 
-cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax) {
+cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax, int key_bits) {
+    const f64 cells = (f64) (key_bits == 64 ? Morton<u64>::val_count : Morton<u32>::val_count);
     BBox b{};
     for (int k = 0; k < 3; k++) {
-        b.lo[k] = bmin[k];
-        b.hi[k] = bmax[k];
+        b.lo[k]   = bmin[k];
+        b.hi[k]   = bmax[k];
+        b.fact[k] = (bmax[k] - bmin[k]) / cells;
+        b.inv[k]  = b.fact[k] > 1e-300 && b.fact[k] < 1e300 ? 1.0 / b.fact[k] : 0.0;
     }
     cudaError_t e = cudaMemcpyAsync(c.d_bbox.p, &b, sizeof(BBox), cudaMemcpyHostToDevice, c.stream);
     if (e != cudaSuccess) return e;
-    // grid step for both key widths is filled by tree_build (depends on key width)
     return cudaStreamSynchronize(c.stream);
-}
-
-cudaError_t bbox_from_merged(Ctx &c, u32 n) {
-    Scalars *dsc = c.d_scalars.as<Scalars>();
-    ProfScope ps(c, kProfMerge, 0);
-    { k_bbox_init<<<1, 32, 0, c.stream>>>(dsc); GBSPH_COUNTED; }
-    u32 blocks = div_up(n, 256);
-    if (blocks > 1216) blocks = 1216;
-    if (blocks == 0) blocks = 1;
-    { k_bbox_reduce<<<blocks, 256, 0, c.stream>>>(c.mx.as<f64>(), c.my.as<f64>(), c.mz.as<f64>(), n,
-                                                dsc); GBSPH_COUNTED; }
-    { k_bbox_finalize<<<1, 32, 0, c.stream>>>(dsc, c.d_bbox.as<BBox>(), Morton<u32>::val_count); GBSPH_COUNTED; }
-    return cudaGetLastError();
 }
 
 cudaError_t tree_build(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
                        u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort) {
-    if (key_bits == 64) {
-        { k_bbox_fact<<<1, 32, 0, c.stream>>>(c.d_bbox.as<BBox>(), Morton<u64>::val_count); GBSPH_COUNTED; }
-        return tree_build_impl<u64>(c, x, y, z, h, n, level, htol, morton_count, false);
-    }
-    { k_bbox_fact<<<1, 32, 0, c.stream>>>(c.d_bbox.as<BBox>(), Morton<u32>::val_count); GBSPH_COUNTED; }
+    if (key_bits == 64) return tree_build_impl<u64>(c, x, y, z, h, n, level, htol, morton_count, false);
     return tree_build_impl<u32>(c, x, y, z, h, n, level, htol, morton_count, fast_sort);
 }
 
@@ -771,11 +724,9 @@ __global__ void k_export_boxes(const NodeBox *__restrict__ b, u32 T, f64 *__rest
 cudaError_t morton_codes_dev(Ctx &c, const f64 *x, const f64 *y, const f64 *z, u32 n, u32 P,
                              int key_bits, void *out) {
     if (key_bits == 64) {
-        { k_bbox_fact<<<1, 32, 0, c.stream>>>(c.d_bbox.as<BBox>(), Morton<u64>::val_count); GBSPH_COUNTED; }
         { k_morton_only<u64><<<div_up(P, 256), 256, 0, c.stream>>>(x, y, z, n, P, c.d_bbox.as<BBox>(),
                                                                  (u64 *) out); GBSPH_COUNTED; }
     } else {
-        { k_bbox_fact<<<1, 32, 0, c.stream>>>(c.d_bbox.as<BBox>(), Morton<u32>::val_count); GBSPH_COUNTED; }
         { k_morton_only<u32><<<div_up(P, 256), 256, 0, c.stream>>>(x, y, z, n, P, c.d_bbox.as<BBox>(),
                                                                  (u32 *) out); GBSPH_COUNTED; }
     }
