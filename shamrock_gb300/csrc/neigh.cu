@@ -553,14 +553,18 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // exact FP64 test decides, so the cache is the FP64 one.
 //
 // A warp walks one leaf: the rows that the leaf owns share its candidates, so the warp
-// expands the leaf's rank runs once, loads each candidate's record once, coalesced, and
-// keeps its position relative to the leaf in shared memory; a row is then tested against 32
-// candidates at a time and the accepted lanes are placed by a ballot, in rank order.  Bound
-// by instruction issue (about 60 a row and 32 candidates); a thread per row loads a record
-// per candidate and row, 10 L1 wavefronts a request, its lanes diverge over runs of
-// different lengths, and a state of 2,048 particles runs on 64 warps: 104 -> 18 us there,
-// 131,072 particles 181 -> 138 us, 1,048,576 1000 -> 875 us, disc 1146 -> 916 us,
-// homogeneous 8.5 M 5.57 -> 5.36 ms.  Relative positions are rounded to FP32:
+// expands the leaf's rank runs once, loads each candidate's record once, coalesced, drops
+// those out of reach of the rows' box and keeps the others' positions relative to the leaf in
+// shared memory; a row is then tested against 64 of them at a time and the accepted lanes are
+// placed by ballots, in rank order.  Bound by instruction issue (76 % of the peak at 25 a row
+// and 32 candidates).  131,072 / 1,048,576 / homogeneous 8.5 M / clustered 3 M / disc 1 M:
+//   a thread per row                       181 / 1000 us / 5.57 ms / - / 1146 us
+//   32 at a time, 48 registers             137 /  880    / 5.37 / 1.92 /  915
+//   64 at a time, 64 registers             123 /  760    / 4.65 / 1.70 /  804
+//   and the rows' box                      118 /  684    / 4.73 / 1.67 /  801
+// (a thread per row loads a record per candidate and row, 10 L1 wavefronts a request, and its
+// lanes diverge; at 48 registers, five blocks an SM, either of the last two steps is a loss).
+// Relative positions are rounded to FP32:
 // with S the largest of the rows' own, r^2 / thr of a pair near the threshold errs by at
 // most 2.1e-7 (2 S / sqrt(thr) + 2), and the hi/lo records themselves by 2.5e-14 M /
 // sqrt(thr) for coordinates of size M; a row for which these do not stay well inside the
@@ -585,10 +589,17 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     return r;
 }
 
+// least of the lanes' floats (no NaN; -0 and 0 alike)
+__device__ __forceinline__ float warp_min(float v) {
+    const u32 b = __float_as_uint(v), o = b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+    const u32 m = __reduce_min_sync(0xffffffffu, o);
+    return __uint_as_float(m ^ ((m >> 31) ? 0x80000000u : 0xffffffffu));
+}
+
 constexpr u32 kCandBlock = 256; // candidates of a leaf held at a time
 
 template<int MODE>
-__global__ void __launch_bounds__(256, 5) k_part_cache(
+__global__ void __launch_bounds__(256, 4) k_part_cache(
     u32 L, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
     const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
     const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
@@ -602,7 +613,7 @@ __global__ void __launch_bounds__(256, 5) k_part_cache(
     constexpr u32 kAll = 0xffffffffu;
     float4 *cand = s_cand[wid];
     u32 *ids     = s_id[wid];
-    const float lo_f = 1.f - 1e-5f, band = (1.f + 1e-5f) / (1.f - 1e-5f);
+    const float lo_f = 1.f - 1e-5f, band = (1.f + 1e-5f) / (1.f - 1e-5f), big = 3e38f;
     u32 c_max = 0;
     u64 c_sum = 0;
     for (u32 l = blockIdx.x * 8 + wid; l < L; l += gridDim.x * 8) {
@@ -628,7 +639,7 @@ __global__ void __launch_bounds__(256, 5) k_part_cache(
                         oz = __shfl_sync(kAll, Ph.z, 0);
             const float xa = __fadd_rn(__fsub_rn(Ph.x, ox), Pl.x), ya = __fadd_rn(__fsub_rn(Ph.y, oy), Pl.y),
                         za = __fadd_rn(__fsub_rn(Ph.z, oz), Pl.z), thr = Pl.w;
-            float tlo; // the lower end of the band; NaN: decide in FP64
+            float tlo, tmax; // the lower end of the band, and the rows' largest; NaN: decide in FP64
             {
                 const float mine = lane < m ? fmaxf(fmaxf(fabsf(xa), fabsf(ya)), fabsf(za)) : 0.f;
                 const float S    = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(mine)));
@@ -636,7 +647,15 @@ __global__ void __launch_bounds__(256, 5) k_part_cache(
                 // 2 S / sqrt(thr) + 2 <= 24 and M / sqrt(thr) <= 1e8
                 const bool ok = S * S <= 121.f * thr && M * M <= 1e16f * thr && thr > 1e-30f;
                 tlo           = ok ? thr * lo_f : __int_as_float(0x7fc00000);
+                tmax          = __uint_as_float(__reduce_max_sync(kAll, lane < m && ok ? __float_as_uint(tlo) : 0u));
+                if (__any_sync(kAll, lane < m && !ok)) tmax = __int_as_float(0x7fc00000);
             }
+            // The rows' box.  Rounding is monotone, so for a candidate outside it every row's
+            // rounded separation is at least the box's: one beyond the band of the largest
+            // threshold from the box is beyond its own band from every row.
+            const float lox = warp_min(lane < m ? xa : big), hix = -warp_min(lane < m ? -xa : big);
+            const float loy = warp_min(lane < m ? ya : big), hiy = -warp_min(lane < m ? -ya : big);
+            const float loz = warp_min(lane < m ? za : big), hiz = -warp_min(lane < m ? -za : big);
             for (u32 kb = 0; kb < nk; kb += 32) {
                 const uint2 run = kb + lane < nk ? leaf_ent[k0 + kb + lane] : make_uint2(0, 0);
                 const u32 len   = run.y - run.x;
@@ -647,52 +666,69 @@ __global__ void __launch_bounds__(256, 5) k_part_cache(
                     if (lane >= o) end += v;
                 }
                 const u32 total = __shfl_sync(kAll, end, 31), start = end - len;
-                for (u32 t0 = 0; t0 < total; t0 += kCandBlock) {
-                    const u32 nb = min(kCandBlock, total - t0);
+                for (u32 t = 0; t < total;) {
+                    // candidates that no row can pair with are dropped here
+                    u32 nb = 0;
                     __syncwarp();
-                    for (u32 t = t0; t < t0 + nb; t += 32) {
+                    for (; t < total && nb + 32 <= kCandBlock; t += 32) {
                         // slot t + lane lies in the last run that starts at or before it
                         const u32 d    = start - t;
                         const u32 here = __reduce_or_sync(kAll, len && d < 32 ? 1u << d : 0u);
                         const u32 past = __popc(__ballot_sync(kAll, len && start < t));
                         const u32 j    = past + __popc(here & upto) - 1;
                         const u32 b    = __shfl_sync(kAll, run.x - start, j) + t + lane;
-                        // (slots past the end: far away)
-                        float4 q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
-                        if (t + lane < total) {
+                        bool keep      = t + lane < total;
+                        float4 q;
+                        if (keep) {
                             const F8 rec = ldg256(&P[2 * (size_t) b]);
                             q = make_float4(__fadd_rn(__fsub_rn(rec.a.x, ox), rec.b.x),
                                             __fadd_rn(__fsub_rn(rec.a.y, oy), rec.b.y),
                                             __fadd_rn(__fsub_rn(rec.a.z, oz), rec.b.z), rec.b.w * lo_f);
+                            const float gx = fmaxf(fmaxf(lox - q.x, q.x - hix), 0.f);
+                            const float gy = fmaxf(fmaxf(loy - q.y, q.y - hiy), 0.f);
+                            const float gz = fmaxf(fmaxf(loz - q.z, q.z - hiz), 0.f);
+                            const float g2 = __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, gx * gx));
+                            keep           = !(g2 > max_nan(tmax, q.w) * band);
                         }
-                        cand[t - t0 + lane] = q;
-                        ids[t - t0 + lane]  = t + lane < total ? b : kNone;
+                        const u32 kept = __ballot_sync(kAll, keep), at = nb + __popc(kept & below);
+                        if (keep) cand[at] = q, ids[at] = b;
+                        nb += __popc(kept);
                     }
+                    // the last ones are filled up far away
+                    for (u32 k = nb + lane; k < ((nb + 63u) & ~63u); k += 32)
+                        cand[k] = make_float4(1e30f, 1e30f, 1e30f, 0.f), ids[k] = kNone;
                     __syncwarp();
                     for (u32 r = 0; r < m; r++) {
                         const float x = __shfl_sync(kAll, xa, r), y = __shfl_sync(kAll, ya, r),
                                     z = __shfl_sync(kAll, za, r);
                         // rows decided in FP64 alone: no candidate is certain
                         const float ta = __shfl_sync(kAll, tlo, r);
-                        const u32 rr   = __shfl_sync(kAll, ra, r);
                         u32 *out       = ent + __shfl_sync(kAll, w, r);
                         u32 cr         = __shfl_sync(kAll, c, r);
 #pragma unroll 1
-                        for (u32 t = 0; t < nb; t += 32) {
-                            const float4 q = cand[t + lane];
-                            const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
-                            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-                            const float tm = max_nan(ta, q.w);
-                            const bool sure = r2 < tm, open = !sure & !(r2 > tm * band);
-                            u32 bits        = __ballot_sync(kAll, sure);
-                            if (__any_sync(kAll, open)) {
-                                const u32 b = open ? ids[t + lane] : kNone;
-                                bits |= __ballot_sync(kAll, b != kNone && pair_inside(sx, sy, sz, sh, h_tol, rr, b));
+                        for (u32 t = 0; t < nb; t += 64) {
+                            // 64 candidates at a time: the second 32 beyond nb are far away
+                            const float4 q0 = cand[t + lane], q1 = cand[t + 32 + lane];
+                            const float dx0 = x - q0.x, dy0 = y - q0.y, dz0 = z - q0.z;
+                            const float dx1 = x - q1.x, dy1 = y - q1.y, dz1 = z - q1.z;
+                            const float r20 = __fmaf_rn(dz0, dz0, __fmaf_rn(dy0, dy0, dx0 * dx0));
+                            const float r21 = __fmaf_rn(dz1, dz1, __fmaf_rn(dy1, dy1, dx1 * dx1));
+                            const float tm0 = max_nan(ta, q0.w), tm1 = max_nan(ta, q1.w);
+                            const bool sure0 = r20 < tm0, open0 = !sure0 & !(r20 > tm0 * band);
+                            const bool sure1 = r21 < tm1, open1 = !sure1 & !(r21 > tm1 * band);
+                            u32 bits0 = __ballot_sync(kAll, sure0), bits1 = __ballot_sync(kAll, sure1);
+                            if (__any_sync(kAll, open0 | open1)) {
+                                const u32 rr = __shfl_sync(kAll, ra, r);
+                                const u32 b0 = open0 ? ids[t + lane] : kNone, b1 = open1 ? ids[t + 32 + lane] : kNone;
+                                bits0 |= __ballot_sync(kAll, b0 != kNone && pair_inside(sx, sy, sz, sh, h_tol, rr, b0));
+                                bits1 |= __ballot_sync(kAll, b1 != kNone && pair_inside(sx, sy, sz, sh, h_tol, rr, b1));
                             }
-                            const u32 at   = cr + __popc(bits & below);
-                            if (MODE != kCount && (bits >> lane & 1u) && (MODE == kFill || at < cap))
-                                out[at] = ids[t + lane];
-                            cr += __popc(bits);
+                            const u32 at0 = cr + __popc(bits0 & below);
+                            cr += __popc(bits0);
+                            const u32 at1 = cr + __popc(bits1 & below);
+                            cr += __popc(bits1);
+                            if (MODE != kCount && (bits0 >> lane & 1u) && (MODE == kFill || at0 < cap)) out[at0] = ids[t + lane];
+                            if (MODE != kCount && (bits1 >> lane & 1u) && (MODE == kFill || at1 < cap)) out[at1] = ids[t + 32 + lane];
                         }
                         if (lane == r) c = cr;
                     }
@@ -918,13 +954,13 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     bool one_pass = slots_fit(c.row_cap);
     if (one_pass)
         if ((e = c.csr_ent.ensure(sizeof(u32) * ((size_t) n * c.row_cap + 4), s)) != cudaSuccess) return e;
-    // launch helper for the stage-2 kernel family: a warp per leaf, in four times the five
+    // launch helper for the stage-2 kernel family: a warp per leaf, in six times the four
     // blocks that an SM holds (41 KB of candidates each; with one such grid the leaves'
     // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics
     // on the totals, 10 ns each, take longer than the build)
     auto part = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
-        const u32 blocks   = std::min(div_up(L, 8), 20 * c.sms);
+        const u32 blocks   = std::min(div_up(L, 8), 24 * c.sms);
         { k_part_cache<MODE><<<blocks, 256, 0, s>>>(
             L, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
