@@ -118,9 +118,10 @@ __device__ __forceinline__ bool cella_neigh_b(const f64 amin[3], const f64 amax[
 struct LeafCrit {
     const TreeView &t;
     f64 amin[3], amax[3], amin_ext[3], amax_ext[3];
-    __device__ LeafCrit(const TreeView &tv, u32 leaf) : t(tv) {
+    __device__ LeafCrit(const TreeView &tv, u32 leaf) : LeafCrit(tv, tv.off() + leaf, 0) {}
+    __device__ LeafCrit(const TreeView &tv, u32 leaf_node, int) : t(tv) {
         f64 r;
-        load_box(&t.boxes[t.off() + leaf], amin, amax, r);
+        load_box(&t.boxes[leaf_node], amin, amax, r);
         f64 ra = __dmul_rn(r, kRkern);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -143,15 +144,19 @@ struct LeafCrit {
 };
 
 // The same criterion with the leaf's FP64 box loaded at each call: for the one-pass
-// traversal, which decides almost every node in FP32 and calls this only inside the
-// rounding band, keeping twelve doubles out of its registers.
+// traversals, which decide almost every node in FP32 and come here only inside the
+// rounding band; a call keeps its two dozen doubles out of their registers.
+static __device__ __noinline__ bool leaf_crit_call(const NodeBox *boxes, u32 leaf_node, u32 node) {
+    TreeView t{};
+    t.boxes = boxes;
+    return LeafCrit(t, leaf_node, 0)(node);
+}
 struct LazyLeafCrit {
     const TreeView &t;
     u32 leaf_node;
     __device__ LazyLeafCrit(const TreeView &tv, u32 leaf) : t(tv), leaf_node(tv.off() + leaf) {}
     __device__ bool operator()(u32 node) const {
-        const LeafCrit eager(t, leaf_node - t.off());
-        return eager(node);
+        return leaf_crit_call(t.boxes, leaf_node, node);
     }
 };
 
@@ -183,14 +188,20 @@ __global__ void k_leaf_fill(TreeView t, const u32 *__restrict__ off, uint2 *__re
 // separation s = max(n.lo - a.hi, a.lo - n.hi).  The FP32 estimate of s carries at most
 // ~2e-7 of the largest coordinate M plus 1e-7 relative; outside a band of
 // 1e-6 (M + R) the FP32 answer is certain, inside it the FP64 criterion decides.
-// Stage 1 over the child-pair records.  A popped internal node loads both children's
-// boxes in one record and tests them together, pushing those that pass (right, then
-// left, so the left subtree is walked first); a popped leaf has passed and is
-// reported.  Every node is tested once, when its parent is expanded, so the leaves and
-// their order are those of dfs() with the same criterion; per step the traversal waits
-// on one record load instead of a box load and a child-index load per node.
-// leaf_thr (optional, see k_owner): a leaf owning no row gets an empty list, and a
-// candidate leaf that no owned row can pair with is dropped (the cache is unchanged).
+// Stage 1 over the child-pair records.  An internal node loads both children's boxes in one
+// record and tests them together; the walk goes on in the left child that passes, and the
+// right one waits on the stack if both do.  Every node is tested once, when its parent is
+// expanded, so the leaves and their order are those of dfs() with the same criterion; per
+// step the traversal waits on one record load instead of a box load and a child-index load
+// per node.  leaf_thr (see k_owner): a leaf owning no row gets an empty list, and a node
+// below which no owned row can find a pair is dropped (the cache is unchanged).
+// Local memory is what this kernel must not touch: each lane's stack stands at its own
+// height, so an access is up to 32 lines.  The first twelve places are in shared memory, a
+// bank per lane, the FP64 criterion is a call, and the registers are not bounded (72; with
+// 64, 40 bytes of spills make it three times slower).  1,048,576 / 8.5 M particles 580 us /
+// 3.92 ms with the stack in local memory and every passing child pushed, 538 / 3.56 with
+// inner nodes dropped too, 472 / 3.19 now; disc 940 -> 802 us.
+constexpr int kNear = 12;
 __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *__restrict__ fb,
                                                     const NodePairF *__restrict__ rec,
                                                     u32 *__restrict__ cnt, u32 *__restrict__ off,
@@ -243,28 +254,37 @@ __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *
         float tb = fmaxf(thr_own, nlo.w * nlo.w * 1.000001f);
         return !(d2 > tb * 1.00001f);
     };
-    u32 stack[kStack];
+    __shared__ u32 s_near[kNear][128]; // the first places of the lanes' stacks, a bank each
+    u32 far[kStack - kNear];
     int top = 0;
     bool ok = true;
     RangeWriter w(ent, t.reduc, base, cap);
-    if (test(0, rlo, rhi) && (offn > 0 || keep(rlo, rhi))) stack[top++] = 0;
-    while (top > 0) {
-        const u32 n = stack[--top];
+    u32 n = test(0, rlo, rhi) && keep(rlo, rhi) ? 0u : kNone;
+    while (n != kNone) {
+        u32 next = kNone;
         if (n >= offn) {
             w.add(n - offn, n - offn + 1);
-            continue;
+        } else {
+            const F8 bl = ldg256(&rec[n].l), br = ldg256(&rec[n].r);
+            const u32 li = __float_as_uint(bl.b.w), ri = __float_as_uint(br.b.w);
+            const bool pl = test(li, bl.a, bl.b) && keep(bl.a, bl.b);
+            const bool pr = test(ri, br.a, br.b) && keep(br.a, br.b);
+            if (top + 2 > kStack) {
+                ok = false;
+                break;
+            }
+            if (pl && pr) {
+                if (top < kNear) s_near[top][threadIdx.x] = ri;
+                else far[top - kNear] = ri;
+                top++;
+            }
+            next = pl ? li : (pr ? ri : kNone);
         }
-        const F8 bl = ldg256(&rec[n].l), br = ldg256(&rec[n].r);
-        const u32 li = __float_as_uint(bl.b.w), ri = __float_as_uint(br.b.w);
-        bool pl = test(li, bl.a, bl.b), pr = test(ri, br.a, br.b);
-        if (pl && li >= offn) pl = keep(bl.a, bl.b);
-        if (pr && ri >= offn) pr = keep(br.a, br.b);
-        if (top + 2 > kStack) {
-            ok = false;
-            break;
+        if (next == kNone && top > 0) {
+            top--;
+            next = top < kNear ? s_near[top][threadIdx.x] : far[top - kNear];
         }
-        if (pr) stack[top++] = ri;
-        if (pl) stack[top++] = li;
+        n = next;
     }
     w.flush();
     const u32 c = w.c;
@@ -851,11 +871,14 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // decide inside the rounding band), made with the boxes
     const NodeBoxF *fb = c.fboxes.as<NodeBoxF>();
     const NodePairF *rec = c.fpairs.as<NodePairF>();
-    // Stage 1 on the 8-ary hierarchy (built here, three levels per launch) while a thread per
-    // leaf would leave an SM fewer than 512 threads: the binary walk is a chain of dependent
-    // loads, 113 us for 1,399 leaves and 219 us for 35,981 against 36 and 139 us; from about
-    // 100,000 leaves on its throughput wins (245,000 leaves: 0.58 against 0.80 ms).
-    const bool wide = L <= 512 * c.sms;
+    // Stage 1 on the 8-ary hierarchy (built here, three levels per launch) while the leaves
+    // that own rows (their share is about the rows' share of the particles) would leave an SM
+    // fewer than 320 threads of the binary walk, a chain of dependent loads: 119 us for 1,399
+    // leaves and 178 us for 35,981, 26,000 of them owners, against 34 and 135 us; 84,255
+    // leaves with 29,000 owners 368 against 212, 50,404 owners of a disc 338 against 280.
+    // From about 50,000 owners on its throughput wins (60,000 in a Sedov state 210 against
+    // 255 us, 75,000 in a disc 379 against 393).
+    const bool wide = (u64) L * n <= 320ull * c.sms * c.n_obj;
     WideTree wt{};
     wt.level[0] = fb + (L - 1);
     wt.n[0]     = L;

@@ -48,3 +48,49 @@ def test_step_sort_is_the_networks(shape, ties):
     n = len(model.collect_data()["hpart"])
     assert torch.equal(perm[:n], want[:n])
     assert (len(torch.unique(keys[:n])) < n) == (ties > 0)
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 513, 40000, 60000])
+def test_cache_routes_vs_oracle(gctx, n):
+    """Stage 1 on the wide hierarchy (up to 320 owning leaves an SM) and on the binary tree, one
+    leaf per particle, with a clump of small h far from the origin (rows decided in FP64)
+    and rows longer than the 64 candidates that stage 2 tests at a time."""
+    from oracle import oracle as O
+    from shamrock_gb300 import modules as M
+
+    rng = np.random.default_rng(n)
+    pos = 5.0 + rng.random((n, 3))
+    h = rng.uniform(0.5, 1.1, n) * (30.0 / max(n, 30)) ** (1 / 3) * 0.5
+    k = n // 10
+    pos[:k] = 5.5 + 1e-4 * rng.standard_normal((k, 3))
+    h[:k] = 3e-5
+    lo, hi = np.nextafter(pos.min(0), -np.inf), np.nextafter(pos.max(0), np.inf)
+    M.Tree(gctx, pos, lo, hi, 0, h=h, htol=1.1)
+    csr = M.neighbour_cache(gctx, n, 1.1, "mixed")
+    o = O.Tree(pos, lo, hi, 0, h=h, htol=1.1)
+    oc = o.neigh_cache(pos, h, n, 1.1)
+    for key in ("cnt", "scanned", "entries"):
+        assert np.array_equal(csr[key].cpu().numpy().view(np.uint32), oc[key]), key
+
+
+def _sms():
+    import torch
+
+    return torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 152
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (5, 7, 3), (32, 32, _sms() // 4), (32, 32, _sms() // 4 + 1)])
+def test_row_routes_mixed_vs_fp64(shape):
+    """Mixed step with four lanes per row (up to 256 rows an SM) and a thread per row in the
+    density passes, four lanes in the derivatives, free boundary (rows of every length):
+    within the tier's 1e-5 of the FP64 step from the same state."""
+    s = _lattice_state(*shape, 0, seed=3)
+    out = []
+    for precision in ("mixed", "fp64"):
+        model, _ = make_pair(s, precision=precision, periodic=False)
+        model.set_next_dt(0.0)
+        model.evolve_once()
+        out.append(model.collect_data())
+    for key in ("hpart", "omega", "axyz", "duint"):
+        a, b = out[0][key], out[1][key]
+        assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-300), key
