@@ -167,7 +167,7 @@ __device__ __forceinline__ void density_sums(const RowSpace &rs, u32 a, u32 k0, 
 // particle: a particle's update reads only its own h, so it iterates until its own
 // eps <= eps_p (1e-6 in the reference), becomes -1, or the iteration cap is reached).
 // The rows of a warp iterate together until the last of them is done.
-__global__ void __launch_bounds__(128, 8) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
+__global__ void __launch_bounds__(128, 7) k_h_iterate(RowSpace rs, const f64 *__restrict__ h_old,
                                                    f64 *__restrict__ h_new, f64 *__restrict__ eps,
                                                    f64 pmass, f64 h_evol_max, f64 h_evol_iter_max,
                                                    u32 iters, f64 eps_p, Scalars *sc) {
