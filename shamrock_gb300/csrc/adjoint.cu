@@ -80,6 +80,16 @@ struct AdjLocal {
     f64 *gal, *gain, *gcsin;
 };
 
+// Four entries of a row by one load (rows of the library's cache start on 16-byte boundaries
+// and their slots are padded to four), for the density passes, which load little else: a
+// thread per row reads entries from a line of its own, so four single loads cost four times
+// the L1 wavefronts, and they ran at 80 % of the L1's rate.  With the four records requested
+// together k_adj_omega_a / _b of 262,144 particles 168 / 195 -> 109 / 121 us, disc of 300,007
+// 150 / 202 -> 96 / 118 us.  (k_adj_derivs, bound by its arithmetic, gains nothing.)
+__device__ __forceinline__ uint4 entries4(const u32 *__restrict__ ent, u32 k) {
+    return __ldg((const uint4 *) (ent + k));
+}
+
 // -------------------------------------------------------------- particle sources
 // A source gives, per rank, what the reverse pair loops read: the row's own values and,
 // for a neighbour, its differences to the row (positions, velocities, cotangents) and
@@ -112,18 +122,17 @@ struct Src64 {
         ay = r.y;
         az = r.z;
     }
-    __device__ void pos(u32 c, f64 &px, f64 &py, f64 &pz, f64 &ph) const {
-        px = x[c];
-        py = y[c];
-        pz = z[c];
-        ph = h[c];
+    struct Rec {
+        f64 x, y, z, h;
+    };
+    __device__ Rec rec(u32 b) const { return Rec{x[b], y[b], z[b], h[b]}; }
+    __device__ static f64 h_of(const Rec &r) { return r.h; }
+    __device__ static void dpos(const Rec &b, const Rec &c, f64 &dx, f64 &dy, f64 &dz) {
+        dx = c.x - b.x;
+        dy = c.y - b.y;
+        dz = c.z - b.z;
     }
-    __device__ void dpos(u32 b, f64 px, f64 py, f64 pz, f64 &dx, f64 &dy, f64 &dz, f64 &hb) const {
-        dx = px - x[b];
-        dy = py - y[b];
-        dz = pz - z[b];
-        hb = h[b];
-    }
+    __device__ f64 csq(u32) const { return 0; } // evaluated per pair
     __device__ void mult(u32 b, f64 &nub, f64 &lomb) const {
         nub  = nu[b];
         lomb = lom[b];
@@ -133,11 +142,14 @@ struct Src64 {
 // FP32 records (rank order), differences taken on hi/lo pairs:
 //   P[2r..2r+1] = {x_hi, y_hi, z_hi, h | x_lo, y_lo, z_lo, Omega}
 //   V[2r..2r+1] = {v_hi, u | v_lo, mu},   Lr[r] = {lambda, alpha},   M[r] = {nu, lom}
+//   C[r] = c_s^2 of the locally isothermal form: a power per particle instead of one per
+//   pair, k_adj_derivs of a disc of 300,007 466 -> 405 us
 // (alpha: the per-particle viscosity of the varying forms, 0 for the constant one)
 struct Src32 {
     using T = float;
     const float4 *P, *V, *Lr;
     const float2 *M;
+    const float *C;
     struct Row {
         F8 p, v;
         float4 l;
@@ -162,17 +174,15 @@ struct Src32 {
         ay = r.p.a.y + r.p.b.y;
         az = r.p.a.z + r.p.b.z;
     }
-    __device__ void pos(u32 c, F8 &pc, float &ph) const {
-        pc = ldg256(&P[2 * (size_t) c]);
-        ph = pc.a.w;
-    }
-    __device__ void dpos(u32 b, const F8 &pc, float &dx, float &dy, float &dz, float &hb) const {
-        const F8 p = ldg256(&P[2 * (size_t) b]);
+    using Rec = F8;
+    __device__ Rec rec(u32 b) const { return ldg256(&P[2 * (size_t) b]); }
+    __device__ static float h_of(const Rec &r) { return r.a.w; }
+    __device__ static void dpos(const Rec &p, const Rec &pc, float &dx, float &dy, float &dz) {
         dx = (pc.a.x - p.a.x) + (pc.b.x - p.b.x);
         dy = (pc.a.y - p.a.y) + (pc.b.y - p.b.y);
         dz = (pc.a.z - p.a.z) + (pc.b.z - p.b.z);
-        hb = p.a.w;
     }
+    __device__ float csq(u32 b) const { return __ldg(&C[b]); }
     __device__ void mult(u32 b, float &nub, float &lomb) const {
         const float2 v = __ldg(&M[b]);
         nub  = v.x;
@@ -231,8 +241,8 @@ __global__ void k_adj_stage32(u32 N, u32 n, const u32 *__restrict__ sort_index,
                               const f64 *__restrict__ h, const f64 *__restrict__ om,
                               const f64 *__restrict__ lx, const f64 *__restrict__ ly,
                               const f64 *__restrict__ lz, const f64 *__restrict__ mu,
-                              const f64 *__restrict__ al, float4 *__restrict__ P,
-                              float4 *__restrict__ V, float4 *__restrict__ Lr) {
+                              const f64 *__restrict__ al, AdjParams p, float4 *__restrict__ P,
+                              float4 *__restrict__ V, float4 *__restrict__ Lr, float *__restrict__ C) {
     u32 r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= N) return;
     u32 id  = sort_index[r];
@@ -245,6 +255,12 @@ __global__ void k_adj_stage32(u32 N, u32 n, const u32 *__restrict__ sort_index,
     V[r2]     = make_float4(hi32(a), hi32(b), hi32(c), hi32(u[src]));
     V[r2 + 1] = make_float4(lo32(a), lo32(b), lo32(c), hi32(mu[src]));
     Lr[r]     = make_float4(hi32(lx[src]), hi32(ly[src]), hi32(lz[src]), al ? hi32(al[src]) : 0.f);
+    if (p.eos_kind == 1) {
+        const float cs0sq = (float) (p.cs0 * p.cs0), ir0sq = (float) (1 / (p.r0 * p.r0)), mq = (float) -p.q;
+        const float xb = P[r2].x + P[r2 + 1].x, yb = P[r2].y + P[r2 + 1].y, zb = P[r2].z + P[r2 + 1].z;
+        const float rsq = xb * xb + yb * yb + zb * zb;
+        C[r]            = cs0sq * pow(rsq * ir0sq, mq);
+    }
 }
 __global__ void k_adj_stage32m(u32 N, u32 n, const u32 *__restrict__ sort_index,
                                const u32 *__restrict__ ghost_src, const f64 *__restrict__ nu,
@@ -279,7 +295,8 @@ __global__ void __launch_bounds__(128) k_adj_derivs(RowSpace rs, Src src, AdjPar
         const T cs0sq = T(p.cs0 * p.cs0), ir0sq = T(1 / (p.r0 * p.r0)), mq = T(-p.q);
         const T rhoc = rho_of_h(m, hc);
         // adiabatic: P = (gamma - 1) rho u; LP07: c_s^2 = cs0^2 (R^2 / r0^2)^(-q), P = c_s^2 rho
-        const T csqc = lp07 ? cs0sq * pow(self.rsq * ir0sq, mq) : gam * gm1 * uc;
+        constexpr bool staged = std::is_same<T, float>::value;
+        const T csqc = lp07 ? (staged ? src.csq(c) : cs0sq * pow(self.rsq * ir0sq, mq)) : gam * gm1 * uc;
         const T Pc   = lp07 ? csqc * rhoc : gm1 * rhoc * uc;
         const T csc  = sqrt(csqc);
         const T subc = rhoc * rhoc * omc;
@@ -300,7 +317,7 @@ __global__ void __launch_bounds__(128) k_adj_derivs(RowSpace rs, Src src, AdjPar
             const T ex = dx * ir, ey = dy * ir, ez = dz * ir;
             const T ub = nb.u, omb = nb.om;
             const T rhob = rho_of_h(m, hb);
-            const T csqb = lp07 ? cs0sq * pow(nb.rsq * ir0sq, mq) : gam * gm1 * ub;
+            const T csqb = lp07 ? (staged ? src.csq(b) : cs0sq * pow(nb.rsq * ir0sq, mq)) : gam * gm1 * ub;
             const T Pb   = lp07 ? csqb * rhob : gm1 * rhob * ub;
             const T csb  = psqrt(csqb);
             const T subb = rhob * rhob * omb;
@@ -428,23 +445,28 @@ __global__ void __launch_bounds__(256) k_adj_omega_a(RowSpace rs, Src src, const
     if (t >= rs.n) return;
     const u32 c = rs.row_rank[t], i = rs.row_local[t];
     const T sig = T(kNorm3d);
-    typename std::conditional<std::is_same<T, f64>::value, f64, F8>::type pc;
-    T px = 0, py = 0, pz = 0, hc;
-    if constexpr (std::is_same<T, f64>::value) src.pos(c, px, py, pz, hc);
-    else src.pos(c, pc, hc);
+    const auto pc = src.rec(c);
+    const T hc    = src.h_of(pc);
     const T ihc = T(1) / hc, ih4 = ihc * ihc * ihc * ihc;
     T S = 0, Sh = 0; // sum dW/dh, sum d2W/dh2 (self pair included)
     const u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
-    for (u32 k = k0; k < k1; k++) {
-        const u32 b = rs.ent[k];
-        T dx, dy, dz, hb;
-        if constexpr (std::is_same<T, f64>::value) src.dpos(b, px, py, pz, dx, dy, dz, hb);
-        else src.dpos(b, pc, dx, dy, dz, hb);
-        const T q = psqrt(dx * dx + dy * dy + dz * dz) * ihc;
-        if (q >= T(2)) continue;
-        const T f0 = m4_f(q), f1 = m4_d1(q), f2 = m4_d2(q);
-        S += -sig * (T(3) * f0 + q * f1) * ih4;
-        Sh += sig * (T(12) * f0 + T(8) * q * f1 + q * q * f2) * ih4 * ihc;
+    uint4 nx = k0 < k1 ? entries4(rs.ent, k0) : make_uint4(c, c, c, c);
+    for (u32 k = k0; k < k1; k += 4) {
+        const u32 bb[4] = {nx.x, k + 1 < k1 ? nx.y : c, k + 2 < k1 ? nx.z : c, k + 3 < k1 ? nx.w : c};
+        typename Src::Rec pb[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) pb[j] = src.rec(bb[j]);
+        if (k + 4 < k1) nx = entries4(rs.ent, k + 4);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            T dx, dy, dz;
+            src.dpos(pb[j], pc, dx, dy, dz);
+            const T q = psqrt(dx * dx + dy * dy + dz * dz) * ihc;
+            if (k + j >= k1 || q >= T(2)) continue;
+            const T f0 = m4_f(q), f1 = m4_d1(q), f2 = m4_d2(q);
+            S += -sig * (T(3) * f0 + q * f1) * ih4;
+            Sh += sig * (T(12) * f0 + T(8) * q * f1 + q * q * f2) * ih4 * ihc;
+        }
     }
     // scalar tail in FP64 from the local h and Omega
     const f64 h64 = h_local[i], om64 = om_local[i];
@@ -465,36 +487,44 @@ __global__ void __launch_bounds__(256) k_adj_omega_b(RowSpace rs, Src src, f64 p
     if (t >= rs.n) return;
     const u32 c = rs.row_rank[t], i = rs.row_local[t];
     const T sig = T(kNorm3d);
-    typename std::conditional<std::is_same<T, f64>::value, f64, F8>::type pc;
-    T px = 0, py = 0, pz = 0, hc;
-    if constexpr (std::is_same<T, f64>::value) src.pos(c, px, py, pz, hc);
-    else src.pos(c, pc, hc);
+    const auto pc = src.rec(c);
+    const T hc    = src.h_of(pc);
     T nuc, lomc;
     src.mult(c, nuc, lomc);
     const T ihc = T(1) / hc, ihc5 = ihc * ihc * ihc * ihc * ihc;
     T gx = 0, gy = 0, gz = 0;
     const u32 k0 = rs.off[t], k1 = k0 + rs.cnt[t];
-    for (u32 k = k0; k < k1; k++) {
-        const u32 b = rs.ent[k];
-        T dx, dy, dz, hb;
-        if constexpr (std::is_same<T, f64>::value) src.dpos(b, px, py, pz, dx, dy, dz, hb);
-        else src.dpos(b, pc, dx, dy, dz, hb);
-        const T r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 == T(0)) continue;
-        const T r = psqrt(r2), ir = pdiv(T(1), r);
-        const T ihb = pdiv(T(1), hb);
-        const T qc = r * ihc, qb = r * ihb;
-        if (qc >= T(2) && qb >= T(2)) continue;
-        T nub, lomb;
-        src.mult(b, nub, lomb);
-        const T d1c = m4_d1(qc), d2c = m4_d2(qc), d1b = m4_d1(qb), d2b = m4_d2(qb);
-        const T ihb5 = ihb * ihb * ihb * ihb * ihb;
-        const T Grc = -sig * (T(4) * d1c + qc * d2c) * ihc5, Grb = -sig * (T(4) * d1b + qb * d2b) * ihb5;
-        const T Fc = sig * d1c * ihc5 * hc, Fb = sig * d1b * ihb5 * hb;
-        const T s = T(pmass) * (lomc * Grc + lomb * Grb + nuc * Fc + nub * Fb) * ir;
-        gx += s * dx;
-        gy += s * dy;
-        gz += s * dz;
+    uint4 nx = k0 < k1 ? entries4(rs.ent, k0) : make_uint4(c, c, c, c);
+    for (u32 k = k0; k < k1; k += 4) {
+        const u32 bb[4] = {nx.x, k + 1 < k1 ? nx.y : c, k + 2 < k1 ? nx.z : c, k + 3 < k1 ? nx.w : c};
+        typename Src::Rec pb[4];
+        T nub[4], lomb[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            pb[j] = src.rec(bb[j]);
+            src.mult(bb[j], nub[j], lomb[j]);
+        }
+        if (k + 4 < k1) nx = entries4(rs.ent, k + 4);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            T dx, dy, dz;
+            src.dpos(pb[j], pc, dx, dy, dz);
+            const T hb = src.h_of(pb[j]);
+            const T r2 = dx * dx + dy * dy + dz * dz;
+            if (k + j >= k1 || r2 == T(0)) continue;
+            const T r = psqrt(r2), ir = pdiv(T(1), r);
+            const T ihb = pdiv(T(1), hb);
+            const T qc = r * ihc, qb = r * ihb;
+            if (qc >= T(2) && qb >= T(2)) continue;
+            const T d1c = m4_d1(qc), d2c = m4_d2(qc), d1b = m4_d1(qb), d2b = m4_d2(qb);
+            const T ihb5 = ihb * ihb * ihb * ihb * ihb;
+            const T Grc = -sig * (T(4) * d1c + qc * d2c) * ihc5, Grb = -sig * (T(4) * d1b + qb * d2b) * ihb5;
+            const T Fc = sig * d1c * ihc5 * hc, Fb = sig * d1b * ihb5 * hb;
+            const T s = T(pmass) * (lomc * Grc + lomb[j] * Grb + nuc * Fc + nub[j] * Fb) * ir;
+            gx += s * dx;
+            gy += s * dy;
+            gz += s * dz;
+        }
     }
     L.gx[0][i] += gx;
     L.gx[1][i] += gy;
@@ -1132,7 +1162,7 @@ cudaError_t adjoint_backward(Ctx &c, const RowSpace &rs, u32 n, const f64 *h_loc
     L.gal   = B + 21 * n_;
     L.gain  = B + 22 * n_;
     L.gcsin = B + 23 * n_;
-    // rank-order staging: FP64 arrays (12 per rank) or FP32 records (88 bytes per rank)
+    // rank-order staging: FP64 arrays (12 per rank) or FP32 records (92 bytes per rank)
     f64 *R = c.adj_rank.as<f64>();
     // varying viscosity: the previous accelerations and alpha by rank, the cotangents of the
     // velocity-gradient sums by local id (32 each) and by rank
@@ -1161,7 +1191,8 @@ cudaError_t adjoint_backward(Ctx &c, const RowSpace &rs, u32 n, const f64 *h_loc
     float4 *V32 = P32 + 2 * N_;
     float4 *L32 = V32 + 2 * N_;
     float2 *M32 = (float2 *) (L32 + N_);
-    Src32 s32{P32, V32, L32, M32};
+    float *C32  = (float *) (M32 + N_);
+    Src32 s32{P32, V32, L32, M32, C32};
     const u32 *si = c.sort_index.as<u32>(), *gs = c.ghost_src.as<u32>();
     const u32 vs = cot.vs;
     const u32 gb = div_up(n, 256), gN = div_up(N, 256);
@@ -1184,7 +1215,7 @@ cudaError_t adjoint_backward(Ctx &c, const RowSpace &rs, u32 n, const f64 *h_loc
             { k_adj_stage32<<<gN, 256, 0, s>>>(N, n, si, gs, rs.x, rs.y, rs.z, sv, sv + n_,
                                              sv + 2 * n_, sv + 3 * n_, h_local, omega_local,
                                              L.lam[0], L.lam[1], L.lam[2], L.mu,
-                                             var ? sa + 3 * n_ : nullptr, P32, V32, L32); GBSPH_COUNTED; }
+                                             var ? sa + 3 * n_ : nullptr, p, P32, V32, L32, C32); GBSPH_COUNTED; }
             if (p.eos_kind == 1)
                 { k_adj_derivs<Src32, true><<<div_up(n, 128), 128, 0, s>>>(rs, s32, p, L, g_alpha); GBSPH_COUNTED; }
             else
