@@ -34,6 +34,12 @@ FIELDS_AV_VEC = ("curlv",)
 G_SI = 6.6743015e-11
 
 
+def _vec3(t):
+    """A (3, N) tensor's components (pointer arithmetic: indexing makes a tensor per component)."""
+    p, step = t.data_ptr(), t.stride(0) * t.element_size()
+    return L.Vec3(p, p + step, p + 2 * step, 1, 0)
+
+
 class UnitSystem:
     """shamrock.UnitSystem (shamunits/UnitSystem.hpp:148-160, pyUnits.cpp:30-55): the SI
     value of one code unit of time, length and mass."""
@@ -407,9 +413,7 @@ class Model:
         p = L.Particles()
         p.n = n
         for k in FIELDS_VEC:
-            t = d[k]
-            v = L.Vec3(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), 1, 0)
-            setattr(p, k, v)
+            setattr(p, k, _vec3(d[k]))
         p.hpart = d["hpart"].data_ptr()
         p.uint = d["uint"].data_ptr()
         p.duint = d["duint"].data_ptr()
@@ -419,8 +423,7 @@ class Model:
             p.soundspeed = d["soundspeed"].data_ptr()
             p.divv = d["divv"].data_ptr()
             p.dtdivv = d["dtdivv"].data_ptr()
-            t = d["curlv"]
-            p.curlv = L.Vec3(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), 1, 0)
+            p.curlv = _vec3(d["curlv"])
         return p
 
     def _config_struct(self, tier=None):
