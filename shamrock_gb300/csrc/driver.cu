@@ -78,6 +78,7 @@ Ctx::~Ctx() {
     cudaSetDevice(device);
     for (DevBuf *b : bufs) b->release(stream);
     cudaStreamSynchronize(stream);
+    if (posted) cudaEventDestroy(posted);
     if (h_scalars) cudaFreeHost(h_scalars);
 }
 
@@ -270,6 +271,7 @@ int gbsph_create(gbsph_ctx **out, int device) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
         ctx->c.sms = (u32) sms;
     if (cudaMallocHost(&ctx->c.h_scalars, sizeof(Scalars)) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->c.posted, cudaEventDisableTiming) != cudaSuccess ||
         ctx->c.d_scalars.ensure(sizeof(Scalars), 0) != cudaSuccess ||
         ctx->c.d_bbox.ensure(sizeof(BBox), 0) != cudaSuccess) {
         delete ctx;
@@ -693,6 +695,16 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
     f64 max_eps = 0, min_eps = 0;
     bool converged = false;
     RowSpace rs{};
+    // What follows an h iteration whether or not its sub-cycle converged: the iterated h is
+    // written back, and Omega taken at it (a sub-cycle that follows builds its own cache, and
+    // its Omega replaces this one).  The compensated tier finishes h first, so only then.
+    auto after_h = [&]() -> cudaError_t {
+        cudaError_t e = scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h);
+        if (e != cudaSuccess || comp) return e;
+        if (mixed)
+            return omega_compact_mixed(c, rs, n + c.n_ghost, n, lf.h, c.hnew_row.as<f64>(), c.omega_local.as<f64>());
+        return omega64(c, rs, c.hnew_row.as<f64>(), cfg->pmass, c.omega_local.as<f64>(), c.row_local.as<u32>());
+    };
     for (; hstep < cfg->h_max_subcycles; hstep++) {
         if (cfg->periodic) {
             CU(periodic_ghosts(c, lf.x, lf.y, lf.z, lf.vs, lf.h, n, cfg->box_min, cfg->box_max,
@@ -702,12 +714,14 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         }
         CU(merge_positions(c, lf.x, lf.y, lf.z, lf.vs, lf.h, n, true));
         u32 N = n + c.n_ghost;
+        // The rows and the FP32 positions need only the sorted order.  Both precisions pre-test
+        // the pairs in FP32 (exact FP64 test inside the rounding band): the cache is the FP64
+        // one either way
         CU(tree_build(c, c.mx.as<f64>(), c.my.as<f64>(), c.mz.as<f64>(), c.mh.as<f64>(), N,
-                      cfg->tree_reduction_level, cfg->htol_up_coarse, 32, 0, true));
-        CU(build_rows(c, n));
-        // both precisions pre-test the pairs in FP32 (exact FP64 test inside the rounding
-        // band): the cache is the FP64 one either way
-        CU(stage_positions_mixed(c, N, cfg->htol_up_coarse));
+                      cfg->tree_reduction_level, cfg->htol_up_coarse, 32, 0, true, [&]() {
+                          const cudaError_t e = build_rows(c, n);
+                          return e != cudaSuccess ? e : stage_positions_mixed(c, N, cfg->htol_up_coarse);
+                      }));
         CU(neigh_cache_build(c, cfg->htol_up_coarse, mixed_positions(c)));
         rs = RowSpace{n,                  c.row_rank.as<u32>(), c.row_local.as<u32>(),
                       c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>(),
@@ -723,7 +737,9 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                 CU(h_iterate64(c, rs, c.h_old_row.as<f64>(), c.hnew_row.as<f64>(),
                                c.eps_row.as<f64>(), cfg->pmass, cfg->htol_up_coarse,
                                cfg->htol_up_fine, cfg->h_iter_per_subcycles, eps_p));
-            CU(sync_scalars(c));
+            CU(post_scalars(c));
+            CU(after_h());
+            CU(wait_scalars(c));
             max_eps     = ordered_to_f64(c.h_scalars->eps_max);
             min_eps     = ordered_to_f64(c.h_scalars->eps_min);
             iters_total = c.h_scalars->iters_max;
@@ -744,10 +760,9 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                 iters_total++;
                 if (max_eps < cfg->epsilon_h) break;
             }
+            CU(after_h());
         }
         lg.h_iterations += iters_total;
-        // the iterated h is written back whether or not the sub-cycle converged
-        CU(scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h));
         converged = (max_eps < cfg->epsilon_h) && !(min_eps < 0);
         if (converged) break;
     }
@@ -764,11 +779,8 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         CU(dens_polish_df(c, rs, c.h_old_row.as<f64>(), c.hnew_row.as<f64>(), c.eps_row.as<f64>(),
                           cfg->htol_up_coarse, cfg->htol_up_fine, c.omega_local.as<f64>()));
         CU(scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h));
-    } else if (mixed) {
-        CU(omega_compact_mixed(c, rs, N, n, lf.h, c.hnew_row.as<f64>(), c.omega_local.as<f64>()));
-    } else {
-        CU(omega64(c, rs, c.hnew_row.as<f64>(), cfg->pmass, c.omega_local.as<f64>(),
-                   c.row_local.as<u32>()));
+    } else if (hstep == 0 && cfg->h_max_subcycles == 0) {
+        CU(after_h());
     }
     if (p->omega)
         CU(cudaMemcpyAsync(p->omega, c.omega_local.p, 8 * (size_t) n, cudaMemcpyDeviceToDevice, s));

@@ -6,6 +6,7 @@
 #include "gbsph_internal.cuh"
 
 #include <string>
+#include <functional>
 #include <vector>
 
 namespace gbsph {
@@ -120,6 +121,7 @@ struct Ctx {
 
     DevBuf scan_scratch;
     DevBuf d_scalars; // Scalars
+    cudaEvent_t posted = nullptr; // end of the last copy of the scalars (post_scalars)
     Scalars *h_scalars = nullptr; // pinned mirror
     DevBuf d_bbox;    // BBox
 
@@ -224,10 +226,18 @@ struct ProfScope {
 // fast_sort: sort the n real keys with the radix sort (the permutation equals the bitonic
 // network's whenever the keys are distinct, which it checks; the padding's order is not
 // kept, so only builds whose sorted padding is never exported may ask for it)
+// between: enqueues what needs only the sorted order and the rank-order copies, while the
+// host waits for the leaf count
 cudaError_t tree_build(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
-                       u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort = false);
+                       u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort = false,
+                       const std::function<cudaError_t()> &between = nullptr);
 cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax, int key_bits);
 cudaError_t sync_scalars(Ctx &c);            // copy Scalars to pinned host, wait
+// The same in two parts: work enqueued between them keeps the GPU busy while the host wakes
+// up and decides (about 12 us).  It must not depend on the decision, and stay in bounds and
+// be redone where the decision is to redo what came before.
+cudaError_t post_scalars(Ctx &c);
+cudaError_t wait_scalars(Ctx &c);
 
 // neigh.cu
 cudaError_t build_rows(Ctx &c, u32 n_local);

@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(128) k_leaf_lists_wide(TreeView t, const NodeB
 // what a cache build accumulates into: no owned row, no threshold, no flag, no entry
 __global__ void k_cache_init(u32 L, u32 *__restrict__ head, u32 *__restrict__ leaf_thr, Scalars *sc) {
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l == 0) sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = 0, sc->csr_entries = 0;
+    if (l == 0) sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = 0, sc->csr_entries = sc->csr_kept = 0;
     if (l >= L) return;
     head[l]     = kNone;
     leaf_thr[l] = 0;
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
     const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
     const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
     const f64 *__restrict__ sz, const f64 *__restrict__ sh, f64 h_tol, u32 *__restrict__ cnt,
-    u32 *__restrict__ off, u32 *__restrict__ ent, Scalars *sc, u32 cap) {
+    u32 *__restrict__ off, u32 *__restrict__ ent, Scalars *sc, u32 cap, u32 leaf_cap) {
     __shared__ float4 s_cand[8][kCandBlock];
     __shared__ u32 s_id[8][kCandBlock];
     const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
     u64 c_sum = 0;
     for (u32 l = blockIdx.x * 8 + wid; l < L; l += gridDim.x * 8) {
         u32 cur      = head[l];
-        const u32 k0 = leaf_off[l], nk = leaf_cnt[l];
+        const u32 k0 = leaf_off[l], nk = min(leaf_cnt[l], leaf_cap); // (an overflowing list is rebuilt)
         while (cur != kNone) {
             // the next 32 rows at most, a lane each
             u32 row = kNone, m = 0;
@@ -935,34 +935,6 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         if ((e = cudaMemcpyAsync(&dsc->flags, &ovf, sizeof(u32), cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
         if ((e = cudaMemcpyAsync(&dsc->leaf_cnt_max, &c.leaf_cap, sizeof(u32), cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
     }
-    if ((e = sync_scalars(c)) != cudaSuccess) return e;
-    if (c.h_scalars->flags & (kFlagStackOverflow | kFlagOwnerMissing)) {
-        c.err = "neighbour cache: tree traversal failed (stack overflow or particle outside every leaf box)";
-        return cudaErrorUnknown;
-    }
-    c.leaf_csr_total = 0;
-    if (c.h_scalars->flags & kFlagLeafCap) {
-        const u32 cap = (c.h_scalars->leaf_cnt_max + 31u) & ~31u;
-        const bool fits = s1_one_pass && slots_ok(L, cap, sizeof(uint2));
-        if ((e = cudaMemsetAsync(&dsc->flags, 0, sizeof(u32), s)) != cudaSuccess) return e;
-        if (fits) {
-            // one pass again with slots that hold the largest list
-            c.leaf_cap = cap;
-            if ((e = stage1()) != cudaSuccess) return e;
-        } else {
-            // exact two-pass build
-            ProfScope ps(c, kProfStage1, 0);
-            { k_leaf_count<<<div_up(L, 128), 128, 0, s>>>(t, c.leaf_cnt.as<u32>(), &dsc->flags); GBSPH_COUNTED; }
-            if ((e = scan_exclusive_u32(c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), L, &dsc->total,
-                                        c.scan_scratch, s)) != cudaSuccess)
-                return e;
-            if ((e = sync_scalars(c)) != cudaSuccess) return e;
-            c.leaf_csr_total = c.h_scalars->total;
-            if ((e = c.leaf_ent.ensure(sizeof(uint2) * (c.leaf_csr_total + 1), s)) != cudaSuccess) return e;
-            { k_leaf_fill<<<div_up(L, 128), 128, 0, s>>>(t, c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>()); GBSPH_COUNTED; }
-        }
-    }
-
     if ((e = c.csr_cnt.ensure(sizeof(u32) * ((size_t) n + 1), s)) != cudaSuccess) return e;
     if ((e = c.csr_off.ensure(sizeof(u32) * ((size_t) n + 1), s)) != cudaSuccess) return e;
     // the padded one-pass layout needs row * cap to fit the u32 offsets
@@ -981,22 +953,60 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // blocks that an SM holds (41 KB of candidates each; with one such grid the leaves'
     // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics
     // on the totals, 10 ns each, take longer than the build)
+    u32 leaf_slots = c.leaf_cap; // no bound for the lists of the exact stage 1
     auto part = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
         const u32 blocks   = std::min(div_up(L, 8), 24 * c.sms);
         { k_part_cache<MODE><<<blocks, 256, 0, s>>>(
             L, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
-            c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap); GBSPH_COUNTED; }
+            c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
     };
     using OnePass = std::integral_constant<int, kOnePass>;
     using Count   = std::integral_constant<int, kCount>;
     using Fill    = std::integral_constant<int, kFill>;
-    if (n && one_pass) {
+    auto stage2 = [&]() -> cudaError_t {
+        if (!n || !one_pass) return cudaSuccess;
         ProfScope ps(c, kProfCacheFill, n);
         part(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
-    }
+        return cudaGetLastError();
+    };
+    // Stage 2 follows at once: a list that overflowed its slots is read up to its slots only,
+    // and both stages run again.
+    if (s1_one_pass && (e = stage2()) != cudaSuccess) return e;
     if ((e = sync_scalars(c)) != cudaSuccess) return e;
+    if (c.h_scalars->flags & (kFlagStackOverflow | kFlagOwnerMissing)) {
+        c.err = "neighbour cache: tree traversal failed (stack overflow or particle outside every leaf box)";
+        return cudaErrorUnknown;
+    }
+    c.leaf_csr_total = 0;
+    if (c.h_scalars->flags & kFlagLeafCap) {
+        const u32 cap = (c.h_scalars->leaf_cnt_max + 31u) & ~31u;
+        const bool fits = s1_one_pass && slots_ok(L, cap, sizeof(uint2));
+        if ((e = cudaMemsetAsync(&dsc->flags, 0, sizeof(u32), s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(&dsc->row_cnt_max, 0, sizeof(u32), s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(&dsc->csr_entries, 0, sizeof(u64), s)) != cudaSuccess) return e;
+        if (fits) {
+            // one pass again with slots that hold the largest list
+            c.leaf_cap = leaf_slots = cap;
+            if ((e = stage1()) != cudaSuccess) return e;
+        } else {
+            // exact two-pass build
+            ProfScope ps(c, kProfStage1, 0);
+            { k_leaf_count<<<div_up(L, 128), 128, 0, s>>>(t, c.leaf_cnt.as<u32>(), &dsc->flags); GBSPH_COUNTED; }
+            if ((e = scan_exclusive_u32(c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), L, &dsc->total,
+                                        c.scan_scratch, s)) != cudaSuccess)
+                return e;
+            if ((e = sync_scalars(c)) != cudaSuccess) return e;
+            c.leaf_csr_total = c.h_scalars->total;
+            leaf_slots       = 0xffffffffu;
+            if ((e = c.leaf_ent.ensure(sizeof(uint2) * (c.leaf_csr_total + 1), s)) != cudaSuccess) return e;
+            { k_leaf_fill<<<div_up(L, 128), 128, 0, s>>>(t, c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>()); GBSPH_COUNTED; }
+        }
+        // stage 2 ran over cut lists, or not at all
+        if ((e = stage2()) != cudaSuccess) return e;
+        if ((e = sync_scalars(c)) != cudaSuccess) return e;
+    }
     c.csr_total = c.h_scalars->csr_entries;
     if (n && one_pass && (c.h_scalars->flags & kFlagCsrCap)) {
         // a row overflowed: one pass again with slots that hold the largest row

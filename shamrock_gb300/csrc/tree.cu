@@ -554,7 +554,8 @@ constexpr u32 kNetworkKeys = 1u << 20;
 
 template<class K>
 cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
-                            u32 level, f64 htol, u32 morton_count, bool fast_sort) {
+                            u32 level, f64 htol, u32 morton_count, bool fast_sort,
+                            const std::function<cudaError_t()> &between) {
     cudaStream_t s = c.stream;
     cudaError_t e;
     u32 P = morton_count;
@@ -589,6 +590,7 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     // For many keys the radix sort is tried first when allowed; equal keys (whose order is
     // the network's) send the build back to the bitonic sort, found at the sync below.
     const bool radix = fast_sort && std::is_same<K, u32>::value && P > kNetworkKeys;
+    bool posted = false;
     for (int attempt = radix ? 0 : 1; attempt < 2; attempt++) {
         {
             ProfScope ps(c, kProfSort, P);
@@ -612,9 +614,18 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
                          &dsc->total)) != cudaSuccess)
             return e;
         if (prof_tree >= 0) prof_end(c, prof_tree);
-        if ((e = sync_scalars(c)) != cudaSuccess) return e;
-        if (attempt == 0 && !c.h_scalars->dup_keys) break;
+        if (attempt == 0) {
+            if ((e = sync_scalars(c)) != cudaSuccess) return e;
+            if (!c.h_scalars->dup_keys) break;
+        } else {
+            if ((e = post_scalars(c)) != cudaSuccess) return e;
+            posted = true;
+        }
     }
+    { k_permute<<<div_up(n, T), T, 0, s>>>(vals, n, x, y, z, h, c.sx.as<f64>(), c.sy.as<f64>(),
+                                         c.sz.as<f64>(), c.sh.as<f64>(), c.rank_of.as<u32>()); GBSPH_COUNTED; }
+    if (between && (e = between()) != cudaSuccess) return e;
+    if (posted && (e = wait_scalars(c)) != cudaSuccess) return e;
     ProfScope ps_tree(c, kProfTree, 0);
     u32 L        = c.h_scalars->total;
     c.leaf_count = L;
@@ -634,8 +645,6 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     { k_karras<K><<<div_up(L, T), T, 0, s>>>(c.reduced.as<K>(), L, c.lchild.as<u32>(),
                                            c.rchild.as<u32>(), c.lflag.as<u8>(), c.rflag.as<u8>(),
                                            c.endrange.as<u32>(), c.parent.as<u32>(), c.visit.as<u32>()); GBSPH_COUNTED; }
-    { k_permute<<<div_up(n, T), T, 0, s>>>(vals, n, x, y, z, h, c.sx.as<f64>(), c.sy.as<f64>(),
-                                         c.sz.as<f64>(), c.sh.as<f64>(), c.rank_of.as<u32>()); GBSPH_COUNTED; }
     { k_leaf_boxes_up<<<div_up(L, T), T, 0, s>>>(
         c.reduc.as<u32>(), L, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
         h ? c.sh.as<f64>() : nullptr, htol, c.lchild.as<u32>(), c.rchild.as<u32>(),
@@ -653,6 +662,13 @@ cudaError_t sync_scalars(Ctx &c) {
     return cudaStreamSynchronize(c.stream);
 }
 
+cudaError_t post_scalars(Ctx &c) {
+    cudaError_t e = cudaMemcpyAsync(c.h_scalars, c.d_scalars.p, sizeof(Scalars),
+                                    cudaMemcpyDeviceToHost, c.stream);
+    return e != cudaSuccess ? e : cudaEventRecord(c.posted, c.stream);
+}
+cudaError_t wait_scalars(Ctx &c) { return cudaEventSynchronize(c.posted); }
+
 cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax, int key_bits) {
     const f64 cells = (f64) (key_bits == 64 ? Morton<u64>::val_count : Morton<u32>::val_count);
     BBox b{};
@@ -668,9 +684,10 @@ cudaError_t set_bbox_host(Ctx &c, const f64 *bmin, const f64 *bmax, int key_bits
 }
 
 cudaError_t tree_build(Ctx &c, const f64 *x, const f64 *y, const f64 *z, const f64 *h, u32 n,
-                       u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort) {
-    if (key_bits == 64) return tree_build_impl<u64>(c, x, y, z, h, n, level, htol, morton_count, false);
-    return tree_build_impl<u32>(c, x, y, z, h, n, level, htol, morton_count, fast_sort);
+                       u32 level, f64 htol, int key_bits, u32 morton_count, bool fast_sort,
+                       const std::function<cudaError_t()> &between) {
+    if (key_bits == 64) return tree_build_impl<u64>(c, x, y, z, h, n, level, htol, morton_count, false, between);
+    return tree_build_impl<u32>(c, x, y, z, h, n, level, htol, morton_count, fast_sort, between);
 }
 
 // explicit entry points for module-level exports (driver.cu)

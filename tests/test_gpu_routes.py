@@ -94,3 +94,23 @@ def test_row_routes_mixed_vs_fp64(shape):
     for key in ("hpart", "omega", "axyz", "duint"):
         a, b = out[0][key], out[1][key]
         assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-300), key
+
+
+def test_cache_overflowing_lists_vs_oracle():
+    """Stage-1 lists and rows longer than their slots in a new context: stage 2 has then run
+    over cut lists and both stages run again; the next build has the slots."""
+    from oracle import oracle as O
+    from shamrock_gb300 import _lib, modules as M
+
+    rng = np.random.default_rng(8)
+    n = 2000
+    pos = rng.random((n, 3))
+    h = np.where(rng.random(n) < 0.5, 0.6, 0.01)
+    lo, hi = np.nextafter(pos.min(0), -np.inf), np.nextafter(pos.max(0), np.inf)
+    oc = O.Tree(pos, lo, hi, 0, h=h, htol=1.1).neigh_cache(pos, h, n, 1.1)
+    ctx = _lib.Context(0)
+    for _ in range(2):
+        M.Tree(ctx, pos, lo, hi, 0, h=h, htol=1.1)
+        csr = M.neighbour_cache(ctx, n, 1.1, "mixed")
+        for key in ("cnt", "scanned", "entries"):
+            assert np.array_equal(csr[key].cpu().numpy().view(np.uint32), oc[key]), key
