@@ -67,7 +67,7 @@ Ctx::~Ctx() {
     for (cudaEvent_t e : prof.pool) cudaEventDestroy(e);
     DevBuf *bufs[] = {&scan_scratch, &d_scalars, &d_bbox, &keys, &sort_index, &flags_a, &flags_b,
                       &offsets, &reduc, &reduced, &radix_k, &radix_v, &radix_hist, &radix_off, &lchild, &rchild, &lflag, &rflag, &endrange,
-                      &parent, &boxes, &visit, &fboxes, &fpairs, &wboxes, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
+                      &parent, &boxes, &fboxes, &fpairs, &lboxes, &wboxes, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
                       &row_local, &leaf_cnt, &leaf_off, &leaf_ent,
                       &leaf_head, &next_row, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
                       &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &scs, &rec64,

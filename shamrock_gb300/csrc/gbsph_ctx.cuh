@@ -73,6 +73,27 @@ struct __align__(32) NodeBoxF {
     float4 hi;
 };
 
+// An 8-ary hierarchy over the leaves in Morton order: level 0 are the leaves, node i of level
+// m + 1 bounds the nodes 8 i .. 8 i + 7 of level m; the top level has eight nodes at most.
+constexpr int kWideLevels = 9; // 8^8 leaves, then the top nodes are walked in eights
+struct LevelPlan {
+    u32 n[kWideLevels];
+    u32 at[kWideLevels]; // first node of a level (m >= 1) in the arrays of all levels
+    u32 total;           // nodes of the levels 1 .. top
+    int top;
+};
+inline LevelPlan level_plan(u32 L) {
+    LevelPlan p{};
+    p.n[0] = L;
+    while (p.top + 1 < kWideLevels && p.n[p.top] > 8) {
+        p.n[p.top + 1]  = (p.n[p.top] + 7) / 8;
+        p.at[p.top + 1] = p.total;
+        p.total += p.n[p.top + 1];
+        p.top++;
+    }
+    return p;
+}
+
 // The two children of an internal node with their FP32 boxes (64 bytes, two 256-bit
 // loads), so a traversal tests both children of a node together; hi.w of each box
 // carries the child's node index (internal n, or leaf L - 1 + l) as raw bits.
@@ -130,7 +151,7 @@ struct Ctx {
     u32 n_obj = 0, morton_count = 0, leaf_count = 0;
     DevBuf keys, sort_index, flags_a, flags_b, offsets, reduc, reduced;
     DevBuf radix_k, radix_v, radix_hist, radix_off; // radix sort ping-pong and digit tables
-    DevBuf lchild, rchild, lflag, rflag, endrange, parent, boxes, visit, fboxes, fpairs, wboxes;
+    DevBuf lchild, rchild, lflag, rflag, endrange, parent, boxes, fboxes, fpairs, lboxes, wboxes;
     bool has_rint = false;
 
     // ---- rank-ordered copies of merged fields

@@ -297,68 +297,15 @@ __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *
     off[l] = base;
 }
 
-// ---- an 8-ary hierarchy over the leaves in Morton order for stage 1
-// Level 0 are the leaves' FP32 boxes, node i of level m + 1 bounds the nodes 8 i .. 8 i + 7 of
-// level m (boxes united, the largest interaction radius).  The criterion grows with the
-// boxes and radii (rounding is monotonic), so every leaf that passes lies below nodes that
-// pass, whatever the hierarchy; this one needs no pointers, its eight children are 256
-// consecutive bytes, and eight lanes test them together.
-constexpr int kWideLevels = 9; // 8^8 leaves, then the top nodes are walked in eights
+// ---- stage 1 on the 8-ary hierarchy over the leaves (LevelPlan), FP32 boxes
+// The criterion grows with the boxes and radii (rounding is monotonic), so every leaf that
+// passes lies below nodes that pass, whatever the hierarchy; this one needs no pointers, its
+// eight children are 256 consecutive bytes, and eight lanes test them together.
 struct WideTree {
     const NodeBoxF *level[kWideLevels];
     u32 n[kWideLevels];
     int top;
 };
-
-__device__ __forceinline__ float min8(float v) {
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ float max8(float v) {
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// three levels above n nodes: 512 of them to 64, 8 and 1 per block
-__global__ void __launch_bounds__(512) k_wide_levels(const NodeBoxF *__restrict__ in, u32 n,
-                                                     NodeBoxF *__restrict__ l1,
-                                                     NodeBoxF *__restrict__ l2,
-                                                     NodeBoxF *__restrict__ l3) {
-    __shared__ NodeBoxF s1[64], s2[32];
-    const float big = 3.0e38f;
-    NodeBoxF none;
-    none.lo = make_float4(big, big, big, 0.f);
-    none.hi = make_float4(-big, -big, -big, 0.f);
-    const u32 t = threadIdx.x, i = blockIdx.x * 512 + t;
-    auto unite = [](NodeBoxF v) {
-        v.lo = make_float4(min8(v.lo.x), min8(v.lo.y), min8(v.lo.z), max8(v.lo.w));
-        v.hi = make_float4(max8(v.hi.x), max8(v.hi.y), max8(v.hi.z), 0.f);
-        return v;
-    };
-    NodeBoxF v = unite(i < n ? in[i] : none);
-    const u32 n1 = (n + 7) / 8, n2 = (n1 + 7) / 8, n3 = (n2 + 7) / 8;
-    if ((t & 7) == 0) {
-        const u32 o = blockIdx.x * 64 + t / 8;
-        s1[t / 8]   = v;
-        if (o < n1) l1[o] = v;
-    }
-    __syncthreads();
-    if (t < 64) {
-        v = unite(s1[t]);
-        if ((t & 7) == 0) {
-            const u32 o = blockIdx.x * 8 + t / 8;
-            s2[t / 8]   = v;
-            if (l2 && o < n2) l2[o] = v;
-        }
-    }
-    __syncthreads();
-    if (t < 32) {
-        v = unite(t < 8 ? s2[t] : none);
-        if (t == 0 && l3 && blockIdx.x < n3) l3[blockIdx.x] = v;
-    }
-}
 
 // Stage 1 for few leaves: eight lanes walk the hierarchy for one leaf, testing a node's eight children per
 // step; the children that pass are a byte of a 64-bit mask per level, so the next node in
@@ -871,7 +818,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // decide inside the rounding band), made with the boxes
     const NodeBoxF *fb = c.fboxes.as<NodeBoxF>();
     const NodePairF *rec = c.fpairs.as<NodePairF>();
-    // Stage 1 on the 8-ary hierarchy (built here, three levels per launch) while the leaves
+    // Stage 1 on the 8-ary hierarchy (built with the boxes) while the leaves
     // that own rows (their share is about the rows' share of the particles) would leave an SM
     // fewer than 320 threads of the binary walk, a chain of dependent loads: 119 us for 1,399
     // leaves and 178 us for 35,981, 26,000 of them owners, against 34 and 135 us; 84,255
@@ -879,26 +826,12 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // From about 50,000 owners on its throughput wins (60,000 in a Sedov state 210 against
     // 255 us, 75,000 in a disc 379 against 393).
     const bool wide = (u64) L * n <= 320ull * c.sms * c.n_obj;
+    const LevelPlan lp = level_plan(L);
     WideTree wt{};
-    wt.level[0] = fb + (L - 1);
-    wt.n[0]     = L;
-    size_t wide_nodes = 0;
-    while (wide && wt.top + 1 < kWideLevels && wt.n[wt.top] > 8) {
-        wt.n[wt.top + 1] = (wt.n[wt.top] + 7) / 8;
-        wt.top++;
-        wide_nodes += wt.n[wt.top];
-    }
-    if ((e = c.wboxes.ensure(sizeof(NodeBoxF) * (wide_nodes + 1), s)) != cudaSuccess) return e;
-    {
-        NodeBoxF *at = c.wboxes.as<NodeBoxF>();
-        for (int m = 1; m <= wt.top; m++) {
-            wt.level[m] = at;
-            at += wt.n[m];
-        }
-        auto lv = [&](int m) { return m <= wt.top ? const_cast<NodeBoxF *>(wt.level[m]) : nullptr; };
-        for (int m = 0; m < wt.top; m += 3) {
-            { k_wide_levels<<<div_up(wt.n[m], 512), 512, 0, s>>>(wt.level[m], wt.n[m], lv(m + 1), lv(m + 2), lv(m + 3)); GBSPH_COUNTED; }
-        }
+    wt.top = lp.top;
+    for (int m = 0; m <= lp.top; m++) {
+        wt.level[m] = m ? c.wboxes.as<NodeBoxF>() + lp.at[m] : fb + (L - 1);
+        wt.n[m]     = lp.n[m];
     }
     // Owner leaves first: they also record, per leaf, the largest threshold of the rows
     // it owns, which lets stage 1 drop leaves that no owned row can pair with (and skip

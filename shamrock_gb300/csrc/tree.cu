@@ -381,9 +381,8 @@ struct LeafPlace {
 template<class K>
 __global__ void k_karras(const K *__restrict__ m, u32 L, u32 *__restrict__ lchild,
                          u32 *__restrict__ rchild, u8 *__restrict__ lflag, u8 *__restrict__ rflag,
-                         u32 *__restrict__ endrange, u32 *__restrict__ parent, u32 *__restrict__ visit) {
+                         u32 *__restrict__ endrange, u32 *__restrict__ parent) {
     u32 ui = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ui < L) visit[ui] = 0; // the counters of the pass over the boxes
     if (ui == 0) parent[0] = kNone;
     if (ui + 1 >= L) return;
     i32 i = (i32) ui;
@@ -460,19 +459,65 @@ __device__ __forceinline__ void store_box(NodeBox *b, const BoxKeys &k) {
     p[3]       = make_double2(ordered_to_f64(k.hi[2]), 0.0);
 }
 
-// One thread per leaf; of two siblings the one that arrives last unites both boxes and goes
-// on up, with its own box in registers, and writes the FP32 copies and the child-pair records
-// that the neighbour search walks (passes of their own over the boxes otherwise).  The links of the parent are fetched beside the
-// counter, as a level costs the latencies that follow each other (about 1.5 us).
-// 1,048,576 particles 117 -> 99 us, 8.5 M 471 -> 446 us, of which the copies and records take 5
-// and 59 (18 and 130 us as passes of their own).
-__global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 *__restrict__ sx,
-                                const f64 *__restrict__ sy, const f64 *__restrict__ sz,
-                                const f64 *__restrict__ sh, f64 htol, const u32 *__restrict__ lchild,
-                                const u32 *__restrict__ rchild, const u8 *__restrict__ lflag,
-                                const u8 *__restrict__ rflag, const u32 *__restrict__ parent,
-                                u32 *__restrict__ visit, NodeBox *__restrict__ boxes, NodeBoxF *__restrict__ fb,
-                                NodePairF *__restrict__ rec) {
+__device__ __forceinline__ BoxKeys no_box() {
+    BoxKeys k;
+#pragma unroll
+    for (int c = 0; c < 3; c++) k.lo[c] = ~0ull, k.hi[c] = 0ull;
+    k.rint = 0ull;
+    return k;
+}
+__device__ __forceinline__ void unite(BoxKeys &k, const BoxKeys &o) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        min_key(k.lo[c], o.lo[c]);
+        max_key(k.hi[c], o.hi[c]);
+    }
+    max_key(k.rint, o.rint);
+}
+__device__ __forceinline__ BoxKeys load_keys(const NodeBox *__restrict__ b) {
+    const double2 *s = (const double2 *) b;
+    const double2 s0 = s[0], s1 = s[1], s2 = s[2];
+    const f64 hz = ((const f64 *) b)[6];
+    return BoxKeys{{f64_to_ordered(s0.x), f64_to_ordered(s0.y), f64_to_ordered(s1.x)},
+                   {f64_to_ordered(s2.x), f64_to_ordered(s2.y), f64_to_ordered(hz)},
+                   is_nan_bits(s1.y) ? 0ull : f64_to_ordered(s1.y)};
+}
+__device__ __forceinline__ NodeBoxF box_f32(const BoxKeys &k) {
+    NodeBoxF f;
+    f.lo = make_float4(narrow64(ordered_to_f64(k.lo[0])), narrow64(ordered_to_f64(k.lo[1])),
+                       narrow64(ordered_to_f64(k.lo[2])), narrow64(__dmul_rn(ordered_to_f64(k.rint), kRkern)));
+    f.hi = make_float4(narrow64(ordered_to_f64(k.hi[0])), narrow64(ordered_to_f64(k.hi[1])),
+                       narrow64(ordered_to_f64(k.hi[2])), 0.f);
+    return f;
+}
+
+// a node's box, its FP32 copy, and the copy in its parent's child-pair record
+__device__ __forceinline__ void put_node(u32 node, u32 off, const BoxKeys &k, const u32 *__restrict__ lchild,
+                                         const u8 *__restrict__ lflag, const u32 *__restrict__ parent,
+                                         NodeBox *__restrict__ boxes, NodeBoxF *__restrict__ fb,
+                                         NodePairF *__restrict__ rec) {
+    store_box(&boxes[node], k);
+    NodeBoxF f = box_f32(k);
+    fb[node]   = f;
+    const u32 p = parent[node];
+    if (p == kNone) return;
+    f.hi.w = __uint_as_float(node);
+    if (lchild[p] + off * (u32) lflag[p] == node) rec[p].l = f;
+    else rec[p].r = f;
+}
+
+// Boxes of the nodes without a walk up the tree: an internal node covers a range of leaves,
+// whose box is united from the few nodes of the 8-ary hierarchy that make it up (minimum and
+// maximum are exact, so the order does not matter).  A walk with arrival counters is a chain
+// of one to two microseconds a level.  Leaves, levels and nodes together, against the walk and
+// the hierarchy built after it: 1,399 leaves 23 us against 31, 35,981 33 against 49, 239,928 79
+// against 103, 2.0 M 373 against 446 (bytes: 0.28 GB of boxes and records there, 45 us).
+__global__ void __launch_bounds__(256) k_leaf_boxes(const u32 *__restrict__ reduc, u32 L, const f64 *__restrict__ sx,
+                                                    const f64 *__restrict__ sy, const f64 *__restrict__ sz,
+                                                    const f64 *__restrict__ sh, f64 htol,
+                                                    const u32 *__restrict__ lchild, const u8 *__restrict__ lflag,
+                                                    const u32 *__restrict__ parent, NodeBox *__restrict__ boxes,
+                                                    NodeBoxF *__restrict__ fb, NodePairF *__restrict__ rec) {
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= L) return;
     const f64 big = 1.7976931348623157e308;
@@ -498,50 +543,74 @@ __global__ void k_leaf_boxes_up(const u32 *__restrict__ reduc, u32 L, const f64 
             max_key(hm, is_nan_bits(h) ? 0ull : f64_to_ordered(h));
         }
     }
-    k.rint   = f64_to_ordered(sh ? __dmul_rn(ordered_to_f64(hm), htol) : 0.0);
-    u32 off  = L - 1;
-    u32 node = off + l;
-    store_box(&boxes[node], k);
-    NodeBoxF f; // rounding is monotone, so a united box's FP32 copy is the union of the copies
-    f.lo = make_float4(narrow64(ordered_to_f64(k.lo[0])), narrow64(ordered_to_f64(k.lo[1])),
-                       narrow64(ordered_to_f64(k.lo[2])), narrow64(__dmul_rn(ordered_to_f64(k.rint), kRkern)));
-    f.hi = make_float4(narrow64(ordered_to_f64(k.hi[0])), narrow64(ordered_to_f64(k.hi[1])),
-                       narrow64(ordered_to_f64(k.hi[2])), 0.f);
-    fb[node] = f;
-    __threadfence();
-    u32 p = parent[node];
-    while (p != kNone) {
-        const u32 a = lchild[p] + off * (u32) lflag[p];
-        const u32 b = rchild[p] + off * (u32) rflag[p];
-        const u32 up = parent[p];
-        if (atomicAdd(&visit[p], 1u) == 0) return;
-        __threadfence();
-        const u32 sib    = a == node ? b : a;
-        const double2 *s = (const double2 *) &boxes[sib];
-        const float4 glo = __ldcg(&fb[sib].lo), ghi = __ldcg(&fb[sib].hi);
-        const double2 s0 = __ldcg(s), s1 = __ldcg(s + 1), s2 = __ldcg(s + 2), s3 = __ldcg(s + 3);
-        const f64 slo[3] = {s0.x, s0.y, s1.x}, shi[3] = {s2.x, s2.y, s3.x};
+    k.rint = f64_to_ordered(sh ? __dmul_rn(ordered_to_f64(hm), htol) : 0.0);
+    put_node(L - 1 + l, L - 1, k, lchild, lflag, parent, boxes, fb, rec);
+}
+
+// three levels of the hierarchy above n boxes: 512 of them to 64, 8 and 1 per block
+__device__ __forceinline__ BoxKeys unite8(BoxKeys k) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        BoxKeys x;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            min_key(k.lo[c], f64_to_ordered(slo[c]));
-            max_key(k.hi[c], f64_to_ordered(shi[c]));
+            x.lo[c] = __shfl_xor_sync(0xffffffffu, k.lo[c], o);
+            x.hi[c] = __shfl_xor_sync(0xffffffffu, k.hi[c], o);
         }
-        const u64 sr = f64_to_ordered(s1.y);
-        if (is_nan_bits(ordered_to_f64(k.rint))) k.rint = sr;
-        else if (!is_nan_bits(s1.y)) max_key(k.rint, sr);
-        store_box(&boxes[p], k);
-        NodePairF pair{f, NodeBoxF{glo, ghi}};
-        if (a != node) pair = NodePairF{NodeBoxF{glo, ghi}, f};
-        pair.l.hi.w = __uint_as_float(a);
-        pair.r.hi.w = __uint_as_float(b);
-        rec[p]      = pair;
-        f.lo = make_float4(fminf(f.lo.x, glo.x), fminf(f.lo.y, glo.y), fminf(f.lo.z, glo.z), fmaxf(f.lo.w, glo.w));
-        f.hi = make_float4(fmaxf(f.hi.x, ghi.x), fmaxf(f.hi.y, ghi.y), fmaxf(f.hi.z, ghi.z), 0.f);
-        fb[p] = f;
-        __threadfence();
-        node = p;
-        p    = up;
+        x.rint = __shfl_xor_sync(0xffffffffu, k.rint, o);
+        unite(k, x);
     }
+    return k;
+}
+__global__ void __launch_bounds__(512) k_box_levels(const NodeBox *__restrict__ in, LevelPlan lp, int m,
+                                                    NodeBox *__restrict__ lb, NodeBoxF *__restrict__ wb) {
+    __shared__ BoxKeys s1[64], s2[8];
+    const u32 t = threadIdx.x, i = blockIdx.x * 512 + t;
+    auto put = [&](int level, u32 o, const BoxKeys &k) {
+        if (level > lp.top || o >= lp.n[level]) return;
+        store_box(&lb[lp.at[level] + o], k);
+        wb[lp.at[level] + o] = box_f32(k);
+    };
+    BoxKeys k = unite8(i < lp.n[m] ? load_keys(&in[i]) : no_box());
+    if ((t & 7) == 0) {
+        s1[t / 8] = k;
+        put(m + 1, blockIdx.x * 64 + t / 8, k);
+    }
+    __syncthreads();
+    if (t < 64) {
+        k = unite8(s1[t]);
+        if ((t & 7) == 0) {
+            s2[t / 8] = k;
+            put(m + 2, blockIdx.x * 8 + t / 8, k);
+        }
+    }
+    __syncthreads();
+    if (t < 32) {
+        k = unite8(t < 8 ? s2[t] : no_box());
+        if (t == 0) put(m + 3, blockIdx.x, k);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_node_boxes(u32 L, LevelPlan lp, const u32 *__restrict__ endrange,
+                                                    const u32 *__restrict__ lchild, const u8 *__restrict__ lflag,
+                                                    const u32 *__restrict__ parent, const NodeBox *__restrict__ lb,
+                                                    NodeBox *boxes, NodeBoxF *__restrict__ fb,
+                                                    NodePairF *__restrict__ rec) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i + 1 >= L) return;
+    const u32 j = endrange[i];
+    u32 a = min(i, j), b = max(i, j) + 1; // the nodes [a, b) of level m
+    const NodeBox *level = boxes + (L - 1);
+    BoxKeys k            = no_box();
+    for (int m = 0; a < b; m++) {
+        const bool top = m == lp.top;
+        while (a < b && ((a & 7u) || top)) unite(k, load_keys(&level[a++]));
+        while (a < b && (b & 7u)) unite(k, load_keys(&level[--b]));
+        a >>= 3;
+        b >>= 3;
+        level = lb + lp.at[min(m + 1, lp.top)];
+    }
+    put_node(i, L - 1, k, lchild, lflag, parent, boxes, fb, rec);
 }
 
 // Up to this many keys (padded to a power of two) the network sorts at once.  Where keys are
@@ -637,19 +706,28 @@ cudaError_t tree_build_impl(Ctx &c, const f64 *x, const f64 *y, const f64 *z, co
     ENS(c.rflag, I + 1);
     ENS(c.endrange, sizeof(u32) * (I + 1));
     ENS(c.parent, sizeof(u32) * Tn);
-    ENS(c.visit, sizeof(u32) * (I + 1));
     ENS(c.boxes, sizeof(NodeBox) * Tn);
     ENS(c.fboxes, sizeof(NodeBoxF) * Tn);
     ENS(c.fpairs, sizeof(NodePairF) * (size_t) L);
+    const LevelPlan lp = level_plan(L);
+    ENS(c.lboxes, sizeof(NodeBox) * ((size_t) lp.total + 1));
+    ENS(c.wboxes, sizeof(NodeBoxF) * ((size_t) lp.total + 1));
 #undef ENS
     { k_karras<K><<<div_up(L, T), T, 0, s>>>(c.reduced.as<K>(), L, c.lchild.as<u32>(),
                                            c.rchild.as<u32>(), c.lflag.as<u8>(), c.rflag.as<u8>(),
-                                           c.endrange.as<u32>(), c.parent.as<u32>(), c.visit.as<u32>()); GBSPH_COUNTED; }
-    { k_leaf_boxes_up<<<div_up(L, T), T, 0, s>>>(
-        c.reduc.as<u32>(), L, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
-        h ? c.sh.as<f64>() : nullptr, htol, c.lchild.as<u32>(), c.rchild.as<u32>(),
-        c.lflag.as<u8>(), c.rflag.as<u8>(), c.parent.as<u32>(), c.visit.as<u32>(),
-        c.boxes.as<NodeBox>(), c.fboxes.as<NodeBoxF>(), c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
+                                           c.endrange.as<u32>(), c.parent.as<u32>()); GBSPH_COUNTED; }
+    NodeBox *boxes = c.boxes.as<NodeBox>();
+    { k_leaf_boxes<<<div_up(L, T), T, 0, s>>>(c.reduc.as<u32>(), L, c.sx.as<f64>(), c.sy.as<f64>(), c.sz.as<f64>(),
+                                            h ? c.sh.as<f64>() : nullptr, htol, c.lchild.as<u32>(), c.lflag.as<u8>(),
+                                            c.parent.as<u32>(), boxes, c.fboxes.as<NodeBoxF>(),
+                                            c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
+    for (int m = 0; m < lp.top; m += 3)
+        { k_box_levels<<<div_up(lp.n[m], 512), 512, 0, s>>>(m ? c.lboxes.as<NodeBox>() + lp.at[m] : boxes + (L - 1), lp, m,
+                                                          c.lboxes.as<NodeBox>(), c.wboxes.as<NodeBoxF>()); GBSPH_COUNTED; }
+    if (L > 1)
+        { k_node_boxes<<<div_up(L - 1, T), T, 0, s>>>(L, lp, c.endrange.as<u32>(), c.lchild.as<u32>(), c.lflag.as<u8>(),
+                                                    c.parent.as<u32>(), c.lboxes.as<NodeBox>(), boxes,
+                                                    c.fboxes.as<NodeBoxF>(), c.fpairs.as<NodePairF>()); GBSPH_COUNTED; }
     return cudaGetLastError();
 }
 
