@@ -81,10 +81,9 @@ struct AdjLocal {
 };
 
 // Four entries of a row by one load (rows of the library's cache start on 16-byte boundaries
-// and their slots are padded to four), for the density passes, which load little else: a
-// thread per row reads entries from a line of its own, so four single loads cost four times
-// the L1 wavefronts, and they ran at 80 % of the L1's rate.  With the four records requested
-// together k_adj_omega_a / _b of 262,144 particles 168 / 195 -> 109 / 121 us, disc of 300,007
+// and their slots are padded to four), for the density passes, which load little else and
+// ran at 80 % of the L1's rate, with one entry and one record in flight a thread.  With the
+// four records requested together k_adj_omega_a / _b of 262,144 particles 168 / 195 -> 109 / 121 us, disc of 300,007
 // 150 / 202 -> 96 / 118 us.  (k_adj_derivs, bound by its arithmetic, gains nothing.)
 __device__ __forceinline__ uint4 entries4(const u32 *__restrict__ ent, u32 k) {
     return __ldg((const uint4 *) (ent + k));

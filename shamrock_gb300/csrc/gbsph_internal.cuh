@@ -7,8 +7,8 @@
 //   rank       : position in Morton-sorted order, [0, N); sort_index[rank] = merged id
 //   row        : position of a local particle in rank order, [0, n_local);
 //                row_rank[row] = its rank, row_local[row] = its local id.
-// Pair kernels run one thread per row so that neighbouring threads touch
-// neighbouring particles; all per-particle fields they read are gathered into
+// Pair kernels run one thread or four lanes per row, in row order, so that neighbouring
+// threads touch neighbouring particles; all per-particle fields they read are gathered into
 // rank order first.
 #pragma once
 

@@ -247,7 +247,8 @@ __device__ __forceinline__ void derivs_row_comp(const RowSpace &rs, const MixedS
 }
 
 // Compensated derivatives + v_sig + leapfrog corrector + CFL, the counterpart of
-// k_derivs_step_mixed (same outputs and reductions)
+// k_derivs_sums_mixed and k_correct_mixed in one (same outputs and reductions).  A thread per
+// row: the loop is bound by the issue of its double-float arithmetic, not by its loads.
 template<bool COND>
 __global__ void __launch_bounds__(128) k_derivs_step_comp(RowSpace rs, MixedSpace ms,
                                                           const float4 *__restrict__ E,
