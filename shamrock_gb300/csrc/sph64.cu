@@ -821,12 +821,35 @@ __device__ __forceinline__ f64 fmod_wrap(f64 r, const WrapAxis &w) {
     return fmod_far(r, w.delt);
 }
 
+// acceleration of the central point mass, component n = -GM x over r^3; the plain operators
+// where a quotient or the root fails its proof
+__device__ __noinline__ f64 point_mass_plain(f64 x, f64 y, f64 z, f64 n) {
+    f64 r  = sqrt(x * x + y * y + z * z);
+    f64 r3 = r * r * r;
+    return n / r3;
+}
+__device__ __forceinline__ void point_mass(f64 mGM, f64 x, f64 y, f64 z, f64 *ax, f64 *ay, f64 *az) {
+    bool bad     = false;
+    const f64 r  = root_value(root64(mul64i(x, x) + mul64i(y, y) + mul64i(z, z), bad));
+    const f64 r3 = mul64i(mul64i(r, r), r);
+    auto over    = [&](f64 n) {
+        const u64 b    = bits64(n), sign = b & 0x8000000000000000ull;
+        bool odd       = bad;
+        const f64 q    = quotient64(from64(b ^ sign), r3, odd);
+        return odd ? point_mass_plain(x, y, z, n) : from64(bits64(q) | sign);
+    };
+    *ax = over(mul64i(mGM, x));
+    *ay = over(mul64i(mGM, y));
+    *az = over(mul64i(mGM, z));
+}
+
 // leapfrog predictor (half kick, drift, half kick) + periodic wrap, one pass.  Bound by the
 // FP64 pipe (16 cycles of an SM for a warp's instruction): its sums are the 23 FP64
 // instructions left of about 55, the products go to the integer pipes, comparisons are
 // integer ones and the box's constants come from the host: 1,048,576 particles 100 -> 63 us,
 // 8.5 M 793 -> 475 us (1.22 GB of fields, 185 us at the copy rate); with the products on
-// the FP64 pipe too 75 and 585 us.
+// the FP64 pipe too 75 and 585 us.  With the point mass (a root and three quotients by the
+// forms of lean64.cuh) 1,000,003 particles 102 -> 72 us.
 __global__ void __launch_bounds__(256, 5) k_predict(LocalFields lf, u32 n, f64 dt, f64 dt_half, int periodic, Wrap wrap, f64 mGM,
                           f64 *__restrict__ ext_x, f64 *__restrict__ ext_y, f64 *__restrict__ ext_z) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -842,11 +865,7 @@ __global__ void __launch_bounds__(256, 5) k_predict(LocalFields lf, u32 n, f64 d
     u  = u + ku;
     if (ext_x) {
         // central point mass at the drifted position, before the wrap
-        f64 r  = sqrt(x * x + y * y + z * z);
-        f64 r3 = r * r * r;
-        ext_x[i] = mGM * x / r3;
-        ext_y[i] = mGM * y / r3;
-        ext_z[i] = mGM * z / r3;
+        point_mass(mGM, x, y, z, &ext_x[i], &ext_y[i], &ext_z[i]);
     }
     if (periodic) {
         f64 p[3] = {x, y, z};
