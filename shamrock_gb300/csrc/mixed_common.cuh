@@ -37,11 +37,13 @@ __device__ __forceinline__ float hi32(f64 v) { return __double2float_rn(v); }
 __device__ __forceinline__ float lo32(f64 v) { return __double2float_rn(v - (f64) __double2float_rn(v)); }
 // 1/v from the FP32 reciprocal refined by one FP64 Newton step (relative error ~1e-14,
 // so its FP32 rounding is the correctly rounded 1/v but for rare ties); plain FP64
-// division where the FP32 reciprocal leaves the normal range
+// division where the FP32 reciprocal leaves the normal range (a call, and the conversions
+// on the integer pipes: each would be an FP64-pipe instruction beside the two of the step)
+__device__ __noinline__ f64 rcp64_plain(f64 v) { return 1.0 / v; }
 __device__ __forceinline__ f64 rcp64(f64 v) {
-    const float y0 = __frcp_rn(__double2float_rn(v));
-    if (!(fabsf(y0) < 3.0e38f && fabsf(y0) > 1.0e-37f)) return 1.0 / v;
-    const f64 y = (f64) y0;
+    const float y0 = __frcp_rn(narrow64(v));
+    if (!(fabsf(y0) < 3.0e38f && fabsf(y0) > 1.0e-37f)) return rcp64_plain(v);
+    const f64 y = widen32(y0);
     return y * (2.0 - v * y);
 }
 // kNorm3d / hfact^3: rho_sum / rho_h = kC sum f(q), h (d rho/dh) / rho_h = -kC sum (3f + q f')
