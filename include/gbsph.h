@@ -94,7 +94,7 @@ typedef struct {
     double htol_up_coarse, htol_up_fine; /* 1.1, 1.1 */
     double epsilon_h;               /* 1e-6 */
     uint32_t h_iter_per_subcycles;  /* 50 */
-    uint32_t h_max_subcycles;       /* 100 */
+    uint32_t h_max_subcycles;       /* 100; at least 1 */
     uint32_t tree_reduction_level;  /* 3 */
     uint32_t periodic;              /* 1 periodic box, 0 free boundaries */
     double box_min[3], box_max[3];

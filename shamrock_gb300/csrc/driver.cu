@@ -648,6 +648,8 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
     REQUIRE_ARG(cfg->av_kind == GBSPH_AV_CONSTANT || cfg->av_kind == GBSPH_AV_VARYING_CD10 ||
                     cfg->av_kind == GBSPH_AV_VARYING_MM97,
                 "unknown artificial viscosity");
+    // without a sub-cycle there are no rows, no cache and no h for the rest of the step
+    REQUIRE_ARG(cfg->h_max_subcycles > 0, "h_max_subcycles must be at least 1");
     // varying viscosity (CD10 or MM97): per-particle alpha from the velocity gradients
     const bool cd10 = cfg->av_kind != GBSPH_AV_CONSTANT;
     REQUIRE_ARG(!cd10 || (p->alpha_AV && p->soundspeed),
@@ -779,8 +781,6 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         CU(dens_polish_df(c, rs, c.h_old_row.as<f64>(), c.hnew_row.as<f64>(), c.eps_row.as<f64>(),
                           cfg->htol_up_coarse, cfg->htol_up_fine, c.omega_local.as<f64>()));
         CU(scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h));
-    } else if (hstep == 0 && cfg->h_max_subcycles == 0) {
-        CU(after_h());
     }
     if (p->omega)
         CU(cudaMemcpyAsync(p->omega, c.omega_local.p, 8 * (size_t) n, cudaMemcpyDeviceToDevice, s));
