@@ -268,11 +268,18 @@ GBSPH_HD double mul64i(double a, double b) {
 // zero proves the cell (the correctly rounded quotient lies in the same cell); a zero
 // fraction, infinities and NaN take the quotient itself.  Two FP64 instructions instead of
 // about 25 with the clamps and the division.
+// The device's own conversion (saturating, NaN to 2^31) decides what is no cell: a quotient of
+// 0 / 0 or inf / inf, in a box without extent along the axis or an unbounded one, takes the
+// top cell.  The host check's twin, where such a conversion is undefined, takes cell 0.
 static GBSPH_HD_RARE uint32_t grid_cell_plain(double p, double lo, double hi, double step, uint32_t top) {
     const double r = fmin(fmax(p, lo), hi);
     const double q = (r - lo) / step;
+#ifdef __CUDA_ARCH__
+    return min(__double2uint_rz(q), top);
+#else
     if (!(q > 0.)) return 0u;
     return q < (double) top ? (uint32_t) q : top;
+#endif
 }
 GBSPH_HD uint32_t grid_cell(double p, double lo, double hi, double step, double inv, uint32_t top) {
     const double d    = p - lo;
