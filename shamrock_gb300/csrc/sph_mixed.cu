@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
     // float bits of the reductions' operands, all of them non-negative (or NaN, which
     // orders above): their unsigned order is that of the values
     u32 ev2 = 0, dtm = 0xffffffffu, c_fa = 0, c_fu = 0, c_a = 0, c_du = 0;
-    float v2 = 0.f;
+    f64 v2 = 0;
     for (u32 i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
         const F8 o = ldg256(&sums[2 * (size_t) rank_of[i]]);
         const float Fx = o.a.x, Fy = o.a.y, Fz = o.a.z, U = o.a.w, vm = o.b.x;
@@ -842,12 +842,13 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
         lf.vy[iv] = nvy;
         lf.vz[iv] = nvz;
         lf.u[i]   = u + hdt * (tdu - odu);
-        // the rerun test, the mean |v|^2 and the CFL step only need FP32 (they feed a
-        // 1e-2 threshold, a normalisation and a time step)
+        // the rerun test, each |v|^2 and the CFL step only need FP32 (they feed a 1e-2
+        // threshold, a normalisation and a time step); the sum of |v|^2 over the particles is
+        // FP64, so neither its error nor its range depends on how many a thread adds up
         const float fix = narrow64(ix), fiy = narrow64(iy), fiz = narrow64(iz);
         ev2 = max(ev2, __float_as_uint(fix * fix + fiy * fiy + fiz * fiz));
         const float fvx = narrow64(nvx), fvy = narrow64(nvy), fvz = narrow64(nvz);
-        v2 += fvx * fvx + fvy * fvy + fvz * fvz;
+        v2 += widen32(fvx * fvx + fvy * fvy + fvz * fvz);
         const float ffx = narrow64(fx), ffy = narrow64(fy), ffz = narrow64(fz);
         const float abs_a = sqrtf(ffx * ffx + ffy * ffy + ffz * ffz);
         float dt = fminf(__int_as_float(0x7f800000), (float) C_cour * hf / vm);
@@ -855,9 +856,9 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
         dtm      = min(dtm, __float_as_uint(dt));
     }
     __shared__ u32 part[6][8];
-    __shared__ float part_v2[8];
+    __shared__ f64 part_v2[8];
     const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    v2 = warp_reduce(v2, OpAddF32{});
+    v2 = warp_reduce(v2, OpAddF64{});
     const u32 r[6] = {__reduce_max_sync(0xffffffffu, ev2), __reduce_min_sync(0xffffffffu, dtm),
                       COND ? __reduce_max_sync(0xffffffffu, c_fa) : 0u,
                       COND ? __reduce_max_sync(0xffffffffu, c_fu) : 0u,
@@ -884,9 +885,9 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
             break;
         }
         case 2: {
-            float s = 0.f;
+            f64 s = 0;
             for (int k = 0; k < 8; k++) s += part_v2[k];
-            atomicAdd(&sc->sum_v2, (f64) s);
+            atomicAdd(&sc->sum_v2, s);
             break;
         }
         case 3: raise_u64(&sc->cond_fa, max_of(2)); break;
