@@ -625,6 +625,16 @@ static f64 err_estimate(u64 sum_bits, u64 max_bits) {
     return kErrBase + kErrCond * s / m;
 }
 
+// Whether Omega is taken while the host waits for the h iteration's result, which it does not
+// need.  Ahead of the wait it saves 3 us a step (2,048 Sedov particles 447 -> 444 us, 37,044
+// 591 -> 588) and nothing from 131,072 on (988 against 986, 1,048,576 3805 against 3808); where
+// h then takes another sub-cycle, the pass was for nothing: 10 to 21 us for so few rows, 58 at
+// 131,072, and 207 to 498 in FP64.  So only for few rows, and only after a step whose h took one
+// sub-cycle (which can cost time here and nothing else: Omega is the last h's either way).
+static bool omega_ahead(const Ctx &c, u32 n, u32 tier) {
+    return tier == GBSPH_MIXED && c.one_subcycle && quad_rows(c, n);
+}
+
 // One step (Solver::evolve_once) in one precision tier (GBSPH_FP64, GBSPH_MIXED or
 // GBSPH_MIXED_COMPENSATED).  With a tape, exactly tape->forced_iters corrector
 // evaluations run and the velocity / energy before each is recorded.
@@ -697,16 +707,14 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
     f64 max_eps = 0, min_eps = 0;
     bool converged = false;
     RowSpace rs{};
-    // What follows an h iteration whether or not its sub-cycle converged: the iterated h is
-    // written back, and Omega taken at it (a sub-cycle that follows builds its own cache, and
-    // its Omega replaces this one).  The compensated tier finishes h first, so only then.
-    auto after_h = [&]() -> cudaError_t {
-        cudaError_t e = scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h);
-        if (e != cudaSuccess || comp) return e;
+    // the iterated h is written back whether or not its sub-cycle converged
+    auto store_h   = [&]() { return scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h); };
+    auto take_omega = [&]() -> cudaError_t {
         if (mixed)
             return omega_compact_mixed(c, rs, n + c.n_ghost, n, lf.h, c.hnew_row.as<f64>(), c.omega_local.as<f64>());
         return omega64(c, rs, c.hnew_row.as<f64>(), cfg->pmass, c.omega_local.as<f64>(), c.row_local.as<u32>());
     };
+    bool omega_taken = false; // at the last sub-cycle's h
     for (; hstep < cfg->h_max_subcycles; hstep++) {
         if (cfg->periodic) {
             CU(periodic_ghosts(c, lf.x, lf.y, lf.z, lf.vs, lf.h, n, cfg->box_min, cfg->box_max,
@@ -740,7 +748,9 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                                c.eps_row.as<f64>(), cfg->pmass, cfg->htol_up_coarse,
                                cfg->htol_up_fine, cfg->h_iter_per_subcycles, eps_p));
             CU(post_scalars(c));
-            CU(after_h());
+            CU(store_h());
+            omega_taken = hstep == 0 && omega_ahead(c, n, tier);
+            if (omega_taken) CU(take_omega());
             CU(wait_scalars(c));
             max_eps     = ordered_to_f64(c.h_scalars->eps_max);
             min_eps     = ordered_to_f64(c.h_scalars->eps_min);
@@ -762,7 +772,7 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
                 iters_total++;
                 if (max_eps < cfg->epsilon_h) break;
             }
-            CU(after_h());
+            CU(store_h());
         }
         lg.h_iterations += iters_total;
         converged = (max_eps < cfg->epsilon_h) && !(min_eps < 0);
@@ -771,6 +781,7 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
     // hstep + 1 sub-cycles ran; h_max_subcycles + 1 flags "never converged", after which
     // the reference logs an error and carries on with the step (Solver.cpp:1271-1273)
     lg.h_subcycles = hstep + 1;
+    c.one_subcycle = hstep == 0;
     lg.max_eps_h   = max_eps;
     lg.n_ghost     = c.n_ghost;
     lg.leaf_count  = c.leaf_count;
@@ -781,6 +792,8 @@ static int evolve_tier(gbsph_ctx *ctx, const gbsph_particles *p, const gbsph_con
         CU(dens_polish_df(c, rs, c.h_old_row.as<f64>(), c.hnew_row.as<f64>(), c.eps_row.as<f64>(),
                           cfg->htol_up_coarse, cfg->htol_up_fine, c.omega_local.as<f64>()));
         CU(scatter_rows(c, n, c.hnew_row.as<f64>(), lf.h));
+    } else if (!omega_taken) {
+        CU(take_omega());
     }
     if (p->omega)
         CU(cudaMemcpyAsync(p->omega, c.omega_local.p, 8 * (size_t) n, cudaMemcpyDeviceToDevice, s));

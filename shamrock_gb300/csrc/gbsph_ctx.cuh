@@ -200,6 +200,8 @@ struct Ctx {
     bool cond_this_step = true;
     DevBuf guard_state;
 
+    bool one_subcycle = false; // h of the last step converged in its first sub-cycle
+
     // ---- per-row / per-local work arrays
     DevBuf h_old_row, eps_row, omega_local, a_old, du_old, hnew_row, omega_row;
     DevBuf aext; // external acceleration of the step (3 n, SoA)
