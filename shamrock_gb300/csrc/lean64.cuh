@@ -10,7 +10,8 @@
 // last place is exact in an FMA, and g is the correctly rounded root if and only if
 //     -g u < x - g^2 <= g u,        u = ulp(g)     (the square (g +- u/2)^2 expanded),
 // q the correctly rounded quotient if and only if |a - b q| < b ulp(q) / 2 (a quotient of
-// two doubles never lies half-way).  A value that fails the proof (about one in 10^4), and
+// two doubles never lies half-way).  A value that fails the proof (one root in 10^5 and three
+// quotients in 10^6 of ordinary size, tests/native/narrow64_check.cpp), and
 // operands outside the normal range, report `bad` and the caller evaluates the expression
 // with the plain operators, so results are those of the plain operators always.
 // For a denominator known per particle the reciprocal is kept as y = RN(1/b) and the
