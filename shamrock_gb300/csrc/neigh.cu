@@ -210,16 +210,13 @@ __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= t.L) return;
     u32 base = l * cap;
-    float thr_own = 0.f;
-    if (leaf_thr) {
-        const u32 tb = leaf_thr[l];
-        if (tb == 0) { // no row is owned by this leaf: stage 2 never reads its list
-            cnt[l] = 0;
-            off[l] = base;
-            return;
-        }
-        thr_own = __uint_as_float(tb);
+    const u32 tb = leaf_thr[l];
+    if (tb == 0) { // no row is owned by this leaf: stage 2 never reads its list
+        cnt[l] = 0;
+        off[l] = base;
+        return;
     }
+    const float thr_own = __uint_as_float(tb);
     LazyLeafCrit crit(t, l);
     const u32 offn = t.off();
     F8 fa = ldg256(&fb[offn + l]), fr = ldg256(&fb[0]);
@@ -246,13 +243,12 @@ __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *
     // gaps are shrunk by the rounding band and the bound carries a 1e-5 margin, so the
     // skip is certain.
     auto keep = [&](const float4 &nlo, const float4 &nhi) -> bool {
-        if (!leaf_thr) return true;
         float gx = fmaxf(fmaxf(nlo.x - ahi.x, alo.x - nhi.x) - band_abs, 0.f);
         float gy = fmaxf(fmaxf(nlo.y - ahi.y, alo.y - nhi.y) - band_abs, 0.f);
         float gz = fmaxf(fmaxf(nlo.z - ahi.z, alo.z - nhi.z) - band_abs, 0.f);
         float d2 = gx * gx + gy * gy + gz * gz;
-        float tb = fmaxf(thr_own, nlo.w * nlo.w * 1.000001f);
-        return !(d2 > tb * 1.00001f);
+        float tmax = fmaxf(thr_own, nlo.w * nlo.w * 1.000001f);
+        return !(d2 > tmax * 1.00001f);
     };
     __shared__ u32 s_near[kNear][128]; // the first places of the lanes' stacks, a bank each
     u32 far[kStack - kNear];
@@ -531,11 +527,13 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 //   and the rows' box                      118 /  684    / 4.73 / 1.67 /  801
 // (a thread per row loads a record per candidate and row, 10 L1 wavefronts a request, and its
 // lanes diverge; at 48 registers, five blocks an SM, either of the last two steps is a loss).
-// Relative positions are rounded to FP32:
-// with S the largest of the rows' own, r^2 / thr of a pair near the threshold errs by at
-// most 2.1e-7 (2 S / sqrt(thr) + 2), and the hi/lo records themselves by 2.5e-14 M /
-// sqrt(thr) for coordinates of size M; a row for which these do not stay well inside the
-// band takes the FP64 test for every candidate.
+// Relative positions are rounded to FP32 (u = 2^-24, twice a coordinate): with S the rows'
+// largest relative coordinate, a separation errs by u (4 S + 3 |d|) an axis, so r^2 of a pair
+// near the threshold by u (8 sqrt(3) S / sqrt(thr) + 9) relative, and by 2.5e-14 M / sqrt(thr)
+// for the hi/lo records of coordinates of size M; the threshold's own roundings add 3 u.  A row
+// with S <= 6 sqrt(thr) and M <= 1e8 sqrt(thr) stays below 8.2e-6, inside the band; any other
+// takes the FP64 test for every candidate.  (An ordinary leaf is a few h wide, S about
+// sqrt(thr).)
 enum CacheMode { kCount = 0, kFill = 1, kOnePass = 2 };
 
 // the exact test (NeighbourCache.cpp:492-591); a call, as few candidates need it
@@ -611,8 +609,8 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
                 const float mine = lane < m ? fmaxf(fmaxf(fabsf(xa), fabsf(ya)), fabsf(za)) : 0.f;
                 const float S    = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(mine)));
                 const float M    = fmaxf(fmaxf(fabsf(Ph.x), fabsf(Ph.y)), fabsf(Ph.z));
-                // 2 S / sqrt(thr) + 2 <= 24 and M / sqrt(thr) <= 1e8
-                const bool ok = S * S <= 121.f * thr && M * M <= 1e16f * thr && thr > 1e-30f;
+                // S / sqrt(thr) <= 6 and M / sqrt(thr) <= 1e8
+                const bool ok = S * S <= 36.f * thr && M * M <= 1e16f * thr && thr > 1e-30f;
                 tlo           = ok ? thr * lo_f : __int_as_float(0x7fc00000);
                 tmax          = __uint_as_float(__reduce_max_sync(kAll, lane < m && ok ? __float_as_uint(tlo) : 0u));
                 if (__any_sync(kAll, lane < m && !ok)) tmax = __int_as_float(0x7fc00000);
