@@ -232,9 +232,10 @@ int gbsph_tree_query(gbsph_ctx *ctx, const double *qx, const double *qy, const d
  * positions of the last gbsph_build_tree call (built with h).  Pair test
  * !(r^2 > (h_a htol)^2 R^2 && r^2 > (h_b htol)^2 R^2), R = 2.
  * Replaces NeighbourCache::start_neighbors_cache_2stages,
- * shammodels/sph/src/modules/NeighbourCache.cpp:223-596.  With GBSPH_MIXED the pair
+ * shammodels/sph/src/modules/NeighbourCache.cpp:223-596.  In either precision the pair
  * test is first estimated in FP32 and only pairs within 1e-5 of the threshold are
- * decided in FP64: the cache is identical, the work mostly FP32. */
+ * decided in FP64: the cache is that of the FP64 test, the work mostly FP32.  The context
+ * keeps 64 bytes of FP32 positions per merged particle for it. */
 int gbsph_neighbour_cache(gbsph_ctx *ctx, uint32_t n_local, double htol, uint32_t precision,
                           void *stream);
 
@@ -279,7 +280,8 @@ int gbsph_eos_adiabatic(gbsph_ctx *ctx, const double *h, const double *u, uint32
 
 /* UpdateDerivs::update_derivs_constantAV, shammodels/sph/src/modules/UpdateDerivs.cpp:88-288;
  * with vsig != NULL also the v_sig maximum of Solver.cpp:2716-2788.
- * precision GBSPH_FP64 or GBSPH_MIXED. */
+ * precision GBSPH_FP64 or GBSPH_MIXED.  The n_merged particles are first staged in the
+ * context, which keeps 160 bytes (FP64) or 64 bytes (mixed) of each. */
 int gbsph_derivs_constAV(gbsph_ctx *ctx, const uint32_t *cnt, const uint32_t *scanned,
                          const uint32_t *entries, const double *x, const double *y,
                          const double *z, const double *vx, const double *vy, const double *vz,

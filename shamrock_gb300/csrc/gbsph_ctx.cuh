@@ -164,7 +164,7 @@ struct Ctx {
     u32 leaf_cap = 0, row_cap = 0; // one-pass slots per leaf / row (grown on overflow)
     u32 row_seen = 0;              // largest stage-2 row of the last build
     u64 slot_budget = 0;            // bytes of one-pass slots allowed (0: library default)
-    DevBuf leaf_cnt, leaf_off, leaf_ent; // stage 1 (leaf ids)
+    DevBuf leaf_cnt, leaf_off, leaf_ent; // stage 1 (rank ranges of candidate leaves)
     DevBuf leaf_head, next_row;          // the rows each leaf owns, linked
     DevBuf leaf_thr;                     // per leaf: FP32 bits of max thr over its owned rows
     DevBuf csr_cnt, csr_off, csr_ent;    // stage 2, per row, entries are ranks
@@ -177,7 +177,7 @@ struct Ctx {
     DevBuf ghost_block_counts;    // per block x 26
     DevBuf mx, my, mz, mh;        // merged positions / h (merged id order)
     f64 ghost_offsets[26][3];
-    DevBuf d_ghost_offsets;       // f64[26][3]
+    DevBuf d_ghost_offsets;       // the interfaces' bounds and offsets (ghosts.cu)
 
     // ---- per-step fields in rank order (corrector phase)
     DevBuf scs, sh2;

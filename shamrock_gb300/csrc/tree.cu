@@ -1,5 +1,5 @@
 // Compressed-leaf BVH build on the GPU: Morton keys, bitonic key/value sort, leaf
-// reduction, Karras radix tree, leaf AABB / interaction radius and bottom-up union.
+// reduction, Karras radix tree, AABB and interaction radius of leaves and nodes.
 // Bit-exact with the reference semantics (see the oracle restatement):
 //   Morton     shamtree/src/MortonCodeSet.cpp:63-118, shammath/sfc/morton.hpp:46-230
 //   sort       shamalgs/src/details/algorithm/bitonicSort_updated_usm.cpp:26-396
@@ -8,8 +8,9 @@
 //   AABB/field shamtree/src/KarrasRadixTreeAABB.cpp:33-140,
 //              shamtree/include/shamtree/KarrasRadixTreeField.hpp:134-222,
 //              shammodels/sph/src/Solver.cpp:1322-1356
-// The reference propagates node boxes with tree_depth full sweeps; here one
-// bottom-up pass with arrival counters produces the same exact min/max.
+// The reference propagates node boxes with tree_depth full sweeps; here a node's box is
+// united from the few boxes of an 8-ary hierarchy over the leaves that make up its range,
+// with the same exact min/max.
 
 #include "compact.cuh"
 #include "lean64.cuh"
