@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(128, 8) k_omega_compact_quads(RowSpace rs, Mix
 // consecutive ranks, share a line of the warp-wide gathers.  What bounds it now is the L1
 // data pipe (75 % of its wavefronts, issue slots 61 %; a thread per row: 50 % and 36 %,
 // waiting on its gathers).  Per launch, with the corrector pass below: 1,048,576 particles
-// of the jittered lattice 734 -> 440 + 53 us, disc of 1,000,003 1440 -> 457 + 51 us,
+// of the jittered lattice 734 -> 440 + 54 us, disc of 1,000,003 1440 -> 457 + 52 us,
 // homogeneous box of 8.5 M 5.96 -> 3.36 + 0.45 ms.
 struct PairTerms {
     float f, x, y, z, u; // force / r, separation, du/dt term
@@ -812,6 +812,8 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
     // orders above): their unsigned order is that of the values
     u32 ev2 = 0, dtm = 0xffffffffu, c_fa = 0, c_fu = 0, c_a = 0, c_du = 0;
     f64 v2 = 0;
+    float v2_four = 0.f;
+    u32 terms     = 0;
     for (u32 i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
         const F8 o = ldg256(&sums[2 * (size_t) rank_of[i]]);
         const float Fx = o.a.x, Fy = o.a.y, Fz = o.a.z, U = o.a.w, vm = o.b.x;
@@ -843,12 +845,17 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
         lf.vz[iv] = nvz;
         lf.u[i]   = u + hdt * (tdu - odu);
         // the rerun test, each |v|^2 and the CFL step only need FP32 (they feed a 1e-2
-        // threshold, a normalisation and a time step); the sum of |v|^2 over the particles is
-        // FP64, so neither its error nor its range depends on how many a thread adds up
+        // threshold, a normalisation and a time step).  |v|^2 is summed in FP32 over four
+        // particles of the thread and in FP64 beyond, so neither its error nor its range
+        // depends on how many there are
         const float fix = narrow64(ix), fiy = narrow64(iy), fiz = narrow64(iz);
         ev2 = max(ev2, __float_as_uint(fix * fix + fiy * fiy + fiz * fiz));
         const float fvx = narrow64(nvx), fvy = narrow64(nvy), fvz = narrow64(nvz);
-        v2 += widen32(fvx * fvx + fvy * fvy + fvz * fvz);
+        v2_four += fvx * fvx + fvy * fvy + fvz * fvz;
+        if ((++terms & 3u) == 0) {
+            v2 += widen32(v2_four);
+            v2_four = 0.f;
+        }
         const float ffx = narrow64(fx), ffy = narrow64(fy), ffz = narrow64(fz);
         const float abs_a = sqrtf(ffx * ffx + ffy * ffy + ffz * ffz);
         float dt = fminf(__int_as_float(0x7f800000), (float) C_cour * hf / vm);
@@ -856,9 +863,9 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
         dtm      = min(dtm, __float_as_uint(dt));
     }
     __shared__ u32 part[6][8];
-    __shared__ f64 part_v2[8];
+    __shared__ f64 part_v2[256];
     const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    v2 = warp_reduce(v2, OpAddF64{});
+    part_v2[threadIdx.x] = v2 + widen32(v2_four);
     const u32 r[6] = {__reduce_max_sync(0xffffffffu, ev2), __reduce_min_sync(0xffffffffu, dtm),
                       COND ? __reduce_max_sync(0xffffffffu, c_fa) : 0u,
                       COND ? __reduce_max_sync(0xffffffffu, c_fu) : 0u,
@@ -867,10 +874,18 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
     if (lane == 0) {
 #pragma unroll
         for (int q = 0; q < (COND ? 6 : 2); q++) part[q][w] = r[q];
-        part_v2[w] = v2;
     }
     __syncthreads();
-    if (threadIdx.x < (COND ? 7u : 3u)) {
+    // a warp adds up the block's |v|^2 (13 FP64 additions; 48 with a butterfly in every warp),
+    // another the rest
+    if (w == 1) {
+        f64 s = part_v2[lane];
+#pragma unroll
+        for (int k = 1; k < 8; k++) s += part_v2[lane + 32 * k];
+        s = warp_reduce(s, OpAddF64{});
+        if (lane == 0) atomicAdd(&sc->sum_v2, s);
+    }
+    if (threadIdx.x < (COND ? 6u : 2u)) {
         auto max_of = [&](int q) {
             u32 m = part[q][0];
             for (int k = 1; k < 8; k++) m = max(m, part[q][k]);
@@ -884,15 +899,9 @@ __global__ void __launch_bounds__(256) k_correct_mixed(u32 n, const u32 *__restr
             lower_u64(&sc->dt_min, f64_to_ordered((f64) __uint_as_float(m)));
             break;
         }
-        case 2: {
-            f64 s = 0;
-            for (int k = 0; k < 8; k++) s += part_v2[k];
-            atomicAdd(&sc->sum_v2, s);
-            break;
-        }
-        case 3: raise_u64(&sc->cond_fa, max_of(2)); break;
-        case 4: raise_u64(&sc->cond_fu, max_of(3)); break;
-        case 5: raise_u64(&sc->cond_a, max_of(4)); break;
+        case 2: raise_u64(&sc->cond_fa, max_of(2)); break;
+        case 3: raise_u64(&sc->cond_fu, max_of(3)); break;
+        case 4: raise_u64(&sc->cond_a, max_of(4)); break;
         default: raise_u64(&sc->cond_du, max_of(5)); break;
         }
     }
