@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(128, 8) k_omega_compact_quads(RowSpace rs, Mix
 // consecutive ranks, share a line of the warp-wide gathers.  What bounds it now is the L1
 // data pipe (75 % of its wavefronts, issue slots 61 %; a thread per row: 50 % and 36 %,
 // waiting on its gathers).  Per launch, with the corrector pass below: 1,048,576 particles
-// of the jittered lattice 734 -> 440 + 54 us, disc of 1,000,003 1440 -> 457 + 52 us,
+// of the jittered lattice 734 -> 440 + 54 us, disc of 1,000,003 1440 -> 457 + 55 us,
 // homogeneous box of 8.5 M 5.96 -> 3.36 + 0.45 ms.
 struct PairTerms {
     float f, x, y, z, u; // force / r, separation, du/dt term
