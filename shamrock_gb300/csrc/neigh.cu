@@ -405,12 +405,14 @@ __global__ void __launch_bounds__(128) k_leaf_lists_wide(TreeView t, const NodeB
 }
 
 // what a cache build accumulates into: no owned row, no threshold, no flag, no entry
-__global__ void k_cache_init(u32 L, u32 *__restrict__ head, u32 *__restrict__ leaf_thr, Scalars *sc) {
+__global__ void k_cache_init(u32 L, u32 *__restrict__ leaf_rows, u32 *__restrict__ head, u32 *__restrict__ leaf_thr, Scalars *sc) {
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l == 0) sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = 0, sc->csr_entries = sc->csr_kept = 0;
+    if (l == 0)
+        sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = sc->rows_over = 0, sc->csr_entries = sc->csr_kept = 0;
     if (l >= L) return;
-    head[l]     = kNone;
-    leaf_thr[l] = 0;
+    leaf_rows[l] = 0;
+    head[l]      = kNone;
+    leaf_thr[l]  = 0;
 }
 
 // ---- rows: local particles in rank order
@@ -429,11 +431,16 @@ struct RowPlace {
     __device__ __forceinline__ void end(u32) const {}
 };
 
+constexpr u32 kLeafRows    = 32;                // linked rows of a leaf
+constexpr u32 kLinkedEntry = kNone - kLeafRows; // beyond every row
+
 // ---- owner leaf: max leaf index whose box contains the point (inclusive bounds),
 // i.e. the last leaf the reference's left-first DFS reports (NeighbourCache.cpp:419-443).
 // Right-first traversal over the child-pair records (the first leaf reached is the
 // largest); containment is decided in FP32 outside a rounding band, else in FP64.
-// The rows of a leaf are linked: head[leaf], then next_row[row] (their order does not matter).
+// The first 32 rows of a leaf are linked: head[leaf], then next_row[row] (their order does not
+// matter).  Where it owns more, all of its rows are in the list `over` of {row, leaf}, the k-th
+// linked one as {kLinkedEntry + k, leaf}: 32 rows are the most that stage 2 leaves to one warp.
 // leaf_thr: per leaf, the FP32 bits (rounded up) of the largest pair-test
 // threshold thr_a = ((h_a htol)^2) R^2 over the rows it owns, 0 for a leaf owning none.
 // The exact containment test inside the FP32 band compares the doubles' ordered bit
@@ -443,8 +450,9 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
                                                const NodePairF *__restrict__ rec,
                                                const u32 *__restrict__ row_rank, u32 n_rows,
                                                const f64 *__restrict__ sx, const f64 *__restrict__ sy,
-                                               const f64 *__restrict__ sz, u32 *__restrict__ head,
-                                               u32 *__restrict__ next_row, u32 *__restrict__ flags, const f64 *__restrict__ sh,
+                                               const f64 *__restrict__ sz, u32 *__restrict__ leaf_rows,
+                                               u32 *__restrict__ head, u32 *__restrict__ next_row, uint2 *__restrict__ over,
+                                               Scalars *sc, const f64 *__restrict__ sh,
                                                float h_tol_up, u32 *__restrict__ leaf_thr) {
     u32 row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n_rows) return;
@@ -484,14 +492,14 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         const u32 li = __float_as_uint(bl.b.w), ri = __float_as_uint(br.b.w);
         const bool cl = inside(li, bl.a, bl.b), cr = inside(ri, br.a, br.b);
         if (top + 2 > kStack) {
-            atomicOr(flags, kFlagStackOverflow);
+            atomicOr(&sc->flags, kFlagStackOverflow);
             break;
         }
         if (cl) stack[top++] = li;
         if (cr) stack[top++] = ri;
     }
     if (found == kNone) {
-        atomicOr(flags, kFlagOwnerMissing); // the build stops at its next sync
+        atomicOr(&sc->flags, kFlagOwnerMissing); // the build stops at its next sync
         found = 0;
     } else {
         // an FP32 upper bound of thr_a = fl64(fl64(h htol)^2 R^2): every factor rounded up
@@ -500,7 +508,15 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         const float thr  = __fmul_ru(__fmul_ru(rint, rint), (float) (kRkern * kRkern));
         atomicMax(&leaf_thr[found], __float_as_uint(thr));
     }
-    next_row[row] = atomicExch(&head[found], row);
+    const u32 at = atomicAdd(&leaf_rows[found], 1u);
+    if (at < kLeafRows) {
+        next_row[row] = atomicExch(&head[found], row);
+        return;
+    }
+    u32 e = atomicAdd(&sc->rows_over, at == kLeafRows ? kLeafRows + 1 : 1u);
+    if (at == kLeafRows)
+        for (u32 k = 0; k < kLeafRows; k++) over[e++] = make_uint2(kLinkedEntry + k, found);
+    over[e] = make_uint2(row, found);
 }
 
 // ---- stage 2 (NeighbourCache.cpp:492-591)
@@ -515,8 +531,8 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // position records; outside a +-1e-5 relative band the answer is certain, inside it the
 // exact FP64 test decides, so the cache is the FP64 one.
 //
-// A warp walks one leaf: the rows that the leaf owns share its candidates, so the warp
-// expands the leaf's rank runs once, loads each candidate's record once, coalesced, drops
+// A warp walks one leaf that owns up to 32 rows (k_part_rows takes those of more): the rows that
+// the leaf owns share its candidates, so the warp expands the leaf's rank runs once, loads each candidate's record once, coalesced, drops
 // those out of reach of the rows' box and keeps the others' positions relative to the leaf in
 // shared memory; a row is then tested against 64 of them at a time and the accepted lanes are
 // placed by ballots, in rank order.  Bound by instruction issue (76 % of the peak at 25 a row
@@ -561,11 +577,22 @@ __device__ __forceinline__ float warp_min(float v) {
     return __uint_as_float(m ^ ((m >> 31) ? 0x80000000u : 0xffffffffu));
 }
 
+// the largest row of the build (sizes the slots of the next one) and the entries
+template<int MODE>
+__device__ __forceinline__ void cache_totals(u32 c_max, u64 c_sum, Scalars *sc) {
+    u64 mx = block_reduce((u64) c_max, OpMaxU64{}, 0ull);
+    if (threadIdx.x == 0 && mx) raise_u32(&sc->row_cnt_max, (u32) mx);
+    if (MODE != kCount) {
+        u64 tot = block_reduce(c_sum, OpAddU64{}, 0ull);
+        if (threadIdx.x == 0) atomicAdd((unsigned long long *) &sc->csr_entries, (unsigned long long) tot);
+    }
+}
+
 constexpr u32 kCandBlock = 256; // candidates of a leaf held at a time
 
 template<int MODE>
 __global__ void __launch_bounds__(256, 4) k_part_cache(
-    u32 L, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
+    u32 L, const u32 *__restrict__ leaf_rows, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
     const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
     const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
     const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
@@ -582,7 +609,7 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
     u32 c_max = 0;
     u64 c_sum = 0;
     for (u32 l = blockIdx.x * 8 + wid; l < L; l += gridDim.x * 8) {
-        u32 cur      = head[l];
+        u32 cur      = leaf_rows[l] <= kLeafRows ? head[l] : kNone;
         const u32 k0 = leaf_off[l], nk = min(leaf_cnt[l], leaf_cap); // (an overflowing list is rebuilt)
         while (cur != kNone) {
             // the next 32 rows at most, a lane each
@@ -711,15 +738,73 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
             }
         }
     }
-    // the largest row of the build (sizes the slots of the next one)
-    {
-        u64 mx = block_reduce((u64) c_max, OpMaxU64{}, 0ull);
-        if (threadIdx.x == 0 && mx) raise_u32(&sc->row_cnt_max, (u32) mx);
+    cache_totals<MODE>(c_max, c_sum, sc);
+}
+
+// The rows of leaves that own more than 32, as of a clump within one Morton cell: a warp per
+// row, the candidates 32 at a time from their records, whose hi/lo differences need no common
+// origin.  With a warp per leaf whatever its rows, 20,000 particles in one cell took 8.8 s and a
+// profile r ~ u^3 of 300,000 36 s; a thread per row 5.0 and 15 ms, this 0.74 and 8.4 ms.
+// The line at 32 rows: a condensed profile r ~ u^2 of 200,000 takes 3.8 ms of cache builds a step
+// there, 5.0 at 64 and 6.6 at 128, and no state measured is faster with more.
+template<int MODE>
+__global__ void __launch_bounds__(256) k_part_rows(
+    const uint2 *__restrict__ over, u32 n_over, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
+    const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
+    const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
+    const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
+    const f64 *__restrict__ sz, const f64 *__restrict__ sh, f64 h_tol, u32 *__restrict__ cnt,
+    u32 *__restrict__ off, u32 *__restrict__ ent, Scalars *sc, u32 cap, u32 leaf_cap) {
+    const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    constexpr u32 kAll = 0xffffffffu;
+    const float lo_f = 1.f - 1e-5f, hi_f = 1.f + 1e-5f;
+    u32 c_max = 0;
+    u64 c_sum = 0;
+    for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n_over; i += gridDim.x * 8) {
+        const uint2 e  = over[i];
+        u32 row        = e.x;
+        if (row >= kLinkedEntry) {
+            row = head[e.y];
+            for (u32 k = kLinkedEntry; k < e.x; k++) row = next_row[row];
+        }
+        const u32 k0   = leaf_off[e.y], nk = min(leaf_cnt[e.y], leaf_cap); // (an overflowing list is rebuilt)
+        const u32 ra   = row_rank[row];
+        const F8 a     = ldg256(&P[2 * (size_t) ra]);
+        const float M  = fmaxf(fmaxf(fabsf(a.a.x), fabsf(a.a.y)), fabsf(a.a.z));
+        // the hi/lo records' error stays inside the band, or every candidate is decided in FP64
+        const float ta = M * M <= 1e16f * a.b.w && a.b.w > 1e-30f ? a.b.w : __int_as_float(0x7fc00000);
+        const u32 w    = (MODE == kFill) ? off[row] : ((MODE == kOnePass) ? row * cap : 0);
+        u32 c          = 0;
+        for (u32 k = 0; k < nk; k++) {
+            const uint2 run = leaf_ent[k0 + k];
+            for (u32 b0 = run.x; b0 < run.y; b0 += 32) {
+                const u32 b = b0 + lane;
+                bool in = false;
+                if (b < run.y) {
+                    const F8 q     = ldg256(&P[2 * (size_t) b]);
+                    const float dx = __fadd_rn(__fsub_rn(a.a.x, q.a.x), __fsub_rn(a.b.x, q.b.x));
+                    const float dy = __fadd_rn(__fsub_rn(a.a.y, q.a.y), __fsub_rn(a.b.y, q.b.y));
+                    const float dz = __fadd_rn(__fsub_rn(a.a.z, q.a.z), __fsub_rn(a.b.z, q.b.z));
+                    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)), tm = max_nan(ta, q.b.w);
+                    in = r2 < tm * lo_f || (!(r2 > tm * hi_f) && pair_inside(sx, sy, sz, sh, h_tol, ra, b));
+                }
+                const u32 bits = __ballot_sync(kAll, in), at = c + __popc(bits & below);
+                c += __popc(bits);
+                if (MODE != kCount && in && (MODE == kFill || at < cap)) ent[w + at] = b;
+            }
+        }
+        if (lane == 0) {
+            if (MODE != kFill) cnt[row] = c;
+            if (MODE == kCount) off[row] = (c + 3u) & ~3u;
+            if (MODE == kOnePass) {
+                off[row] = w;
+                if (c > cap) atomicOr(&sc->flags, kFlagCsrCap);
+            }
+            c_max = max(c_max, c);
+            c_sum += c;
+        }
     }
-    if (MODE != kCount) {
-        u64 tot = block_reduce(c_sum, OpAddU64{}, 0ull);
-        if (threadIdx.x == 0) atomicAdd((unsigned long long *) &sc->csr_entries, (unsigned long long) tot);
-    }
+    cache_totals<MODE>(c_max, c_sum, sc);
 }
 
 // ---- generic object query (CLBVHObjectIterator::rtree_for, CLBVHObjectIterator.hpp:127-169)
@@ -834,16 +919,19 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // Owner leaves first: they also record, per leaf, the largest threshold of the rows
     // it owns, which lets stage 1 drop leaves that no owned row can pair with (and skip
     // leaves that own no row); the cache is unchanged.
-    if ((e = c.next_row.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
+    if ((e = c.leaf_rows.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = c.leaf_head.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
+    if ((e = c.next_row.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
+    // at most every row, once
+    if ((e = c.rows_over.ensure(sizeof(uint2) * (size_t) n, s)) != cudaSuccess) return e;
     if ((e = c.leaf_thr.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     u32 *leaf_thr = c.leaf_thr.as<u32>();
-    { k_cache_init<<<div_up(L, 256), 256, 0, s>>>(L, c.leaf_head.as<u32>(), leaf_thr, dsc); GBSPH_COUNTED; }
+    { k_cache_init<<<div_up(L, 256), 256, 0, s>>>(L, c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), leaf_thr, dsc); GBSPH_COUNTED; }
     if (n) {
         ProfScope ps(c, kProfOwner, n);
         { k_owner<<<div_up(n, 128), 128, 0, s>>>(t, fb, rec, c.row_rank.as<u32>(), n, c.sx.as<f64>(),
-                                               c.sy.as<f64>(), c.sz.as<f64>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(),
-                                               &dsc->flags, c.sh.as<f64>(), up_f32(h_tol), leaf_thr); GBSPH_COUNTED; }
+                                               c.sy.as<f64>(), c.sz.as<f64>(), c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(),
+                                               c.rows_over.as<uint2>(), dsc, c.sh.as<f64>(), up_f32(h_tol), leaf_thr); GBSPH_COUNTED; }
     }
     auto stage1 = [&]() -> cudaError_t {
         cudaError_t err = c.leaf_ent.ensure(sizeof(uint2) * ((size_t) L * c.leaf_cap + 1), s);
@@ -885,13 +973,23 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics
     // on the totals, 10 ns each, take longer than the build)
     u32 leaf_slots = c.leaf_cap; // no bound for the lists of the exact stage 1
+    u32 n_over     = 0;          // rows of leaves that own more than 32, known after a sync
+    auto part_rows = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
+        constexpr int MODE = decltype(mode_tag)::value;
+        if (n_over == 0) return;
+        { k_part_rows<MODE><<<std::min(div_up(n_over, 8), 24 * c.sms), 256, 0, s>>>(
+            c.rows_over.as<uint2>(), n_over, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
+            c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
+            c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
+    };
     auto part = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
         const u32 blocks   = std::min(div_up(L, 8), 24 * c.sms);
         { k_part_cache<MODE><<<blocks, 256, 0, s>>>(
-            L, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
+            L, c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
             c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
+        part_rows(mode_tag, cnt, off, ent);
     };
     using OnePass = std::integral_constant<int, kOnePass>;
     using Count   = std::integral_constant<int, kCount>;
@@ -911,6 +1009,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         return cudaErrorUnknown;
     }
     c.leaf_csr_total = 0;
+    n_over           = c.h_scalars->rows_over;
     if (c.h_scalars->flags & kFlagLeafCap) {
         const u32 cap = (c.h_scalars->leaf_cnt_max + 31u) & ~31u;
         const bool fits = s1_one_pass && slots_ok(L, cap, sizeof(uint2));
@@ -936,6 +1035,10 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         }
         // stage 2 ran over cut lists, or not at all
         if ((e = stage2()) != cudaSuccess) return e;
+        if ((e = sync_scalars(c)) != cudaSuccess) return e;
+    } else if (n_over && one_pass) {
+        ProfScope ps(c, kProfCacheFill, 0);
+        part_rows(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
     }
     c.csr_total = c.h_scalars->csr_entries;
