@@ -547,9 +547,10 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // largest relative coordinate, a separation errs by u (4 S + 3 |d|) an axis, so r^2 of a pair
 // near the threshold by u (8 sqrt(3) S / sqrt(thr) + 9) relative, and by 2.5e-14 M / sqrt(thr)
 // for the hi/lo records of coordinates of size M; the threshold's own roundings add 3 u.  A row
-// with S <= 6 sqrt(thr) and M <= 1e8 sqrt(thr) stays below 8.2e-6, inside the band; any other
+// with S <= 10 sqrt(thr) and M <= 1e7 sqrt(thr) stays below 9.3e-6, inside the band; any other
 // takes the FP64 test for every candidate.  (An ordinary leaf is a few h wide, S about
-// sqrt(thr).)
+// sqrt(thr); with the line at 6 the builds of a thin sheet of 100,000, whose leaves span more,
+// took twice as long, 0.68 against 0.34 ms a step.)
 enum CacheMode { kCount = 0, kFill = 1, kOnePass = 2 };
 
 // the exact test (NeighbourCache.cpp:492-591); a call, as few candidates need it
@@ -636,8 +637,8 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
                 const float mine = lane < m ? fmaxf(fmaxf(fabsf(xa), fabsf(ya)), fabsf(za)) : 0.f;
                 const float S    = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(mine)));
                 const float M    = fmaxf(fmaxf(fabsf(Ph.x), fabsf(Ph.y)), fabsf(Ph.z));
-                // S / sqrt(thr) <= 6 and M / sqrt(thr) <= 1e8
-                const bool ok = S * S <= 36.f * thr && M * M <= 1e16f * thr && thr > 1e-30f;
+                // S / sqrt(thr) <= 10 and M / sqrt(thr) <= 1e7
+                const bool ok = S * S <= 100.f * thr && M * M <= 1e14f * thr && thr > 1e-30f;
                 tlo           = ok ? thr * lo_f : __int_as_float(0x7fc00000);
                 tmax          = __uint_as_float(__reduce_max_sync(kAll, lane < m && ok ? __float_as_uint(tlo) : 0u));
                 if (__any_sync(kAll, lane < m && !ok)) tmax = __int_as_float(0x7fc00000);
