@@ -626,13 +626,14 @@ static f64 err_estimate(u64 sum_bits, u64 max_bits) {
 }
 
 // Whether Omega is taken while the host waits for the h iteration's result, which it does not
-// need.  Ahead of the wait it saves 3 us a step (2,048 Sedov particles 447 -> 444 us, 37,044
-// 591 -> 588) and nothing from 131,072 on (988 against 986, 1,048,576 3805 against 3808); where
-// h then takes another sub-cycle, the pass was for nothing: 10 to 21 us for so few rows, 58 at
-// 131,072, and 207 to 498 in FP64.  So only for few rows, and only after a step whose h took one
-// sub-cycle (which can cost time here and nothing else: Omega is the last h's either way).
+// need.  Ahead of the wait it saves 3 to 5 us a step (2,048 Sedov particles 447 -> 444 us, a disc
+// of 42,578 584 -> 580 and of 100,003 815 -> 810), 2 at 131,072 of 990 and nothing at 1,048,576;
+// where h then takes another sub-cycle, the pass was for nothing: 10 us for 2,048 rows, 58 at
+// 131,072, 385 at 1,048,576, and 207 to 498 in FP64.  So up to about 155,000 rows, and only after
+// a step whose h took one sub-cycle (which can cost time here and nothing else: Omega is the
+// last h's either way).
 static bool omega_ahead(const Ctx &c, u32 n, u32 tier) {
-    return tier == GBSPH_MIXED && c.one_subcycle && quad_rows(c, n);
+    return tier == GBSPH_MIXED && c.one_subcycle && n <= 1024 * c.sms;
 }
 
 // One step (Solver::evolve_once) in one precision tier (GBSPH_FP64, GBSPH_MIXED or

@@ -1087,6 +1087,13 @@ cudaError_t stage_positions_mixed(Ctx &c, u32 N, f64 h_tol) {
     return cudaGetLastError();
 }
 
+// Four lanes per row while a thread per row leaves an SM less than one block of 256: the
+// passes are then bound by the latency of each row's chain of loads.  With more rows the
+// thread per row wins, as 32 neighbouring rows gather from the same lines and the quads
+// repeat the additions: h iteration / Omega of a disc of 100,003 85 / 49 us against 93 / 47,
+// 131,072 Sedov 77 / 59 against 66 / 62, 1,048,576 319 / 383 against 422 / 467.
+static bool quad_rows(const Ctx &c, u32 n) { return n <= 256 * c.sms; }
+
 cudaError_t h_iterate_mixed(Ctx &c, const RowSpace &rs, const f64 *h_old, f64 *h_new, f64 *eps,
                             f64 pmass, f64 h_evol_max, f64 h_evol_iter_max, u32 iters, f64 eps_p) {
     ProfScope ps(c, kProfHIter, rs.n);

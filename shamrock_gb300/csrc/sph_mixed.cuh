@@ -1,7 +1,6 @@
 // Mixed-precision (FP32 pair arithmetic) variants of the SPH pair kernels.
 #pragma once
 
-#include "gbsph_ctx.cuh"
 #include "sph_kernels.cuh"
 
 namespace gbsph {
@@ -21,13 +20,6 @@ struct MixedSpace {
     const float4 *P; // 2 per particle
     const float4 *H; // 2 per particle
 };
-
-// Four lanes per row while a thread per row leaves an SM less than one block of 256: the
-// passes are then bound by the latency of each row's chain of loads.  With more rows the
-// thread per row wins, as 32 neighbouring rows gather from the same lines and the quads
-// repeat the additions: h iteration / Omega of a disc of 100,003 85 / 49 us against 93 / 47,
-// 131,072 Sedov 77 / 59 against 66 / 62, 1,048,576 319 / 383 against 422 / 467.
-inline bool quad_rows(const Ctx &c, u32 n) { return n <= 256 * c.sms; }
 
 cudaError_t stage_positions_mixed(Ctx &c, u32 N, f64 h_tol);
 // the position records staged by stage_positions_mixed (B.w = fl32 cache threshold)

@@ -13,11 +13,11 @@ def _omega_passes(ctx):
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("fused", [True, False])
-@pytest.mark.parametrize("cells", [8, 22])
+@pytest.mark.parametrize("cells", [8, 35])
 def test_one_omega_pass_per_step(precision, fused, cells):
     """A first step of several sub-cycles (h started at half its size), a step of one, and a
-    step of several after it, which may have taken Omega ahead once: up to 256 rows an SM
-    (2,048 rows) and beyond (42,592)."""
+    step of several after it, which may have taken Omega ahead once: up to 1,024 rows an SM
+    (2,048 rows) and beyond (171,500)."""
     from shamrock_gb300 import setups
 
     s = setups.sedov_taylor(cells, jitter=0.05, seed=3)
