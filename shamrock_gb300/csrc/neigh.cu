@@ -441,6 +441,7 @@ constexpr u32 kLinkedEntry = kNone - kLeafRows; // beyond every row
 // The first 32 rows of a leaf are linked: head[leaf], then next_row[row] (their order does not
 // matter).  Where it owns more, all of its rows are in the list `over` of {row, leaf}, the k-th
 // linked one as {kLinkedEntry + k, leaf}: 32 rows are the most that stage 2 leaves to one warp.
+// Rows whose pair radius is less than a twentieth of the leaf's width are in that list at once.
 // leaf_thr: per leaf, the FP32 bits (rounded up) of the largest pair-test
 // threshold thr_a = ((h_a htol)^2) R^2 over the rows it owns, 0 for a leaf owning none.
 // The exact containment test inside the FP32 band compares the doubles' ordered bit
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         if (cl) stack[top++] = li;
         if (cr) stack[top++] = ri;
     }
+    bool wide = false; // the leaf is wide for this row (see stage 2)
     if (found == kNone) {
         atomicOr(&sc->flags, kFlagOwnerMissing); // the build stops at its next sync
         found = 0;
@@ -507,6 +509,13 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         const float rint = __fmul_ru(__double2float_ru(sh[r]), h_tol_up);
         const float thr  = __fmul_ru(__fmul_ru(rint, rint), (float) (kRkern * kRkern));
         atomicMax(&leaf_thr[found], __float_as_uint(thr));
+        const F8 lb     = ldg256(&fb[offn + found]);
+        const float ext = fmaxf(fmaxf(lb.b.x - lb.a.x, lb.b.y - lb.a.y), lb.b.z - lb.a.z);
+        wide            = ext * ext > 400.f * thr;
+    }
+    if (wide) {
+        over[atomicAdd(&sc->rows_over, 1u)] = make_uint2(row, found);
+        return;
     }
     const u32 at = atomicAdd(&leaf_rows[found], 1u);
     if (at < kLeafRows) {
@@ -549,8 +558,11 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // for the hi/lo records of coordinates of size M; the threshold's own roundings add 3 u.  A row
 // with S <= 10 sqrt(thr) and M <= 1e7 sqrt(thr) stays below 9.3e-6, inside the band; any other
 // takes the FP64 test for every candidate.  (An ordinary leaf is a few h wide, S about
-// sqrt(thr); with the line at 6 the builds of a thin sheet of 100,000, whose leaves span more,
-// took twice as long, 0.68 against 0.34 ms a step.)
+// sqrt(thr); rows for which it is wider than 20 sqrt(thr) are left to k_part_rows.  With the
+// FP64 test for those too, the cache of a line of 300,000 in leaves of 64 cells took 33 ms
+// instead of 6.9.  In between few rows fail: with S <= 6 sqrt(thr) here the builds of a thin
+// sheet of 100,000 took 0.68 instead of 0.34 ms a step, with 10 sqrt(thr) in the owner search
+// 0.53.)
 enum CacheMode { kCount = 0, kFill = 1, kOnePass = 2 };
 
 // the exact test (NeighbourCache.cpp:492-591); a call, as few candidates need it
@@ -742,15 +754,15 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
     cache_totals<MODE>(c_max, c_sum, sc);
 }
 
-// The rows of leaves that own more than 32, as of a clump within one Morton cell: a warp per
-// row, the candidates 32 at a time from their records, whose hi/lo differences need no common
+// The rows of leaves that own more than 32, as of a clump within one Morton cell, or that are
+// wide for them: a warp per row, the candidates 32 at a time from their records, whose hi/lo differences need no common
 // origin.  With a warp per leaf whatever its rows, 20,000 particles in one cell took 8.8 s and a
 // profile r ~ u^3 of 300,000 36 s; a thread per row 5.0 and 15 ms, this 0.74 and 8.4 ms.
 // The line at 32 rows: a condensed profile r ~ u^2 of 200,000 takes 3.8 ms of cache builds a step
 // there, 5.0 at 64 and 6.6 at 128, and no state measured is faster with more.
 template<int MODE>
 __global__ void __launch_bounds__(256) k_part_rows(
-    const uint2 *__restrict__ over, u32 n_over, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
+    const uint2 *__restrict__ over, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
     const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
     const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
     const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
@@ -759,6 +771,7 @@ __global__ void __launch_bounds__(256) k_part_rows(
     const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     constexpr u32 kAll = 0xffffffffu;
     const float lo_f = 1.f - 1e-5f, hi_f = 1.f + 1e-5f;
+    const u32 n_over = sc->rows_over;
     u32 c_max = 0;
     u64 c_sum = 0;
     for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n_over; i += gridDim.x * 8) {
@@ -974,12 +987,10 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     // uneven work leaves a tail of 10 %, with a block per eight leaves the blocks' atomics
     // on the totals, 10 ns each, take longer than the build)
     u32 leaf_slots = c.leaf_cap; // no bound for the lists of the exact stage 1
-    u32 n_over     = 0;          // rows of leaves that own more than 32, known after a sync
     auto part_rows = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
-        if (n_over == 0) return;
-        { k_part_rows<MODE><<<std::min(div_up(n_over, 8), 24 * c.sms), 256, 0, s>>>(
-            c.rows_over.as<uint2>(), n_over, c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
+        { k_part_rows<MODE><<<std::min(div_up(n, 8), 24 * c.sms), 256, 0, s>>>(
+            c.rows_over.as<uint2>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
             c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
     };
@@ -990,27 +1001,27 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
             L, c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
             c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
-        part_rows(mode_tag, cnt, off, ent);
     };
     using OnePass = std::integral_constant<int, kOnePass>;
     using Count   = std::integral_constant<int, kCount>;
     using Fill    = std::integral_constant<int, kFill>;
-    auto stage2 = [&]() -> cudaError_t {
+    // all: with the rows left to k_part_rows
+    auto stage2 = [&](bool all) -> cudaError_t {
         if (!n || !one_pass) return cudaSuccess;
         ProfScope ps(c, kProfCacheFill, n);
         part(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
+        if (all) part_rows(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
         return cudaGetLastError();
     };
     // Stage 2 follows at once: a list that overflowed its slots is read up to its slots only,
-    // and both stages run again.
-    if (s1_one_pass && (e = stage2()) != cudaSuccess) return e;
+    // and both stages run again.  Whether rows are left to k_part_rows is read with the flags.
+    if (s1_one_pass && (e = stage2(false)) != cudaSuccess) return e;
     if ((e = sync_scalars(c)) != cudaSuccess) return e;
     if (c.h_scalars->flags & (kFlagStackOverflow | kFlagOwnerMissing)) {
         c.err = "neighbour cache: tree traversal failed (stack overflow or particle outside every leaf box)";
         return cudaErrorUnknown;
     }
     c.leaf_csr_total = 0;
-    n_over           = c.h_scalars->rows_over;
     if (c.h_scalars->flags & kFlagLeafCap) {
         const u32 cap = (c.h_scalars->leaf_cnt_max + 31u) & ~31u;
         const bool fits = s1_one_pass && slots_ok(L, cap, sizeof(uint2));
@@ -1035,9 +1046,9 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
             { k_leaf_fill<<<div_up(L, 128), 128, 0, s>>>(t, c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>()); GBSPH_COUNTED; }
         }
         // stage 2 ran over cut lists, or not at all
-        if ((e = stage2()) != cudaSuccess) return e;
+        if ((e = stage2(true)) != cudaSuccess) return e;
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
-    } else if (n_over && one_pass) {
+    } else if (c.h_scalars->rows_over && one_pass) {
         ProfScope ps(c, kProfCacheFill, 0);
         part_rows(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
@@ -1054,6 +1065,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
             {
                 ProfScope ps(c, kProfCacheFill, n);
                 part(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
+                part_rows(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
             }
             if ((e = sync_scalars(c)) != cudaSuccess) return e;
             c.csr_total = c.h_scalars->csr_entries;
@@ -1066,6 +1078,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         {
             ProfScope ps(c, kProfCacheCount, n);
             part(Count{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), nullptr);
+            part_rows(Count{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), nullptr);
         }
         // rows padded to multiples of 4 entries, scanned in place
         if ((e = scan_exclusive_u32(c.csr_off.as<u32>(), c.csr_off.as<u32>(), n, &dsc->total,
@@ -1078,6 +1091,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         {
             ProfScope ps(c, kProfCacheFill, 0);
             part(Fill{}, nullptr, c.csr_off.as<u32>(), c.csr_ent.as<u32>());
+            part_rows(Fill{}, nullptr, c.csr_off.as<u32>(), c.csr_ent.as<u32>());
         }
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
         c.csr_total = c.h_scalars->csr_entries;

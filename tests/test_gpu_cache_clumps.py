@@ -48,6 +48,27 @@ def test_clumped_cache_vs_oracle(sizes, level, budget):
     ctx.close()
 
 
+@pytest.mark.parametrize("ratio", [3.0, 9.0, 11.0, 19.0, 21.0, 200.0])
+def test_rows_of_wide_leaves_vs_oracle(gctx, ratio):
+    """Leaves of two tight groups at opposite ends of a Morton cell, `ratio` pair radii apart."""
+    from shamrock_gb300 import modules as M
+
+    rng = np.random.default_rng(int(ratio))
+    ends = np.floor(1024 * (0.1 + 0.8 * rng.random((40, 3)))) / 1024
+    radius = 9e-4 / ratio
+    groups = [c + np.array([[e, 4e-4, 4e-4]]) + 0.8 * radius * rng.random((12, 3))
+              for c in ends for e in (1e-5, 9.5e-4 - radius)]
+    pos = np.concatenate(groups + [np.array([[0.0, 0, 0], [1, 1, 1]])])
+    h = np.full(len(pos), radius / 2.2) * rng.choice([1.0, 0.7], len(pos))
+    lo, hi = (0.0,) * 3, (np.nextafter(1.0, 2.0),) * 3
+    for level in (0, 4):
+        oc = O.Tree(pos, lo, hi, level, h=h, htol=1.1).neigh_cache(pos, h, len(pos), 1.1)
+        M.Tree(gctx, pos, lo, hi, level, h=h, htol=1.1)
+        csr = M.neighbour_cache(gctx, len(pos), 1.1, "mixed")
+        for key in ("cnt", "scanned", "entries"):
+            assert np.array_equal(csr[key].cpu().numpy().view(np.uint32), oc[key]), (level, key)
+
+
 def test_one_cell_is_the_work_of_many_warps(gctx):
     """20,000 particles of one cell (every row has them all as candidates): about 1 ms, and
     seconds where a leaf's rows are left to one warp."""
