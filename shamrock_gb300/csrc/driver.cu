@@ -69,7 +69,7 @@ Ctx::~Ctx() {
                       &offsets, &reduc, &reduced, &radix_k, &radix_v, &radix_hist, &radix_off, &lchild, &rchild, &lflag, &rflag, &endrange,
                       &parent, &boxes, &fboxes, &fpairs, &lboxes, &wboxes, &rank_of, &sx, &sy, &sz, &sh, &row_rank,
                       &row_local, &leaf_cnt, &leaf_off, &leaf_ent,
-                      &leaf_rows, &leaf_head, &next_row, &rows_over, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
+                      &leaf_rows, &leaf_head, &next_row, &owner, &leaf_thr, &csr_cnt, &csr_off, &csr_ent, &ghost_src, &ghost_oid,
                       &ghost_block_counts, &mx, &my, &mz, &mh, &d_ghost_offsets, &scs, &rec64,
                       &sh2, &f_pos, &f_anchor, &f_aux0, &f_aux1, &f_aux2, &f_comp, &f_sums, &guard_state,
                       &h_old_row, &eps_row, &omega_local, &a_old, &du_old, &hnew_row, &omega_row,

@@ -47,7 +47,7 @@ struct Scalars {
     u32 flags;         // error flags raised by kernels
     u32 leaf_cnt_max;  // largest stage-1 list among leaves that overflowed their slots
     u32 row_cnt_max;   // largest stage-2 row among rows that overflowed their slots
-    u32 rows_over;     // rows of leaves that own more than 32
+    u32 rows_left;     // 1: there are rows for k_part_rows
     u32 dup_keys;      // radix-sorted Morton keys had equal neighbours
     u32 ticket;        // last-block counter, zero between kernels
 };
@@ -166,8 +166,8 @@ struct Ctx {
     u32 row_seen = 0;              // largest stage-2 row of the last build
     u64 slot_budget = 0;            // bytes of one-pass slots allowed (0: library default)
     DevBuf leaf_cnt, leaf_off, leaf_ent; // stage 1 (rank ranges of candidate leaves)
-    DevBuf leaf_rows, leaf_head, next_row; // the rows each leaf owns: how many, the first 32 linked
-    DevBuf rows_over;                    // all rows of leaves that own more
+    DevBuf owner;                        // per row: its leaf
+    DevBuf leaf_rows, leaf_head, next_row; // the rows each leaf owns: how many, and linked
     DevBuf leaf_thr;                     // per leaf: FP32 bits of max thr over its owned rows
     DevBuf csr_cnt, csr_off, csr_ent;    // stage 2, per row, entries are ranks
     u32 n_local = 0;

@@ -405,10 +405,11 @@ __global__ void __launch_bounds__(128) k_leaf_lists_wide(TreeView t, const NodeB
 }
 
 // what a cache build accumulates into: no owned row, no threshold, no flag, no entry
-__global__ void k_cache_init(u32 L, u32 *__restrict__ leaf_rows, u32 *__restrict__ head, u32 *__restrict__ leaf_thr, Scalars *sc) {
+__global__ void k_cache_init(u32 L, u32 *__restrict__ leaf_rows, u32 *__restrict__ head,
+                             u32 *__restrict__ leaf_thr, Scalars *sc) {
     u32 l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l == 0)
-        sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = sc->rows_over = 0, sc->csr_entries = sc->csr_kept = 0;
+        sc->flags = sc->leaf_cnt_max = sc->row_cnt_max = sc->rows_left = 0, sc->csr_entries = sc->csr_kept = 0;
     if (l >= L) return;
     leaf_rows[l] = 0;
     head[l]      = kNone;
@@ -431,17 +432,16 @@ struct RowPlace {
     __device__ __forceinline__ void end(u32) const {}
 };
 
-constexpr u32 kLeafRows    = 32;                // linked rows of a leaf
-constexpr u32 kLinkedEntry = kNone - kLeafRows; // beyond every row
+constexpr u32 kLeafRows = 128;         // rows of a leaf that stage 2 leaves to one warp
+constexpr u32 kWideRow  = 0x80000000u; // beside the owner leaf: the leaf is wide for the row
 
 // ---- owner leaf: max leaf index whose box contains the point (inclusive bounds),
 // i.e. the last leaf the reference's left-first DFS reports (NeighbourCache.cpp:419-443).
 // Right-first traversal over the child-pair records (the first leaf reached is the
 // largest); containment is decided in FP32 outside a rounding band, else in FP64.
-// The first 32 rows of a leaf are linked: head[leaf], then next_row[row] (their order does not
-// matter).  Where it owns more, all of its rows are in the list `over` of {row, leaf}, the k-th
-// linked one as {kLinkedEntry + k, leaf}: 32 rows are the most that stage 2 leaves to one warp.
-// Rows whose pair radius is less than a twentieth of the leaf's width are in that list at once.
+// The rows of a leaf are linked up to kLeafRows: head[leaf], then next_row[row] (their order does
+// not matter).  Rows of leaves that own more, and rows whose pair radius is less than a
+// twentieth of the leaf's width, are left to k_part_rows, which finds them by their owner.
 // leaf_thr: per leaf, the FP32 bits (rounded up) of the largest pair-test
 // threshold thr_a = ((h_a htol)^2) R^2 over the rows it owns, 0 for a leaf owning none.
 // The exact containment test inside the FP32 band compares the doubles' ordered bit
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
                                                const u32 *__restrict__ row_rank, u32 n_rows,
                                                const f64 *__restrict__ sx, const f64 *__restrict__ sy,
                                                const f64 *__restrict__ sz, u32 *__restrict__ leaf_rows,
-                                               u32 *__restrict__ head, u32 *__restrict__ next_row, uint2 *__restrict__ over,
+                                               u32 *__restrict__ head, u32 *__restrict__ next_row, u32 *__restrict__ owner,
                                                Scalars *sc, const f64 *__restrict__ sh,
                                                float h_tol_up, u32 *__restrict__ leaf_thr) {
     u32 row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -513,19 +513,13 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
         const float ext = fmaxf(fmaxf(lb.b.x - lb.a.x, lb.b.y - lb.a.y), lb.b.z - lb.a.z);
         wide            = ext * ext > 400.f * thr;
     }
-    if (wide) {
-        over[atomicAdd(&sc->rows_over, 1u)] = make_uint2(row, found);
-        return;
+    owner[row] = wide ? found | kWideRow : found;
+    if (!wide) {
+        const u32 at = atomicAdd(&leaf_rows[found], 1u);
+        if (at < kLeafRows) next_row[row] = atomicExch(&head[found], row);
+        wide = at == kLeafRows;
     }
-    const u32 at = atomicAdd(&leaf_rows[found], 1u);
-    if (at < kLeafRows) {
-        next_row[row] = atomicExch(&head[found], row);
-        return;
-    }
-    u32 e = atomicAdd(&sc->rows_over, at == kLeafRows ? kLeafRows + 1 : 1u);
-    if (at == kLeafRows)
-        for (u32 k = 0; k < kLeafRows; k++) over[e++] = make_uint2(kLinkedEntry + k, found);
-    over[e] = make_uint2(row, found);
+    if (wide) sc->rows_left = 1;
 }
 
 // ---- stage 2 (NeighbourCache.cpp:492-591)
@@ -540,9 +534,10 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // position records; outside a +-1e-5 relative band the answer is certain, inside it the
 // exact FP64 test decides, so the cache is the FP64 one.
 //
-// A warp walks one leaf that owns up to 32 rows (k_part_rows takes those of more): the rows that
-// the leaf owns share its candidates, so the warp expands the leaf's rank runs once, loads each candidate's record once, coalesced, drops
-// those out of reach of the rows' box and keeps the others' positions relative to the leaf in
+// A warp walks one leaf that owns up to kLeafRows rows (k_part_rows takes those of more): they
+// share the leaf's candidates, so the warp expands the leaf's rank runs once, loads each
+// candidate's record once, coalesced, drops those out of reach of the rows' box and keeps the
+// others' positions relative to the leaf in
 // shared memory; a row is then tested against 64 of them at a time and the accepted lanes are
 // placed by ballots, in rank order.  Bound by instruction issue (76 % of the peak at 25 a row
 // and 32 candidates).  131,072 / 1,048,576 / homogeneous 8.5 M / clustered 3 M / disc 1 M:
@@ -560,7 +555,7 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 // takes the FP64 test for every candidate.  (An ordinary leaf is a few h wide, S about
 // sqrt(thr); rows for which it is wider than 20 sqrt(thr) are left to k_part_rows.  With the
 // FP64 test for those too, the cache of a line of 300,000 in leaves of 64 cells took 33 ms
-// instead of 6.9.  In between few rows fail: with S <= 6 sqrt(thr) here the builds of a thin
+// instead of 8.2.  In between few rows fail: with S <= 6 sqrt(thr) here the builds of a thin
 // sheet of 100,000 took 0.68 instead of 0.34 ms a step, with 10 sqrt(thr) in the owner search
 // 0.53.)
 enum CacheMode { kCount = 0, kFill = 1, kOnePass = 2 };
@@ -754,68 +749,98 @@ __global__ void __launch_bounds__(256, 4) k_part_cache(
     cache_totals<MODE>(c_max, c_sum, sc);
 }
 
-// The rows of leaves that own more than 32, as of a clump within one Morton cell, or that are
-// wide for them: a warp per row, the candidates 32 at a time from their records, whose hi/lo differences need no common
-// origin.  With a warp per leaf whatever its rows, 20,000 particles in one cell took 8.8 s and a
-// profile r ~ u^3 of 300,000 36 s; a thread per row 5.0 and 15 ms, this 0.74 and 8.4 ms.
-// The line at 32 rows: a condensed profile r ~ u^2 of 200,000 takes 3.8 ms of cache builds a step
-// there, 5.0 at 64 and 6.6 at 128, and no state measured is faster with more.
+// The rows of leaves that own more than kLeafRows, as of a clump within one Morton cell, or that
+// are wide for them: two rows a warp, the candidates 32 at a time from their records, whose
+// hi/lo differences need no common origin.  Caches of 20,000 particles of one cell / of condensed
+// profiles r ~ u^2 and r ~ u^3 of 200,000 / of a line of 300,000 in leaves of 64 cells, in ms:
+//   a thread per row                       5.2  /   4.7 /    9.9 /   32
+//   a warp per leaf whatever its rows   8750    / 253   / 5610   / 2310
+//   these rows two (one, four) a warp      0.88 (1.06, 1.19) / 1.9 (2.0, 1.9) / 3.8 (3.9, 4.0) / 8.2 (8.9, 8.6)
+// A row here costs about twice the instructions of one above, so the line lies where a leaf's
+// warp would make a tail: with it at 32 rows a lattice of 300,000 in leaves of 64 cells takes
+// 0.91 instead of 0.44 ms, at 256 the profiles 2.0 and 5.2.
+constexpr u32 kRowsAWarp = 2;
+
 template<int MODE>
 __global__ void __launch_bounds__(256) k_part_rows(
-    const uint2 *__restrict__ over, const u32 *__restrict__ head, const u32 *__restrict__ next_row,
+    const u32 *__restrict__ owner, const u32 *__restrict__ leaf_rows, u32 n_rows,
     const u32 *__restrict__ row_rank, const u32 *__restrict__ leaf_cnt,
     const u32 *__restrict__ leaf_off, const uint2 *__restrict__ leaf_ent,
     const float4 *__restrict__ P, const f64 *__restrict__ sx, const f64 *__restrict__ sy,
     const f64 *__restrict__ sz, const f64 *__restrict__ sh, f64 h_tol, u32 *__restrict__ cnt,
     u32 *__restrict__ off, u32 *__restrict__ ent, Scalars *sc, u32 cap, u32 leaf_cap) {
     const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-    constexpr u32 kAll = 0xffffffffu;
+    constexpr u32 kAll = 0xffffffffu, R = kRowsAWarp;
     const float lo_f = 1.f - 1e-5f, hi_f = 1.f + 1e-5f;
-    const u32 n_over = sc->rows_over;
     u32 c_max = 0;
     u64 c_sum = 0;
-    for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n_over; i += gridDim.x * 8) {
-        const uint2 e  = over[i];
-        u32 row        = e.x;
-        if (row >= kLinkedEntry) {
-            row = head[e.y];
-            for (u32 k = kLinkedEntry; k < e.x; k++) row = next_row[row];
-        }
-        const u32 k0   = leaf_off[e.y], nk = min(leaf_cnt[e.y], leaf_cap); // (an overflowing list is rebuilt)
-        const u32 ra   = row_rank[row];
-        const F8 a     = ldg256(&P[2 * (size_t) ra]);
-        const float M  = fmaxf(fmaxf(fabsf(a.a.x), fabsf(a.a.y)), fabsf(a.a.z));
-        // the hi/lo records' error stays inside the band, or every candidate is decided in FP64
-        const float ta = M * M <= 1e16f * a.b.w && a.b.w > 1e-30f ? a.b.w : __int_as_float(0x7fc00000);
-        const u32 w    = (MODE == kFill) ? off[row] : ((MODE == kOnePass) ? row * cap : 0);
-        u32 c          = 0;
-        for (u32 k = 0; k < nk; k++) {
-            const uint2 run = leaf_ent[k0 + k];
-            for (u32 b0 = run.x; b0 < run.y; b0 += 32) {
-                const u32 b = b0 + lane;
-                bool in = false;
-                if (b < run.y) {
-                    const F8 q     = ldg256(&P[2 * (size_t) b]);
-                    const float dx = __fadd_rn(__fsub_rn(a.a.x, q.a.x), __fsub_rn(a.b.x, q.b.x));
-                    const float dy = __fadd_rn(__fsub_rn(a.a.y, q.a.y), __fsub_rn(a.b.y, q.b.y));
-                    const float dz = __fadd_rn(__fsub_rn(a.a.z, q.a.z), __fsub_rn(a.b.z, q.b.z));
-                    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)), tm = max_nan(ta, q.b.w);
-                    in = r2 < tm * lo_f || (!(r2 > tm * hi_f) && pair_inside(sx, sy, sz, sh, h_tol, ra, b));
+    for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < (n_rows + R - 1) / R; i += gridDim.x * 8) {
+        const u32 row = R * i + lane;
+        const u32 o   = lane < R && row < n_rows ? owner[row] : kNone, leaf = o & ~kWideRow;
+        u32 left = __ballot_sync(kAll, o != kNone && ((o & kWideRow) || leaf_rows[leaf] > kLeafRows));
+        while (left) {
+            // those of one leaf, lane j the j-th row
+            const u32 l    = __shfl_sync(kAll, leaf, __ffs(left) - 1);
+            const u32 rows = __ballot_sync(kAll, leaf == l) & left;
+            const bool mine = rows >> lane & 1u;
+            left &= ~rows;
+            const u32 k0 = leaf_off[l], nk = min(leaf_cnt[l], leaf_cap); // (an overflowing list is rebuilt)
+            u32 ra = 0, w = 0;
+            F8 own{};
+            if (mine) {
+                ra  = row_rank[row];
+                own = ldg256(&P[2 * (size_t) ra]);
+                w   = (MODE == kFill) ? off[row] : ((MODE == kOnePass) ? row * cap : 0);
+                // the hi/lo records' error stays inside the band, or every candidate is decided in FP64
+                const float M = fmaxf(fmaxf(fabsf(own.a.x), fabsf(own.a.y)), fabsf(own.a.z));
+                if (!(M * M <= 1e16f * own.b.w && own.b.w > 1e-30f)) own.b.w = __int_as_float(0x7fc00000);
+            }
+            F8 a[R];
+            u32 c[R] = {}, at0[R];
+#pragma unroll
+            for (u32 j = 0; j < R; j++) {
+                auto of = [&](float v) { return __shfl_sync(kAll, v, j); };
+                a[j].a  = make_float4(of(own.a.x), of(own.a.y), of(own.a.z), 0.f);
+                a[j].b  = make_float4(of(own.b.x), of(own.b.y), of(own.b.z), of(own.b.w));
+                at0[j]  = __shfl_sync(kAll, w, j);
+            }
+            for (u32 k = 0; k < nk; k++) {
+                const uint2 run = leaf_ent[k0 + k];
+                for (u32 b0 = run.x; b0 < run.y; b0 += 32) {
+                    const u32 b     = b0 + lane;
+                    const bool real = b < run.y;
+                    const F8 q      = ldg256(&P[2 * (size_t) (real ? b : run.x)]);
+#pragma unroll
+                    for (u32 j = 0; j < R; j++) {
+                        if (!(rows >> j & 1u)) continue;
+                        const float dx = __fadd_rn(__fsub_rn(a[j].a.x, q.a.x), __fsub_rn(a[j].b.x, q.b.x));
+                        const float dy = __fadd_rn(__fsub_rn(a[j].a.y, q.a.y), __fsub_rn(a[j].b.y, q.b.y));
+                        const float dz = __fadd_rn(__fsub_rn(a[j].a.z, q.a.z), __fsub_rn(a[j].b.z, q.b.z));
+                        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)), tm = max_nan(a[j].b.w, q.b.w);
+                        bool in        = real && r2 < tm * lo_f;
+                        if (__any_sync(kAll, real && !in && !(r2 > tm * hi_f))) {
+                            const u32 rr = __shfl_sync(kAll, ra, j);
+                            if (real && !in && !(r2 > tm * hi_f)) in = pair_inside(sx, sy, sz, sh, h_tol, rr, b);
+                        }
+                        const u32 bits = __ballot_sync(kAll, in), at = c[j] + __popc(bits & below);
+                        if (MODE != kCount && in && (MODE == kFill || at < cap)) ent[at0[j] + at] = b;
+                        c[j] += __popc(bits);
+                    }
                 }
-                const u32 bits = __ballot_sync(kAll, in), at = c + __popc(bits & below);
-                c += __popc(bits);
-                if (MODE != kCount && in && (MODE == kFill || at < cap)) ent[w + at] = b;
             }
-        }
-        if (lane == 0) {
-            if (MODE != kFill) cnt[row] = c;
-            if (MODE == kCount) off[row] = (c + 3u) & ~3u;
-            if (MODE == kOnePass) {
-                off[row] = w;
-                if (c > cap) atomicOr(&sc->flags, kFlagCsrCap);
+            u32 found = c[0];
+#pragma unroll
+            for (u32 j = 1; j < R; j++) found = lane == j ? c[j] : found;
+            if (mine) {
+                if (MODE != kFill) cnt[row] = found;
+                if (MODE == kCount) off[row] = (found + 3u) & ~3u;
+                if (MODE == kOnePass) {
+                    off[row] = w;
+                    if (found > cap) atomicOr(&sc->flags, kFlagCsrCap);
+                }
+                c_max = max(c_max, found);
+                c_sum += found;
             }
-            c_max = max(c_max, c);
-            c_sum += c;
         }
     }
     cache_totals<MODE>(c_max, c_sum, sc);
@@ -936,8 +961,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     if ((e = c.leaf_rows.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = c.leaf_head.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     if ((e = c.next_row.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
-    // at most every row, once
-    if ((e = c.rows_over.ensure(sizeof(uint2) * (size_t) n, s)) != cudaSuccess) return e;
+    if ((e = c.owner.ensure(sizeof(u32) * (size_t) n, s)) != cudaSuccess) return e;
     if ((e = c.leaf_thr.ensure(sizeof(u32) * (size_t) L, s)) != cudaSuccess) return e;
     u32 *leaf_thr = c.leaf_thr.as<u32>();
     { k_cache_init<<<div_up(L, 256), 256, 0, s>>>(L, c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), leaf_thr, dsc); GBSPH_COUNTED; }
@@ -945,7 +969,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         ProfScope ps(c, kProfOwner, n);
         { k_owner<<<div_up(n, 128), 128, 0, s>>>(t, fb, rec, c.row_rank.as<u32>(), n, c.sx.as<f64>(),
                                                c.sy.as<f64>(), c.sz.as<f64>(), c.leaf_rows.as<u32>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(),
-                                               c.rows_over.as<uint2>(), dsc, c.sh.as<f64>(), up_f32(h_tol), leaf_thr); GBSPH_COUNTED; }
+                                               c.owner.as<u32>(), dsc, c.sh.as<f64>(), up_f32(h_tol), leaf_thr); GBSPH_COUNTED; }
     }
     auto stage1 = [&]() -> cudaError_t {
         cudaError_t err = c.leaf_ent.ensure(sizeof(uint2) * ((size_t) L * c.leaf_cap + 1), s);
@@ -989,8 +1013,8 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
     u32 leaf_slots = c.leaf_cap; // no bound for the lists of the exact stage 1
     auto part_rows = [&](auto mode_tag, u32 *cnt, u32 *off, u32 *ent) {
         constexpr int MODE = decltype(mode_tag)::value;
-        { k_part_rows<MODE><<<std::min(div_up(n, 8), 24 * c.sms), 256, 0, s>>>(
-            c.rows_over.as<uint2>(), c.leaf_head.as<u32>(), c.next_row.as<u32>(), c.row_rank.as<u32>(),
+        { k_part_rows<MODE><<<std::min(div_up(n, 8 * kRowsAWarp), 24 * c.sms), 256, 0, s>>>(
+            c.owner.as<u32>(), c.leaf_rows.as<u32>(), n, c.row_rank.as<u32>(),
             c.leaf_cnt.as<u32>(), c.leaf_off.as<u32>(), c.leaf_ent.as<uint2>(), P, c.sx.as<f64>(),
             c.sy.as<f64>(), c.sz.as<f64>(), c.sh.as<f64>(), h_tol, cnt, off, ent, dsc, c.row_cap, leaf_slots); GBSPH_COUNTED; }
     };
@@ -1048,7 +1072,7 @@ cudaError_t neigh_cache_build(Ctx &c, f64 h_tol, const float4 *P) {
         // stage 2 ran over cut lists, or not at all
         if ((e = stage2(true)) != cudaSuccess) return e;
         if ((e = sync_scalars(c)) != cudaSuccess) return e;
-    } else if (c.h_scalars->rows_over && one_pass) {
+    } else if (c.h_scalars->rows_left && one_pass) {
         ProfScope ps(c, kProfCacheFill, 0);
         part_rows(OnePass{}, c.csr_cnt.as<u32>(), c.csr_off.as<u32>(), c.csr_ent.as<u32>());
         if ((e = sync_scalars(c)) != cudaSuccess) return e;

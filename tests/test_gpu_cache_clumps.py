@@ -1,5 +1,5 @@
-"""Neighbour caches of clumps within one Morton cell: the rows of a leaf that owns more than 32
-are the work of many warps."""
+"""Neighbour caches of clumps within one Morton cell: the rows of a leaf that owns more than
+128 are the work of many warps."""
 import time
 
 import numpy as np
@@ -25,7 +25,7 @@ def _clumps(sizes, spread, rng):
     return pos[order], h[order]
 
 
-@pytest.mark.parametrize("sizes", [[31], [32], [33], [64, 65], [33] * 20, [40, 1, 35, 200, 2, 70], [1500]])
+@pytest.mark.parametrize("sizes", [[32], [33], [64, 65], [127], [128], [129], [130] * 5, [300, 40, 700, 1, 133], [1500]])
 @pytest.mark.parametrize("level", [0, 3])
 @pytest.mark.parametrize("budget", [0, 1])
 def test_clumped_cache_vs_oracle(sizes, level, budget):
