@@ -200,7 +200,7 @@ __global__ void k_leaf_fill(TreeView t, const u32 *__restrict__ off, uint2 *__re
 // bank per lane, the FP64 criterion is a call, and the registers are not bounded (72; with
 // 64, 40 bytes of spills make it three times slower).  1,048,576 / 8.5 M particles 580 us /
 // 3.92 ms with the stack in local memory and every passing child pushed, 538 / 3.56 with
-// inner nodes dropped too, 472 / 3.19 now; disc 940 -> 802 us.
+// inner nodes dropped too, 460 / 3.12 now; disc 940 -> 777 us.
 constexpr int kNear = 12;
 __global__ void __launch_bounds__(128) k_leaf_lists(TreeView t, const NodeBoxF *__restrict__ fb,
                                                     const NodePairF *__restrict__ rec,
@@ -545,6 +545,7 @@ __global__ void __launch_bounds__(128) k_owner(TreeView t, const NodeBoxF *__res
 //   32 at a time, 48 registers             137 /  880    / 5.37 / 1.92 /  915
 //   64 at a time, 64 registers             123 /  760    / 4.65 / 1.70 /  804
 //   and the rows' box                      118 /  684    / 4.73 / 1.67 /  801
+//   with a look at the leaf's row count      - /  689    / 4.85 / 1.69 /  810
 // (a thread per row loads a record per candidate and row, 10 L1 wavefronts a request, and its
 // lanes diverge; at 48 registers, five blocks an SM, either of the last two steps is a loss).
 // Relative positions are rounded to FP32 (u = 2^-24, twice a coordinate): with S the rows'
